@@ -56,16 +56,16 @@ E2E_MIN_STEPS = 200
 # epilogue (63.03 MB + 33.37 MB: the flow read and written once).
 JACOBI_TRAFFIC_PER_LAUNCH: dict = {"fxk_jacobi<float>": 25113088 + 768,
                                    "fxk_jacobi_res<float>": (25264640 + 1340928 + 63026944 + 33365504) // 2}
-# The two-sweep pass at 508^3 (too large for a capture): one pass (2 sweeps) of a 508x508x128
-# capture moved 266.7 MB + 104.2 MB of DRAM for 33,032,192 cells; the 508^3 figure scales it by
+# The two-sweep pass at 508^3 (too large for a capture): one pass (2 sweeps) of a 508x508x256
+# capture moved 541.0 MB + 236.3 MB of DRAM for 66,064,384 cells; the 508^3 figure scales it by
 # the cell count (its traffic grows in proportion: the same tiles and chunks over more planes).
-ZM2_CAPTURE_BYTES, ZM2_CAPTURE_CELLS = 266.7e6 + 104.2e6, 508 * 508 * 128
+TWO_SWEEP_CAPTURE_BYTES, TWO_SWEEP_CAPTURE_CELLS = 541.0e6 + 236.3e6, 508 * 508 * 256
 
-JACOBI_KERNEL_NAMES = {1: "fxk_jacobi<float>", 2: "fxk_jacobi_zm<float>", 3: "fxk_jacobi_zm2<float>",
+JACOBI_KERNEL_NAMES = {1: "fxk_jacobi<float>", 2: "fxk_jacobi_zm<float>", 3: "fxk_jacobi_zs<float>",
                        4: "fxk_jacobi_res<float>"}
 
 
-def zm2_roofline(jac: dict, cells: int, peak: float, peak_kind: str) -> dict:
+def two_sweep_roofline(jac: dict, cells: int, peak: float, peak_kind: str) -> dict:
     """The two-sweep pass at 508^3 against the copy bandwidth: algorithmic bytes per launch
     (2 sweeps x 12 B x cells) over the average launch time from the per-pass events, and the
     DRAM traffic of a launch scaled from the 508x508x128 capture."""
@@ -77,13 +77,13 @@ def zm2_roofline(jac: dict, cells: int, peak: float, peak_kind: str) -> dict:
     achieved = alg / (us / 1e6) / 1e9
     return {"roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": peak_kind, "avg_launch_us": us, "algorithmic_bytes_per_launch": alg,
-                         "traffic": ZM2_CAPTURE_BYTES * cells / ZM2_CAPTURE_CELLS,
-                         "traffic_note": "dram bytes of one launch at 508x508x128 (ncu), scaled by the cell count"}}
+                         "traffic": TWO_SWEEP_CAPTURE_BYTES * cells / TWO_SWEEP_CAPTURE_CELLS,
+                         "traffic_note": "dram bytes of one launch at 508x508x256 (ncu), scaled by the cell count"}}
 
 
 def jacobi_kernel_name(diag: dict) -> str:
     if diag.get("jacobi_kernel") == 3 and diag.get("jacobi_block") == 2:
-        return "fxk_jacobi_zm2<float>"  # two sweeps per pass
+        return "fxk_jacobi_zs<float>"  # two sweeps per pass
     return JACOBI_KERNEL_NAMES.get(diag.get("jacobi_kernel"), "fxk_jacobi<float>")
 
 
@@ -627,7 +627,7 @@ def measure_508(warmup: int = 3, steps: int = STEPS_508) -> dict:
                      "target_frac": 0.70},
         "passes": per_pass, "profiled_steps": prof,
         "jacobi": {"kernel": jacobi_kernel_name(diag), "block": diag.get("jacobi_block"),
-                   "zchunk": diag.get("jacobi_zchunk"), **zm2_roofline(per_pass["jacobi"], n, peak, peak_kind)},
+                   "zchunk": diag.get("jacobi_zchunk"), **two_sweep_roofline(per_pass["jacobi"], n, peak, peak_kind)},
         "launches_per_step": diag.get("launches_per_step"),
         "clocks": clk.summary(),
     }

@@ -157,7 +157,8 @@ class Diagnostics(C.Structure):
         ("simulate_by", C.c_int32),
         ("project_fused", C.c_int32),
         ("project_resident", C.c_int32),
-        ("reserved", C.c_int32 * 5),
+        ("jacobi_zrun", C.c_int32),
+        ("reserved", C.c_int32 * 4),
     ]
 
 

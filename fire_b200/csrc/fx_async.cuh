@@ -1,5 +1,5 @@
 // fx_async.cuh — mbarriers, bulk asynchronous copies and barrier helpers shared by the
-// kernels that move data with the Tensor Memory Accelerator (fx_jacobi_zm2t.cuh) or with bulk
+// kernels that move data with the Tensor Memory Accelerator (fx_jacobi_zs.cuh) or with bulk
 // copies issued by a copy warp (fx_jacobi_res.cuh, variant 4). Every wait here is bounded.
 #pragma once
 

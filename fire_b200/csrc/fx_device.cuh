@@ -155,7 +155,11 @@ struct __align__(16) FxSimDev {
     float jc[4];           // Jacobi wx, wy, wz, 2(wx+wy+wz) (shaders.ts:386-389), f32
     float jcRcp;           // RN(1 / jc[3])
     int jcFastDiv;         // 1: x / jc[3] may use fx_div_by_const (checked exhaustively)
-    int pad2[2];
+    int jcTwo;             // 1: x / jc[3] may use the two-operation quotient (checked exhaustively)
+    float jcRh, jcRl;      // its reciprocal 1 / jc[3] as a sum of two floats, jcRl > 0
+    float jcLo;            // smallest |x| it was checked for
+    double jcRcpD;         // RN(1 / jc[3]) in double: the quotients below jcLo
+    int pad2[12];
     void* flow[2];         // float4 records (both storages)
     void* species[2];      // float4 (F32) or 4 x half (MIXED)
     void* p[2];            // primary pressure: float (F32 / COLD) or half (F16 / MIXED)
@@ -179,7 +183,7 @@ struct __align__(16) FxSimDev {
                            // phases (zeroed at every step start)
     int tmapOk;            // 1: tmap holds valid tensor maps (FP32 pressure)
     int tmapPad[15];
-    CUtensorMap tmap[5];   // pressure pair, correction pair, divergence (fx_jacobi_zm2t.cuh)
+    CUtensorMap tmap[5];   // pressure pair, correction pair, divergence (fx_jacobi_zs.cuh)
 };
 
 // Work decomposition shared by every batched pass: each pass walks a flat list of
@@ -205,7 +209,7 @@ struct FxResBox {
 // CELL: 32 x BY x (8 / BY) cells, one thread per cell (simulate); BY = FX_CELL_BY unless
 //       the plan tunes it (firex_set_tiles).
 // ROW4: 256 groups of 4 consecutive x cells in memory order (stencils).
-// COL : tiles x z chunks of the two-sweep Jacobi pass (see fx_jacobi_zm2.cuh).
+// COL : tiles x z chunks of the two-sweep Jacobi pass (see fx_jacobi_zs.cuh).
 // ZM  : z-marching tiles of the single-sweep Jacobi (see fx_jacobi_zm.cuh).
 // TAB : 256 entries of the per-step tables of simulate.
 #define FX_CELL_BX 32

@@ -26,7 +26,7 @@
 #include "fx_internal.h"
 #include "fx_jacobi_res.cuh"
 #include "fx_jacobi_zm.cuh"
-#include "fx_jacobi_zm2.cuh"
+#include "fx_jacobi_zs.cuh"
 
 static_assert(offsetof(FxSimDev, tmap) % 64 == 0, "tensor maps must sit on 64-byte boundaries");
 
@@ -128,14 +128,15 @@ long long bricks_row4(int X, int Y, int Z) {
 struct StepPlan {
     int storage = 0;
     bool half = false;
-    int pmode = FX_TB_F32;    // pressure storage / rounding of the fused Jacobi
     int maxP = 0, maxR = 0;
-    int k = 1, zc = 16;       // fused sweeps per Jacobi launch, z planes per CTA
+    int k = 1, zc = 16;       // fused sweeps per Jacobi launch, z planes per CTA asked for
+    int zrun = 16;            // ... and those the launches take (zs_run)
     int zmZc = 16;            // z planes per CTA of the single-sweep (z-marching) kernel
     bool row4 = false;        // single sweeps by the unblocked kernel instead
     bool fuseP = false, fuseR = false;
     bool pack = false;        // a member packs its render volumes at the end of every step
     bool tma = false;         // the two-sweep pass stages its planes by TMA
+    bool two = false;         // every member's denominator has a checked two-operation quotient
     int simBy = FX_CELL_BY;   // source-pass bricks: 32 x simBy x (8 / simBy) cells
     bool projDiv = true;      // the primary projection and the residual divergence in one pass
     bool res = false;         // every sweep of a phase in one resident launch
@@ -145,7 +146,7 @@ struct StepPlan {
     bool simEarly = false;    // the source pass evaluates its neighbour terms before the advection
     int bricks[FX_NSHAPES] = {};
     auto key() const {
-        return std::tie(storage, half, pmode, maxP, maxR, k, zc, zmZc, row4, fuseP, fuseR, pack, tma, simBy, projDiv, res,
+        return std::tie(storage, half, maxP, maxR, k, zc, zrun, zmZc, row4, fuseP, fuseR, pack, tma, two, simBy, projDiv, res,
                         resVariant, resSmem, projRes, simEarly,
                         bricks[0],
                         bricks[1], bricks[2], bricks[3], bricks[4], bricks[5], bricks[6]);
@@ -160,16 +161,16 @@ struct StepPlan {
 #define FX_PROJ_RES 1  // the residual projection as the resident variant 4's epilogue when it can
 #endif
 
-// A phase of n sweeps may fuse k sweeps per launch when every member runs the same n
-// and the launch count (n/k fused + n%k single) has the parity of n: the result then
-// lands in the buffer the reference's ping-pong leaves it in.
-bool can_fuse(int k, int n) { return k > 1 && n >= k && ((k - 1) * (n / k)) % 2 == 0; }
+// Two-sweep launches of a phase of n sweeps: an even number, the rest (up to three) as single
+// sweeps, so the launch count has the parity of n and the result lands in the buffer the
+// reference's ping-pong leaves it in.
+int fused_pairs(int n) { return (n / 2) & ~1; }
 
 int jacobi_phase_launches(const StepPlan& pl, int phase) {
     const int n = phase == 0 ? pl.maxP : pl.maxR;
     if (pl.res) return n > 0 ? 1 : 0;
     const bool fuse = phase == 0 ? pl.fuseP : pl.fuseR;
-    return fuse ? n / pl.k + n % pl.k : n;
+    return fuse ? n - fused_pairs(n) : n;
 }
 
 void enqueue_jacobi_phase(cudaStream_t st, const StepPlan& pl, FxBatchDev* B, int phase) {
@@ -183,8 +184,8 @@ void enqueue_jacobi_phase(cudaStream_t st, const StepPlan& pl, FxBatchDev* B, in
     const bool fuse = phase == 0 ? pl.fuseP : pl.fuseR;
     int launch = 0, sweep = 0;
     if (fuse) {
-        for (; sweep + pl.k <= n; sweep += pl.k, ++launch)
-            fx_launch_jacobi_tb(st, pl.pmode, pl.k, B, pl.bricks[FX_SHAPE_COL], phase, launch, pl.zc, pl.tma);
+        for (; launch < fused_pairs(n); sweep += 2, ++launch)
+            fx_launch_jacobi_two(st, pl.half, B, pl.bricks[FX_SHAPE_COL], phase, launch, pl.zrun, pl.tma, pl.two);
     }
     for (; sweep < n; ++sweep, ++launch) {
         if (pl.row4) fx_launch_jacobi(st, pl.half, B, pl.bricks[FX_SHAPE_ROW4], phase, launch, sweep);
@@ -214,19 +215,16 @@ void enqueue_step_launches(cudaStream_t st, const StepPlan& pl, FxBatchDev* B) {
     if (pl.pack) fx_launch_pack_batch(st, B, pl.bricks[FX_SHAPE_ROW4]);
 }
 
-// Jacobi kernel when the caller did not choose one (measured on B200, 96+96 sweeps):
-// below 8 Mi cells per batch the unblocked kernel (the pressure pair and the divergence
-// stay in L2 and more CTAs hide latency; at 160x240x160 the z-marching kernel only ties
-// it); from 8 Mi cells, where they outgrow L2, two sweeps per pass by z-marching tiles
-// (the fused kernel with block 2) with 16-plane chunks (192x288x192: 6.29 ms per step
-// against 6.48 with one sweep per pass and 7.52 unblocked), and from 16 Mi cells with
-// 64-plane chunks (508^3: 45.1 ms of Jacobi per step against 56.5 ms for one sweep per
-// pass). fire_b200/autotune.py refines this per workload.
+// Jacobi kernel when the caller did not choose one (measured on B200, 96+96 sweeps): below 2 Mi
+// cells per batch the unblocked kernel; from there two sweeps per pass by z-marching strips
+// (160x240x160: 2.14 ms of Jacobi per step against 3.95 unblocked; 508^3: 31.6 against 56.5
+// for one sweep per pass), in chunks of 16 planes, or 64 from 16 Mi cells, stretched or shortened
+// to fill the device's waves (zs_run). fire_b200/autotune.py refines this per workload.
 void default_jacobi(long long cells, int* kernel, int* k, int* zc) {
-    const bool big = cells >= (16LL << 20), mid = !big && cells >= (8LL << 20);
-    *kernel = (big || mid) ? FIREX_JACOBI_FUSED : FIREX_JACOBI_UNBLOCKED;
-    *k = (big || mid) ? 2 : 1;
-    *zc = big ? 64 : (mid ? 16 : 32);
+    const bool fused = cells >= (2LL << 20);
+    *kernel = fused ? FIREX_JACOBI_FUSED : FIREX_JACOBI_UNBLOCKED;
+    *k = fused ? 2 : 1;
+    *zc = cells >= (16LL << 20) ? 64 : 16;
 }
 
 // Box decomposition of an X x Y x Z grid over at most m CTAs for the resident Jacobi
@@ -387,6 +385,56 @@ static bool fast_division_ok(int device, float d, float rcp, float lo = 1.262177
     return ok;
 }
 
+// The reciprocal 1/d = rh + rl (rh rounded down, so rl > 0) with which fx_div_two equals IEEE
+// x / d for every float x on this device, checked like fast_division_ok: rl rounded to nearest,
+// or one or two steps beside it (that rounding decides the few quotients next to a midpoint).
+struct TwoOpReciprocal {
+    bool ok = false;
+    float rh = 0, rl = 0, lo = 0;
+};
+static TwoOpReciprocal two_op_reciprocal(int device, float d) {
+    static std::map<std::pair<int, uint32_t>, TwoOpReciprocal> cache;
+    static std::mutex mu;
+    TwoOpReciprocal r;
+    if (!(d > 1.0f && d < 1073741824.0f)) return r;
+    std::lock_guard<std::mutex> lock(mu);
+    uint32_t bits;
+    std::memcpy(&bits, &d, 4);
+    auto it = cache.find({device, bits});
+    if (it != cache.end()) return it->second;
+    const double rcp = 1.0 / (double)d;
+    r.rh = (float)rcp;
+    if ((double)r.rh > rcp) r.rh = std::nextafter(r.rh, 0.0f);
+    float rl = (float)(rcp - (double)r.rh);
+    if (rl == 0.0f) rl = std::ldexp(r.rh, -60);  // a power of two: any tiny positive term rounds away
+    r.lo = std::ldexp(1.0f, -60 + std::ilogb(d));
+    const float up = std::nextafter(rl, INFINITY), down = std::nextafter(rl, 0.0f);
+    const float tries[5] = {rl, up, down, std::nextafter(up, INFINITY), std::nextafter(down, 0.0f)};
+    unsigned long long* dcount = nullptr;
+    cudaStream_t st = nullptr;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaMalloc(&dcount, sizeof(unsigned long long)) == cudaSuccess) {
+        for (float t : tries) {
+            unsigned long long bad = ~0ull;
+            if (cudaMemsetAsync(dcount, 0, sizeof(bad), st) != cudaSuccess) break;
+            fx_launch_check_div_two(st, d, r.rh, t, r.lo, rcp, dcount);
+            if (cudaMemcpyAsync(&bad, dcount, sizeof(bad), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                break;
+            if (bad == 0) {
+                r.ok = true;
+                r.rl = t;
+                break;
+            }
+        }
+    }
+    cudaGetLastError();
+    if (dcount) cudaFree(dcount);
+    if (st) cudaStreamDestroy(st);
+    cache[{device, bits}] = r;
+    return r;
+}
+
 // ---- one simulation ------------------------------------------------------------------------
 struct firex_sim {
     int X = 0, Y = 0, Z = 0;
@@ -529,6 +577,12 @@ struct firex_sim {
         h.jc[3] = 2.0f * (h.jc[0] + h.jc[1] + h.jc[2]);
         h.jcRcp = 1.0f / h.jc[3];
         h.jcFastDiv = fast_division_ok(device, h.jc[3], h.jcRcp) ? 1 : 0;
+        const TwoOpReciprocal two = two_op_reciprocal(device, h.jc[3]);
+        h.jcTwo = two.ok ? 1 : 0;
+        h.jcRh = two.rh;
+        h.jcRl = two.rl;
+        h.jcLo = two.lo;
+        h.jcRcpD = 1.0 / (double)h.jc[3];
         // constant divisors of simulate, computed with the same f32 operations as the
         // expressions they stand for
         auto fmaxr = [](float a, float b) { return (a < b) ? b : a; };
@@ -618,6 +672,7 @@ struct firex_batch {
     int projFuse = FIREX_PROJECT_AUTO; // batch override of the projection fusion (AUTO: first member's)
     int tableK = -1, tableZc = -1, tableZmZc = -1;  // launch shapes the prefix sums were built for
     int tableSimBy = -1;
+    bool tableTma = false;
     int tableRes = -1;                               // whether resident boxes were requested
     std::vector<char> tableWater;                    // which members sprayed when the table was filled
     bool resOk = false;                              // ... and the batch fits one resident launch
@@ -647,7 +702,7 @@ struct firex_batch {
 
     // Fills the brick prefix sums for the launch shape (k, zc); resident boxes when wanted,
     // of variant resForce when that is 0-4.
-    void fill_table(int k, int zc, int zmZc, bool wantRes, int resForce, int simBy) {
+    void fill_table(int k, int zc, int zmZc, bool wantRes, int resForce, int simBy, bool tma) {
         int acc[FX_NSHAPES] = {};
         h->nsims = (int)members.size();
         std::vector<FxResBox> boxes;
@@ -688,7 +743,7 @@ struct firex_batch {
             acc[FX_SHAPE_TAB] += (fx_tab_layout(s->X, s->Y, s->Z).total + 255) / 256;
             acc[FX_SHAPE_CELL] += (int)bricks_cell(s->X, s->Y, s->Z, simBy);
             acc[FX_SHAPE_ROW4] += (int)bricks_row4(s->X, s->Y, s->Z);
-            acc[FX_SHAPE_COL] += k == 2 ? fx_zm2_bricks(s->X, s->Y, s->Z, zc) : 0;
+            acc[FX_SHAPE_COL] += k != 2 ? 0 : fx_zs_bricks(s->X, s->Y, s->Z, zc, FX_ZS_TXG);
             acc[FX_SHAPE_ZM] += fx_zm_bricks(s->X, s->Y, s->Z, zmZc);
         }
         for (int j = 0; j < FX_NSHAPES; ++j) {
@@ -697,11 +752,42 @@ struct firex_batch {
         }
         tableK = k;
         tableSimBy = simBy;
+        tableTma = tma;
         tableZc = zc;
         tableZmZc = zmZc;
         tableRes = wantRes ? 2 + resForce : 0;
         tableWater = water_signature();
         tableDirty = true;
+    }
+
+    // z planes per CTA of the two-sweep pass when the caller did not ask for a number: the chunk
+    // length that takes the fewest plane steps, counting a chunk's own planes, the one beside it
+    // at each end and the time its first planes take to arrive (about two steps more), over the
+    // waves of CTAs its bricks make on the device.
+    static int zs_run(const std::vector<firex_sim*>& members, int k) {
+        if (k != 2) return 16;
+        const int slots = fx_zs_capacity(members[0]->half);
+        int best = 16, maxZ = 0;
+        double least = 0;
+        for (firex_sim* s : members) maxZ = std::max(maxZ, s->Z);
+        if (members[0]->half) maxZ = std::min(maxZ, 64);  // FP16 rows: 412x616x412 17.0 ms at 52 planes, 18.0 at 206
+        for (int zc = std::min(4, maxZ); zc <= maxZ; ++zc) {
+            long long bricks = 0, steps = 0;
+            for (firex_sim* s : members) {
+                const long long n = fx_zs_bricks(s->X, s->Y, s->Z, zc, FX_ZS_TXG);
+                const int chunks = (s->Z + zc - 1) / zc;
+                bricks += n;
+                steps += n / chunks * (s->Z + 4LL * chunks);
+            }
+            const double waves = (double)((bricks + slots - 1) / slots);
+            // uneven members fill a wave's end with short chunks: never below the mean load
+            const double cost = std::max(std::min(waves * (zc + 4.0), steps / (double)slots + zc + 4.0), steps / (double)slots);
+            if (least == 0 || cost < least * 0.999) {
+                least = cost;
+                best = zc;
+            }
+        }
+        return best;
     }
 
     std::vector<char> water_signature() const {
@@ -715,7 +801,6 @@ struct firex_batch {
         if (members.empty()) return p;
         p.storage = members[0]->storage;
         p.half = members[0]->half;
-        p.pmode = p.half ? FX_TB_F16_ROUND : FX_TB_F32;
         bool uniformP = true, uniformR = true;
         long long cells = 0;
         for (firex_sim* s : members) {
@@ -734,13 +819,14 @@ struct firex_batch {
         // AUTO and RESIDENT try the resident launch first; the default is the fallback when
         // the batch does not fit on chip
         const bool wantRes = kernel == FIREX_JACOBI_AUTO || kernel == FIREX_JACOBI_RESIDENT;
-        if (kernel == FIREX_JACOBI_AUTO || kernel == FIREX_JACOBI_RESIDENT) {
+        const bool autoKernel = wantRes, zcOwn = zc > 0;
+        if (autoKernel) {
             int dk = 1, dzc = 32;
             default_jacobi(cells, &kernel, &dk, &dzc);
             k = dk;
             if (zc <= 0) zc = dzc;
         }
-        if (kernel != FIREX_JACOBI_FUSED || (k != 2 && k != 3 && k != 4 && k != 6)) k = 1;
+        if (kernel != FIREX_JACOBI_FUSED || k != 2) k = 1;
         long long zm32 = 0, zm16 = 0;
         for (firex_sim* s : members) {
             zm32 += fx_zm_bricks(s->X, s->Y, s->Z, 32);
@@ -748,8 +834,9 @@ struct firex_batch {
         }
         p.k = k;
         p.zc = zc > 0 ? zc : 16;
-        p.fuseP = uniformP && can_fuse(k, p.maxP);
-        p.fuseR = uniformR && can_fuse(k, p.maxR);
+        p.zrun = zcOwn ? p.zc : zs_run(members, k);
+        p.fuseP = k == 2 && uniformP && fused_pairs(p.maxP) > 0;
+        p.fuseR = k == 2 && uniformR && fused_pairs(p.maxR) > 0;
         if (!p.fuseP && !p.fuseR) p.k = 1;
         p.row4 = kernel == FIREX_JACOBI_UNBLOCKED;
         p.zmZc = (kernel == FIREX_JACOBI_ZMARCH && zc > 0) ? zc : zm_chunk(zm32, zm16);
@@ -766,16 +853,21 @@ struct firex_batch {
         // 0.194, 160x240x160 0.353 / 0.361, 192x288x192 0.604 / 0.618; 256^3 1.010 / 0.964;
         // mixed storage HD 0.181 / 0.174, 160x240x160 0.344 / 0.326)
         p.simEarly = p.storage == FX_STORAGE_F32 && cells < FX_SIM_EARLY_CELLS;
-        if (tableK != p.k || tableZc != p.zc || tableZmZc != p.zmZc || tableRes != (wantRes ? 2 + resForce : 0) ||
-            tableWater != water_signature() || tableSimBy != p.simBy)
-            fill_table(p.k, p.zc, p.zmZc, wantRes, resForce, p.simBy);
-        // TMA staging of the two-sweep pass when asked for: FP32 pressure and every member's
-        // tensor maps built. AUTO stages by cp.async, measured faster on B200 (508^3: 45.2 ms of
-        // Jacobi per step against 49.4 with TMA; 192x288x192: 5.64 against 6.10)
+        // The two-sweep pass stages its planes by TMA (FP32 pressure, every member's tensor maps
+        // built) when asked to, or when AUTO chose the pass with chunks that fill the device's
+        // waves: tensor loads then cost a warp next to nothing (160x240x160: 2.14 against 2.56 ms
+        // of Jacobi per step with cp.async, 508^3: 31.6 against 34.8). A pass asked for with a chunk
+        // of the caller's keeps cp.async, whose planes land sooner in short chunks (188x284x196,
+        // 14-plane chunks: 2.63 against 2.85).
         const int staging = this->staging != FIREX_STAGING_AUTO ? this->staging : members[0]->staging;
-        bool maps = p.pmode == FX_TB_F32 && staging == FIREX_STAGING_TMA;
+        bool maps = !p.half && (staging == FIREX_STAGING_TMA || (staging == FIREX_STAGING_AUTO && autoKernel));
         for (firex_sim* s : members) maps = maps && s->h.tmapOk;
         p.tma = p.k == 2 && maps;
+        p.two = true;
+        for (firex_sim* s : members) p.two = p.two && s->h.jcTwo;
+        if (tableK != p.k || tableZc != p.zrun || tableZmZc != p.zmZc || tableRes != (wantRes ? 2 + resForce : 0) ||
+            tableWater != water_signature() || tableSimBy != p.simBy || tableTma != p.tma)
+            fill_table(p.k, p.zrun, p.zmZc, wantRes, resForce, p.simBy, p.tma);
         p.res = wantRes && resOk;
         if (p.res) {
             p.resSmem = resSmem;
@@ -1700,6 +1792,7 @@ int firex_get_diagnostics(const firex_sim* s, firex_diagnostics* out) {
     out->fast_division = s->h.jcFastDiv;
     out->jacobi_block = p.k;
     out->jacobi_zchunk = p.k > 1 ? p.zc : (p.row4 ? 0 : p.zmZc);
+    out->jacobi_zrun = p.k > 1 ? p.zrun : out->jacobi_zchunk;
     out->graph = b->lastGraph ? 1 : 0;
     out->launches_per_step =
         (p.projDiv ? 7 : 8) - (p.projRes ? 1 : 0) + (p.pack ? 1 : 0) + sph_launches(p) + jacobi_phase_launches(p, 0) +

@@ -23,11 +23,12 @@ void fx_launch_jacobi(cudaStream_t s, bool half, const FxBatchDev* B, int bricks
 // One sweep by z-marching tiles of zc planes (fx_jacobi_zm.cuh).
 void fx_launch_jacobi_zm(cudaStream_t s, bool half, const FxBatchDev* B, int bricks, int phase, int launch, int sweep,
                          int zc);
-// K fused sweeps per launch; pmode selects the pressure storage and rounding.
-enum { FX_TB_F32 = 0, FX_TB_F16_ROUND = 1, FX_TB_F16 = 2 };
-// Two sweeps per launch (k = 2); with tma (FP32 pressure only) the planes are staged by TMA.
-bool fx_launch_jacobi_tb(cudaStream_t s, int pmode, int k, const FxBatchDev* B, int bricks, int phase, int launch, int zc,
-                         bool tma);
+// Two sweeps per launch by strips of zc planes (fx_jacobi_zs.cuh); with tma (FP32 pressure only)
+// the planes are staged by tensor loads. two: every member's Jacobi denominator has a checked
+// two-operation quotient (fx_div_two).
+void fx_launch_jacobi_two(cudaStream_t s, bool half, const FxBatchDev* B, int bricks, int phase, int launch, int zc, bool tma,
+                          bool two);
+int fx_zs_capacity(bool half);  // CTAs of that launch the device holds at once
 // Tensor maps of a simulation's pressure pair, correction pair and divergence for the
 // TMA-staged two-sweep pass; false when the driver refuses one (the pass then uses cp.async).
 bool fx_make_tensor_maps(FxSimDev* h);
@@ -62,6 +63,9 @@ void fx_launch_upload_batch(cudaStream_t s, const FxBatchDev& host, FxBatchDev* 
 
 // Exhaustive check of fx_div_by_const against IEEE division for one denominator.
 void fx_launch_check_div(cudaStream_t s, float d, float rcp, float lo, float hi, unsigned long long* mismatches);
+
+// The same for fx_div_two with the reciprocal rh + rl and the small-operand bound lo.
+void fx_launch_check_div_two(cudaStream_t s, float d, float rh, float rl, float lo, double rcp, unsigned long long* mismatches);
 
 // Sets the text that firex_last_error(NULL) returns on the calling thread (fx_engine.cu).
 void fx_set_thread_error(const std::string& msg);

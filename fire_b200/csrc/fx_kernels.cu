@@ -18,8 +18,7 @@
 #include "fx_jacobi_res.cuh"
 #include "fx_sph.cuh"
 #include "fx_jacobi_zm.cuh"
-#include "fx_jacobi_zm2.cuh"
-#include "fx_jacobi_zm2t.cuh"
+#include "fx_jacobi_zs.cuh"
 #include "fx_step_math.cuh"
 #include "fx_storage.cuh"
 
@@ -487,62 +486,48 @@ __global__ void __launch_bounds__(FX_ZM_THREADS, 3) fxk_jacobi_zm(const FxBatchD
     });
 }
 
-// ---- two Jacobi sweeps per pass by z-marching tiles (fx_jacobi_zm2.cuh) ------------------------
-template <typename PT, bool ROUND>
-__global__ void __launch_bounds__(FX_Z2_THREADS, FX_Z2_MINB) fxk_jacobi_zm2(const FxBatchDev* __restrict__ B, int phase, int launch,
-                                                                int zc) {
-    extern __shared__ __align__(16) unsigned char fx_z2_dyn[];
-    FxZ2Smem<PT>& sm = *reinterpret_cast<FxZ2Smem<PT>*>(fx_z2_dyn);
+// ---- two Jacobi sweeps per pass by z-marching strips (fx_jacobi_zs.cuh) ------------------------
+template <typename PT, bool ROUND, bool TWO, bool TMA>
+__global__ void __launch_bounds__(FX_ZS_THREADS, FX_ZS_MINB) fxk_jacobi_zs(const FxBatchDev* __restrict__ B, int phase, int launch, int zc) {
+    extern __shared__ __align__(128) unsigned char fx_zs_dyn[];
+    constexpr int TXG = FX_ZS_TXG;
+    using H = FxZsShape<TXG>;
+    using Smem = FxZsSmem<PT, TXG>;
+    Smem& sm = *reinterpret_cast<Smem*>(fx_zs_dyn);
+    if (TMA) {
+        if (threadIdx.x == 0) {
+            fx_mbar_init(&sm.bar, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        }
+        __syncthreads();
+    }
+    unsigned parity = 0;  // of the barrier's next phase
+    bool ok = true;
     fx_for_bricks<FX_SHAPE_COL>(B, [&](const FxSimDev& S, int b) {
-        const int ntx = (S.X + FX_Z2_TX - 1) / FX_Z2_TX, nty = (S.Y + FX_Z2_TY - 1) / FX_Z2_TY;
+        if (!ok) return;  // a bounded wait ran out in an earlier brick
+        const int ntx = (S.X + H::TX - 1) / H::TX, nty = (S.Y + H::TY - 1) / H::TY;
         const int tx = b % ntx, ty = (b / ntx) % nty, zci = b / (ntx * nty);
         const int z0 = zci * zc, z1 = min(S.Z, z0 + zc);
         const FxSolveBufs bufs = fx_solve_bufs(S, phase, launch);
         const PT* pin = reinterpret_cast<const PT*>(bufs.pin);
         PT* pout = reinterpret_cast<PT*>(bufs.pout);
-        if (bufs.zeroIn) fx_zm2_tile<PT, true, ROUND>(S, pin, pout, tx * FX_Z2_TX, ty * FX_Z2_TY, z0, z1, sm);
-        else fx_zm2_tile<PT, false, ROUND>(S, pin, pout, tx * FX_Z2_TX, ty * FX_Z2_TY, z0, z1, sm);
+        const int x0 = tx * H::TX, y0 = ty * H::TY;
+        const CUtensorMap* mapP = TMA ? fx_zs_map_of(S, bufs.pin) : nullptr;
+        const CUtensorMap* mapD = &S.tmap[FX_TM_DIV];
+        const bool top = y0 + H::TY >= S.Y - 1;  // the tile or its ring reaches the open top
+        if (TMA && threadIdx.x == 0) {  // the thread that issues the tensor loads
+            if (!bufs.zeroIn) fx_zs_map_acquire(mapP);
+            fx_zs_map_acquire(mapD);
+        }
+        if (bufs.zeroIn) {
+            ok = top ? fx_zs_tile<PT, TXG, true, ROUND, TWO, true, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity)
+                     : fx_zs_tile<PT, TXG, true, ROUND, TWO, false, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity);
+        } else {
+            ok = top ? fx_zs_tile<PT, TXG, false, ROUND, TWO, true, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity)
+                     : fx_zs_tile<PT, TXG, false, ROUND, TWO, false, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity);
+        }
+        if (!ok && threadIdx.x == 0) atomicExch(S.sync + 2, 1u);
     });
-}
-
-// ---- two Jacobi sweeps per pass, planes staged by TMA (fx_jacobi_zm2t.cuh), FP32 pressure --------
-__global__ void __launch_bounds__(FX_Z2_THREADS, FX_Z2_MINB) fxk_jacobi_zm2t(const FxBatchDev* __restrict__ B, int phase,
-                                                                int launch, int zc) {
-    extern __shared__ __align__(128) unsigned char fx_t2_dyn[];
-    // the slots must start on 128-byte boundaries: align the dynamic window (128 bytes spare)
-    FxT2Smem& sm = *reinterpret_cast<FxT2Smem*>((reinterpret_cast<uintptr_t>(fx_t2_dyn) + 127) & ~(uintptr_t)127);
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < FX_T2_SLOTS; ++i) fx_mbar_init(&sm.bar[i], 1);
-        sm.err = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    __syncthreads();
-    unsigned phases = 0;  // parity of each slot's next barrier phase (the same in every thread)
-    const int total = B->total[FX_SHAPE_COL];
-    int lo = 0, hi = -1, si = 0;
-    for (int w = blockIdx.x; w < total; w += gridDim.x) {
-        if (w < lo || w >= hi) {
-            si = fx_find_sim(B->start[FX_SHAPE_COL], B->nsims, w);
-            lo = __ldg(&B->start[FX_SHAPE_COL][si]);
-            hi = __ldg(&B->start[FX_SHAPE_COL][si + 1]);
-        }
-        const FxSimDev& S = *B->sims[si];
-        if (!S.active) continue;
-        const int b = w - lo;
-        const int ntx = (S.X + FX_Z2_TX - 1) / FX_Z2_TX, nty = (S.Y + FX_Z2_TY - 1) / FX_Z2_TY;
-        const int tx = b % ntx, ty = (b / ntx) % nty, zci = b / (ntx * nty);
-        const int z0 = zci * zc, z1 = min(S.Z, z0 + zc);
-        const FxSolveBufs bufs = fx_solve_bufs(S, phase, launch);
-        float* pout = reinterpret_cast<float*>(bufs.pout);
-        const bool ok = bufs.zeroIn
-                            ? fx_zm2t_tile<true>(S, nullptr, pout, tx * FX_Z2_TX, ty * FX_Z2_TY, z0, z1, sm, phases)
-                            : fx_zm2t_tile<false>(S, fx_t2_map_of(S, bufs.pin), pout, tx * FX_Z2_TX, ty * FX_Z2_TY, z0,
-                                                  z1, sm, phases);
-        if (!ok) {  // a barrier wait ran out: report it and stop this CTA
-            if (threadIdx.x == 0) atomicExch(S.sync + 2, 1u);
-            return;
-        }
-    }
 }
 
 // Counts the floats x for which fx_div_by_const(x, d, rcp) differs from the IEEE
@@ -555,6 +540,19 @@ __global__ void fxk_check_div(float d, float rcp, float lo, float hi, unsigned l
         const float x = __uint_as_float((unsigned)b);
         const float a = fx_div_range(x, d, rcp, lo, hi), e = __fdiv_rn(x, d);
         bad += (__float_as_uint(a) != __float_as_uint(e)) && !(a != a && e != e);  // NaN == NaN
+    }
+    if (bad) atomicAdd(mismatches, bad);
+}
+
+// The same for fx_div_two.
+__global__ void fxk_check_div_two(float d, float rh, float rl, float lo, double rcp, unsigned long long* __restrict__ mismatches) {
+    unsigned long long bad = 0;
+    const unsigned long long n = 1ull << 32;
+    for (unsigned long long b = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; b < n;
+         b += (unsigned long long)gridDim.x * blockDim.x) {
+        const float x = __uint_as_float((unsigned)b);
+        const float a = fx_div_two(x, rh, rl, lo, d, rcp), e = __fdiv_rn(x, d);
+        bad += (__float_as_uint(a) != __float_as_uint(e)) && !(a != a && e != e);
     }
     if (bad) atomicAdd(mismatches, bad);
 }
@@ -905,21 +903,27 @@ void fx_launch_jacobi_zm(cudaStream_t s, bool half, const FxBatchDev* B, int bri
     else launch_zm<float>(s, B, bricks, phase, launch, sweep, zc);
 }
 
-template <typename PT, bool ROUND>
-static void launch_zm2(cudaStream_t s, const FxBatchDev* B, int bricks, int phase, int launch, int zc) {
-    static int g = [] {
-        cudaFuncSetAttribute((const void*)fxk_jacobi_zm2<PT, ROUND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(FxZ2Smem<PT>));
+template <typename PT, bool TWO, bool TMA>
+static int zs_grid() {  // CTAs the device holds at once
+    static const int g = [] {
+        const void* fn = (const void*)fxk_jacobi_zs<PT, sizeof(PT) == 2, TWO, TMA>;
+        constexpr int smem = (int)sizeof(FxZsSmem<PT, FX_ZS_TXG>);
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fxk_jacobi_zm2<PT, ROUND>, FX_Z2_THREADS,
-                                                      sizeof(FxZ2Smem<PT>));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, FX_ZS_THREADS, smem);
         return (per_sm > 0 ? per_sm : 1) * num_sms();
     }();
-    fxk_jacobi_zm2<PT, ROUND><<<bricks < g ? bricks : g, FX_Z2_THREADS, sizeof(FxZ2Smem<PT>), s>>>(B, phase, launch, zc);
+    return g;
 }
+template <typename PT, bool TWO, bool TMA>
+static void launch_zs(cudaStream_t s, const FxBatchDev* B, int bricks, int phase, int launch, int zc) {
+    const int g = zs_grid<PT, TWO, TMA>();
+    fxk_jacobi_zs<PT, sizeof(PT) == 2, TWO, TMA><<<bricks < g ? bricks : g, FX_ZS_THREADS, sizeof(FxZsSmem<PT, FX_ZS_TXG>), s>>>(B, phase, launch, zc);
+}
+int fx_zs_capacity(bool half) { return half ? zs_grid<__half, true, false>() : zs_grid<float, true, false>(); }
 
-#ifndef FX_T2_L2_PROMOTION
-#define FX_T2_L2_PROMOTION CU_TENSOR_MAP_L2_PROMOTION_L2_128B
+#ifndef FX_ZS_L2_PROMOTION
+#define FX_ZS_L2_PROMOTION CU_TENSOR_MAP_L2_PROMOTION_L2_128B
 #endif
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link-time dependency on
 // the driver library).
@@ -940,15 +944,15 @@ static EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// A 3-D FP32 map of an X x Y x Z field (x fastest) with boxes of FX_Z2_COLS x boxY x 1 cells:
+// A 3-D FP32 map of an X x Y x Z field (x fastest) with boxes of COLS x boxY x 1 cells:
 // row stride X * 4 bytes (a multiple of 16: X is a multiple of 4), out-of-bound cells read 0.
 static bool map_field(EncodeTiledFn fn, CUtensorMap* m, void* base, int X, int Y, int Z, int boxY) {
     const cuuint64_t dims[3] = {(cuuint64_t)X, (cuuint64_t)Y, (cuuint64_t)Z};
     const cuuint64_t strides[2] = {(cuuint64_t)X * 4, (cuuint64_t)X * (cuuint64_t)Y * 4};
-    const cuuint32_t box[3] = {FX_Z2_COLS, (cuuint32_t)boxY, 1};
+    const cuuint32_t box[3] = {FxZsShape<FX_ZS_TXG>::COLS, (cuuint32_t)boxY, 1};
     const cuuint32_t elem[3] = {1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, FX_T2_L2_PROMOTION, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              CU_TENSOR_MAP_SWIZZLE_NONE, FX_ZS_L2_PROMOTION, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 bool fx_make_tensor_maps(FxSimDev* h) {
@@ -957,34 +961,20 @@ bool fx_make_tensor_maps(FxSimDev* h) {
     if (!fn || h->mode == FIREX_PRESSURE_F16 || (h->X & 3) != 0) return false;
     void* bufs[4] = {h->p[0], h->p[1], h->corr[0], h->corr[1]};
     for (int i = 0; i < 4; ++i)
-        if (!map_field(fn, &h->tmap[FX_TM_P0 + i], bufs[i], h->X, h->Y, h->Z, FX_T2_PBOX_Y)) return false;
-    if (!map_field(fn, &h->tmap[FX_TM_DIV], h->div, h->X, h->Y, h->Z, FX_T2_DBOX_Y)) return false;
+        if (!map_field(fn, &h->tmap[FX_TM_P0 + i], bufs[i], h->X, h->Y, h->Z, FxZsShape<FX_ZS_TXG>::PROWS)) return false;
+    if (!map_field(fn, &h->tmap[FX_TM_DIV], h->div, h->X, h->Y, h->Z, FxZsShape<FX_ZS_TXG>::NR)) return false;
     h->tmapOk = 1;
     return true;
 }
 
-static void launch_zm2t(cudaStream_t s, const FxBatchDev* B, int bricks, int phase, int launch, int zc) {
-    constexpr int smem = (int)sizeof(FxT2Smem) + 128;
-    static int g = [] {
-        cudaFuncSetAttribute((const void*)fxk_jacobi_zm2t, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fxk_jacobi_zm2t, FX_Z2_THREADS, smem);
-        return (per_sm > 0 ? per_sm : 1) * num_sms();
-    }();
-    fxk_jacobi_zm2t<<<bricks < g ? bricks : g, FX_Z2_THREADS, smem, s>>>(B, phase, launch, zc);
-}
-
-bool fx_launch_jacobi_tb(cudaStream_t s, int pmode, int k, const FxBatchDev* B, int bricks, int phase, int launch, int zc,
-                         bool tma) {
-    switch (k) {
-        case 2:  // two sweeps per pass: the z-marching form
-            if (pmode == FX_TB_F32 && tma) launch_zm2t(s, B, bricks, phase, launch, zc);
-            else if (pmode == FX_TB_F32) launch_zm2<float, false>(s, B, bricks, phase, launch, zc);
-            else if (pmode == FX_TB_F16_ROUND) launch_zm2<__half, true>(s, B, bricks, phase, launch, zc);
-            else launch_zm2<__half, false>(s, B, bricks, phase, launch, zc);
-            return true;
-    }
-    return false;
+void fx_launch_jacobi_two(cudaStream_t s, bool half, const FxBatchDev* B, int bricks, int phase, int launch, int zc, bool tma,
+                          bool two) {
+    if (half && two) launch_zs<__half, true, false>(s, B, bricks, phase, launch, zc);
+    else if (half) launch_zs<__half, false, false>(s, B, bricks, phase, launch, zc);
+    else if (tma && two) launch_zs<float, true, true>(s, B, bricks, phase, launch, zc);
+    else if (tma) launch_zs<float, false, true>(s, B, bricks, phase, launch, zc);
+    else if (two) launch_zs<float, true, false>(s, B, bricks, phase, launch, zc);
+    else launch_zs<float, false, false>(s, B, bricks, phase, launch, zc);
 }
 
 template <typename PT, int VARIANT>
@@ -1114,4 +1104,8 @@ void fx_launch_upload_batch(cudaStream_t s, const FxBatchDev& host, FxBatchDev* 
 
 void fx_launch_check_div(cudaStream_t s, float d, float rcp, float lo, float hi, unsigned long long* mismatches) {
     fxk_check_div<<<num_sms() * 16, 256, 0, s>>>(d, rcp, lo, hi, mismatches);
+}
+
+void fx_launch_check_div_two(cudaStream_t s, float d, float rh, float rl, float lo, double rcp, unsigned long long* mismatches) {
+    fxk_check_div_two<<<num_sms() * 16, 256, 0, s>>>(d, rh, rl, lo, rcp, mismatches);
 }

@@ -666,6 +666,131 @@ FXD float4 fx_jacobi4(const FxJacobiConst2& c, float l, float4 pc, float r, floa
     }
 }
 
+// ---- the update of the strip kernels (fx_jacobi_zs.cuh) -------------------------------------
+// Division by the constant d > 0 in two operations: with 1/d = rh + rl (two floats, rl > 0),
+// RN(x rh + RN(x rl)) (N. Brisebarre and J.-M. Muller, "Correctly rounded multiplication by
+// arbitrary precision constants", IEEE Trans. Computers 57(2), 2008). The engine enables it for
+// a d only after checking on the device that it equals x / d for every float x, with quotients
+// of 0 < |x| < lo taken by fx_div_small; of 1,450 denominators of grids tried it is exact for
+// 1,428 with one of five roundings of rl. rl > 0 keeps zeros' signs, infinities and NaN.
+//
+// RN(x / d) for any finite x through double precision: the product by rcp = RN(1/d) with one
+// correction step is the correctly rounded double quotient, whose rounding to float is x / d
+// (53 >= 2 * 24 + 2 bits). Zeros, infinities and NaN are returned as they are.
+FXD float fx_div_small(float x, double d, double rcp) {
+    const double q = __dmul_rn((double)x, rcp);
+    const float r = (float)__fma_rn(__fma_rn(-q, d, (double)x), rcp, q);
+    return x == 0.0f || !(fabsf(x) <= 3.402823466e38f) ? x : r;
+}
+FXD float fx_div_two(float x, float rh, float rl, float lo, double d, double rcp) {
+    const float r = __fmaf_rn(x, rh, __fmul_rn(x, rl));
+    return fabsf(x) < lo ? fx_div_small(x, d, rcp) : r;
+}
+
+// Jacobi constants of the strip update. TWO: the two-operation quotient; otherwise Markstein's
+// step or the IEEE division, as in fx_jacobi4.
+template <bool TWO>
+struct FxJacobiK {
+    float wx, wy, wz, nz, rh, rl, lo, denom;
+    double rcpD;
+    bool fast;
+};
+template <bool TWO>
+FXD FxJacobiK<TWO> fx_jacobi_k(const FxSimDev& S) {
+    FxJacobiK<TWO> k;
+    k.wx = S.jc[0];
+    k.wy = S.jc[1];
+    k.wz = S.jc[2];
+    k.denom = S.jc[3];
+    k.rh = TWO ? S.jcRh : S.jcRcp;
+    k.rl = TWO ? S.jcRl : -S.jc[3];
+    k.lo = TWO ? S.jcLo : 1.2621774483536189e-29f;
+    k.rcpD = S.jcRcpD;
+    k.fast = TWO || S.jcFastDiv != 0;
+    k.nz = -0.0f * fabsf(k.denom);  // a run-time -0 (see fx_jacobi4)
+    return k;
+}
+struct FxQuad {  // four consecutive x cells as two pairs
+    float2 a, b;
+};
+FXD FxQuad fx_quad(float4 v) { return FxQuad{make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
+FXD FxQuad fx_quad_zero() { return fx_quad(make_float4(0.0f, 0.0f, 0.0f, 0.0f)); }
+FXD float2 fx_bcast2(float v) { return make_float2(v, v); }
+// Numerators of four consecutive cells of one sweep, the operations of fx_jacobi_numerator cell by
+// cell: c holds the cells, l and r their outer x neighbours, b/t/k/f the y-1, y+1, z-1, z+1
+// rows, d the divergence. The x sums are scalar (their operands straddle the pairs, which packed
+// adds would first have to shuffle together).
+template <bool TWO>
+FXD FxQuad fx_jacobi_numerators(const FxJacobiK<TWO>& K, float l, const FxQuad& c, float r, const FxQuad& b, const FxQuad& t,
+                                const FxQuad& k, const FxQuad& f, const FxQuad& d) {
+    const float2 wx = fx_bcast2(K.wx), wy = fx_bcast2(K.wy), wz = fx_bcast2(K.wz), nz = fx_bcast2(K.nz);
+    const float2 la = make_float2(__fadd_rn(l, c.a.y), __fadd_rn(c.a.x, c.b.x));
+    const float2 lb = make_float2(__fadd_rn(c.a.y, c.b.y), __fadd_rn(c.b.x, r));
+    FxQuad n;
+    n.a = __fadd2_rn(__ffma2_rn(wx, la, nz), __ffma2_rn(wy, __fadd2_rn(b.a, t.a), nz));
+    n.b = __fadd2_rn(__ffma2_rn(wx, lb, nz), __ffma2_rn(wy, __fadd2_rn(b.b, t.b), nz));
+    n.a = __fadd2_rn(n.a, __ffma2_rn(wz, __fadd2_rn(k.a, f.a), nz));
+    n.b = __fadd2_rn(n.b, __ffma2_rn(wz, __fadd2_rn(k.b, f.b), nz));
+    n.a = __fadd2_rn(n.a, make_float2(-d.a.x, -d.a.y));
+    n.b = __fadd2_rn(n.b, make_float2(-d.b.x, -d.b.y));
+    return n;
+}
+// Their quotients by the denominator, right for |numerator| >= K.lo and for zeros (TWO), or for
+// K.lo <= |numerator| <= FLT_MAX.
+template <bool TWO>
+FXD FxQuad fx_jacobi_quotients(const FxJacobiK<TWO>& K, const FxQuad& n) {
+    const float2 rh = fx_bcast2(K.rh), rl = fx_bcast2(K.rl);
+    FxQuad q;
+    if (TWO) {
+        q.a = __ffma2_rn(n.a, rh, __fmul2_rn(n.a, rl));
+        q.b = __ffma2_rn(n.b, rh, __fmul2_rn(n.b, rl));
+    } else {  // Markstein: q = x rcp, e = x - q d, q + e rcp
+        const float2 qa = __fmul2_rn(n.a, rh), qb = __fmul2_rn(n.b, rh);
+        q.a = __ffma2_rn(__ffma2_rn(qa, rl, n.a), rh, qa);
+        q.b = __ffma2_rn(__ffma2_rn(qb, rl, n.b), rh, qb);
+    }
+    return q;
+}
+template <bool TWO>
+FXD FxQuad fx_jacobi_small(const FxJacobiK<TWO>& K, const FxQuad& n) {
+    const double D = K.denom;
+    return FxQuad{make_float2(fx_div_small(n.a.x, D, K.rcpD), fx_div_small(n.a.y, D, K.rcpD)),
+                  make_float2(fx_div_small(n.b.x, D, K.rcpD), fx_div_small(n.b.y, D, K.rcpD))};
+}
+FXD bool fx_odd4(const FxQuad& n) {  // an infinity or NaN among them
+    const float m = 3.402823466e38f;
+    return !(fabsf(n.a.x) <= m && fabsf(n.a.y) <= m && fabsf(n.b.x) <= m && fabsf(n.b.y) <= m);
+}
+// Whether a numerator of n is outside the range its quotient was checked for (lo < 0: the
+// quad's result is not used).
+template <bool TWO>
+FXD bool fx_jacobi_rare(const FxJacobiK<TWO>& K, float lo, const FxQuad& n) {
+    const float least = fminf(fminf(fabsf(n.a.x), fabsf(n.a.y)), fminf(fabsf(n.b.x), fabsf(n.b.y)));
+    bool bad = least < lo;
+    if (!TWO) bad = bad || (lo > 0.0f && (!K.fast || fx_odd4(n)));
+    return bad;
+}
+// The quotients of two quads, guarded by one warp-uniform test: numerators too small for the
+// checked operations, which only the fronts of a spreading solve have, take the quotient through
+// double precision.
+template <bool TWO>
+FXD void fx_jacobi_divide2(const FxJacobiK<TWO>& K, float lo1, float lo2, const FxQuad& n1, const FxQuad& n2, FxQuad& q1,
+                           FxQuad& q2) {
+    q1 = fx_jacobi_quotients<TWO>(K, n1);
+    q2 = fx_jacobi_quotients<TWO>(K, n2);
+    if (__any_sync(0xffffffffu, fx_jacobi_rare<TWO>(K, lo1, n1) || fx_jacobi_rare<TWO>(K, lo2, n2))) {
+        q1 = fx_jacobi_small<TWO>(K, n1);
+        q2 = fx_jacobi_small<TWO>(K, n2);
+    }
+}
+// One cell.
+template <bool TWO>
+FXD float fx_jacobi_cell(const FxJacobiK<TWO>& K, float l, float r, float b, float t, float k, float f, float div) {
+    const float n = fx_jacobi_numerator(FxJacobiConst{K.wx, K.wy, K.wz, K.denom}, l, r, b, t, k, f, div);
+    if (TWO) return fx_div_two(n, K.rh, K.rl, K.lo, K.denom, K.rcpD);
+    return fx_div_small(n, K.denom, K.rcpD);
+}
+
 // One cell of fx_jacobi4 (the same numerator; the checked constant division when enabled).
 FXD float fx_jacobi1(const FxJacobiConst2& c, float l, float r, float b, float t, float k, float f, float div) {
     const float n = fx_jacobi_numerator(FxJacobiConst{c.wxS, c.wyS, c.wzS, c.denom}, l, r, b, t, k, f, div);

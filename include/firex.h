@@ -336,15 +336,16 @@ int firex_set_graphs(firex_sim* sim, int32_t on);
  *   ZMARCH    — x-y tiles marching z through a cp.async shared-memory ring (one read of
  *               each value per sweep: best once the grid outgrows L2);
  *   FUSED     — two sweeps per launch (`block` 2): z-marching tiles with a one-cell ring,
- *               one read of pressure and divergence per two sweeps (AUTO's choice at 8 Mi
+ *               one read of pressure and divergence per two sweeps (AUTO's choice at 2 Mi
  *               cells and above). The fused sweeps give the same results as single sweeps
  *               (with FP16 pressure storage the first sweep is rounded as a stored one). A
- *               phase falls back to single sweeps when the fused launches would leave its
- *               result in the other buffer of the pair (half its sweep count, rounded down,
- *               is odd).
- * `zchunk`: z planes per CTA for ZMARCH and FUSED (0 = auto). AUTO takes RESIDENT when the
- * batch fits on chip, else by its cell count: UNBLOCKED below 8 Mi cells, FUSED with block 2
- * and 16-plane chunks below 16 Mi, FUSED with block 2 and 64-plane chunks from 16 Mi. */
+ *               phase runs an even number of fused launches and its last sweeps, up to three,
+ *               one by one, so that its result lands in the buffer of the pair that single
+ *               sweeps leave it in.
+ * `zchunk`: z planes per CTA for ZMARCH and FUSED (0 = auto: FUSED fits them to the device,
+ * firex_diagnostics.jacobi_zrun). AUTO takes RESIDENT when the batch fits on chip, else by its
+ * cell count: UNBLOCKED below 2 Mi cells, FUSED with block 2 and 16-plane chunks below 16 Mi,
+ * FUSED with block 2 and 64-plane chunks from 16 Mi. */
 #define FIREX_JACOBI_AUTO 0
 #define FIREX_JACOBI_UNBLOCKED 1
 #define FIREX_JACOBI_ZMARCH 2
@@ -363,8 +364,9 @@ int firex_batch_set_jacobi(firex_batch* batch, int32_t kernel, int32_t block, in
 /* How the two-sweep pass (FUSED, block 2) brings its pressure and divergence planes into
  * shared memory. TMA (FP32 pressure only): one elected thread per CTA issues tiled tensor
  * loads (cp.async.bulk.tensor) completing on per-slot mbarriers. CPASYNC: per-thread cp.async
- * copies. Both give the same results bit for bit. AUTO (the default) = CPASYNC, measured
- * faster on B200; FP16 pressure (branch B) always uses CPASYNC. A batch's own setting overrides
+ * copies. Both give the same results bit for bit. AUTO (the default) = TMA where AUTO also
+ * chose the pass, CPASYNC where the caller asked for it; FP16 pressure (branch B) always uses
+ * CPASYNC. A batch's own setting overrides
  * its members' (AUTO: the first member's). No reference counterpart (the reference's tiled
  * solve stages through workgroup memory, shaders.ts:405-459). */
 #define FIREX_STAGING_AUTO 0
@@ -393,7 +395,7 @@ int firex_batch_set_tiles(firex_batch* batch, int32_t simulate_by, int32_t proje
 typedef struct firex_diagnostics {
     int32_t fast_division;    /* 1: the Jacobi division uses the checked constant-divisor path */
     int32_t jacobi_block;     /* sweeps fused per Jacobi launch (1: one sweep per launch) */
-    int32_t jacobi_zchunk;    /* z planes per CTA of the Jacobi launches */
+    int32_t jacobi_zchunk;    /* z planes per CTA of the Jacobi launches, as asked for or by AUTO's rule */
     int32_t graph;            /* 1: steps replay a captured CUDA graph */
     int32_t launches_per_step;
     int32_t jacobi_kernel;    /* FIREX_JACOBI_* kernel the last step ran */
@@ -402,7 +404,8 @@ typedef struct firex_diagnostics {
     int32_t simulate_by;      /* source-pass bricks of 32 x simulate_by x (8 / simulate_by) cells */
     int32_t project_fused;    /* 1: the primary projection and the residual divergence ran as one pass */
     int32_t project_resident; /* 1: the residual projection ran inside the resident Jacobi's launch */
-    int32_t reserved[5];
+    int32_t jacobi_zrun;      /* z planes per CTA the two-sweep launches took (AUTO fits them to the device) */
+    int32_t reserved[4];
 } firex_diagnostics;
 int firex_get_diagnostics(const firex_sim* sim, firex_diagnostics* out);
 

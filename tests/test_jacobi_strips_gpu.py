@@ -1,0 +1,76 @@
+"""GPU tests of the two-sweep Jacobi pass by strips (fx_jacobi_zs.cuh) where it can go wrong: grids
+one tile (32 x 14 cells) wide and high and one group or row beside it, single-group rows, chunks
+of one plane and of the whole grid, both stagings, FP16 pressure, sweep counts that leave one to
+three single sweeps, and solves that start from rest, whose fronts are below the range of the
+two-operation quotient. Every case must equal single sweeps bit for bit."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from fire_b200 import _abi as A
+from fire_b200.sim import FireXSim
+from oracle.oracle import OracleSim
+from tests.helpers import DT, sphere_options
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("flow", "species", "pressure", "reaction", "divergence", "correction")
+
+
+def same(a, b):
+    assert a.state == b.state
+    for f in FIELDS:
+        x, y = a.read(f), b.read(f)
+        assert np.array_equal(x, y), (f, float(np.abs(x.astype(np.float64) - y).max()))
+
+
+def pair(dims, steps=2, zc=0, staging=A.STAGING_AUTO, **kw):
+    one, two = FireXSim(dims, sphere_options(dims, **kw)), FireXSim(dims, sphere_options(dims, **kw))
+    one.set_jacobi("unblocked")
+    two.set_jacobi("fused", 2, zc)
+    two.set_staging(staging)
+    one.step(steps, DT)
+    two.step(steps, DT)
+    assert two.diagnostics["jacobi_block"] == 2
+    same(one, two)
+    one.close()
+    two.close()
+
+
+@pytest.mark.parametrize("staging", [A.STAGING_CPASYNC, A.STAGING_TMA])
+@pytest.mark.parametrize("dims", [(4, 12, 4), (8, 16, 4), (28, 28, 8), (32, 12, 8), (32, 28, 12), (36, 32, 8), (68, 16, 20)])
+def test_tile_edges(dims, staging):
+    for zc in (1, 7, 64):
+        pair(dims, zc=zc, staging=staging, P=8, R=8)
+
+
+@pytest.mark.parametrize("dims", [(4, 12, 4), (36, 16, 12), (100, 44, 8)])
+def test_tile_edges_fp16_pressure(dims):
+    pair(dims, zc=5, P=8, R=8, pressure_mode=A.PRESSURE_F16)
+
+
+@pytest.mark.parametrize("P,R", [(4, 5), (6, 7), (13, 10)])
+def test_remaining_single_sweeps(P, R):
+    pair((36, 32, 20), P=P, R=R)
+
+
+@pytest.mark.parametrize("mode", [A.PRESSURE_WARM_F32, A.PRESSURE_COLD_F32])
+def test_fronts_of_a_solve_from_rest(mode):
+    # no noise: the pressure spreads from the emitter through cells at rest and decays by about a
+    # factor of six a cell, below the smallest float within the grid
+    for staging in (A.STAGING_CPASYNC, A.STAGING_TMA):
+        pair((64, 96, 64), zc=16, staging=staging, P=48, R=40, noise=0.0, pressure_mode=mode)
+
+
+def test_auto_on_a_grid_beyond_the_chip_equals_single_sweeps_and_the_oracle():
+    dims = (256, 144, 128)
+    opts = sphere_options(dims, P=8, R=9)
+    auto, one, o = FireXSim(dims, opts), FireXSim(dims, opts), OracleSim(dims, opts)
+    one.set_jacobi("unblocked")
+    for s in (auto, one, o):
+        s.step(2, 0.0)
+    d = auto.diagnostics
+    assert d["jacobi_kernel"] == A.JACOBI_FUSED and d["jacobi_staging"] == A.STAGING_TMA, d
+    same(auto, one)
+    same(auto, o)
