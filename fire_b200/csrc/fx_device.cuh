@@ -205,6 +205,8 @@ enum FxShape {
 // full x rows, nby x nbz of them (CTA b owns box (b % nby, b / nby)).
 struct FxResBox {
     int by, bz, nby, nbz;
+    int exOff;  // variant 4: the member's first packet (16 bytes) in the batch's exchange buffer
+    int pad[3];
 };
 // CELL: 32 x BY x (8 / BY) cells, one thread per cell (simulate); BY = FX_CELL_BY unless
 //       the plan tunes it (firex_set_tiles).
@@ -222,7 +224,9 @@ struct FxBatchDev {
     int nsims;
     int pad;
     int total[FX_NSHAPES];
-    int colTileX, colTileY;        // interior tile of the COL shape
+    unsigned* ex;                  // exchange buffer of the resident Jacobi's variant 4: [0] the tag
+                                   // its packets start from in this step, the packets from [32]
+    int exPhase, exStep;           // tags of the residual phase and of the next step, from there
     FxSimDev* sims[FX_MAX_BATCH];
     int start[FX_NSHAPES][FX_MAX_BATCH + 1];
     FxResBox res[FX_MAX_BATCH];

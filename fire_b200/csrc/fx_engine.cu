@@ -24,6 +24,7 @@
 
 #include "../../include/firex.h"
 #include "fx_internal.h"
+#include "fx_jacobi_reg.cuh"
 #include "fx_jacobi_res.cuh"
 #include "fx_jacobi_zm.cuh"
 #include "fx_jacobi_zs.cuh"
@@ -141,13 +142,14 @@ struct StepPlan {
     bool projDiv = true;      // the primary projection and the residual divergence in one pass
     bool res = false;         // every sweep of a phase in one resident launch
     int resVariant = 0;       // ... by this variant of the kernel
+    bool resReg = false;      // ... with the pressure in registers (variant 4)
     int resSmem = 0;          // its dynamic shared memory per CTA
     bool projRes = false;     // the residual projection inside the resident launch (variant 4)
     bool simEarly = false;    // the source pass evaluates its neighbour terms before the advection
     int bricks[FX_NSHAPES] = {};
     auto key() const {
         return std::tie(storage, half, maxP, maxR, k, zc, zrun, zmZc, row4, fuseP, fuseR, pack, tma, two, simBy, projDiv, res,
-                        resVariant, resSmem, projRes, simEarly,
+                        resVariant, resReg, resSmem, projRes, simEarly,
                         bricks[0],
                         bricks[1], bricks[2], bricks[3], bricks[4], bricks[5], bricks[6]);
     }
@@ -177,8 +179,8 @@ void enqueue_jacobi_phase(cudaStream_t st, const StepPlan& pl, FxBatchDev* B, in
     const int n = phase == 0 ? pl.maxP : pl.maxR;
     if (pl.res) {  // a failed launch is reported by the caller's cudaGetLastError
         if (n > 0)
-            fx_launch_jacobi_res(st, pl.half, pl.resVariant, B, pl.bricks[FX_SHAPE_RES], phase, pl.resSmem,
-                                 phase == 1 && pl.projRes);
+            fx_launch_jacobi_res(st, FxResKernel{pl.resVariant, pl.half, pl.resReg}, B, pl.bricks[FX_SHAPE_RES], phase, pl.resSmem,
+                                 phase == 1 && pl.projRes, pl.two);
         return;
     }
     const bool fuse = phase == 0 ? pl.fuseP : pl.fuseR;
@@ -236,7 +238,45 @@ void default_jacobi(long long cells, int* kernel, int* k, int* zc) {
 //   variant 0 (columns): thread columns of (x group, row), by * X / 4 <= T, each split into
 //     parts along z; at most FX_RES_MAXG planes per column part.
 // False when no box fits one CTA's shared memory and registers.
+//   variant 4 (registers): boxes of strips of four rows, their columns split along z
+//     (fx_reg_geom), at most FX_REG_MAXZ planes to a thread.
+long long reg_smem(int X, int Y, int Z, const FxResBox& bx) {
+    long long most = 0;
+    for (int iz = 0; iz < bx.nbz; ++iz)
+        for (int iy : {0, bx.nby - 1}) {
+            const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, iz * bx.nby + iy);
+            if (g.cols > FX_REG_THREADS || g.len > FX_REG_MAXZ || g.cols * g.parts > FX_REG_THREADS) return -1;
+            if (2 * (g.ny + g.nz) * (X / 4) > FX_REG_MAXH * FX_REG_THREADS) return -1;
+            most = std::max(most, fx_reg_smem_bytes(X, g));
+        }
+    return most;
+}
+bool reg_box(int X, int Y, int Z, int m, FxResBox* out) {
+    bool found = false;
+    double best = 0;
+    for (int by = 2; by <= Y; by += 2) {
+        const int nby = (Y + by - 1) / by;
+        if (nby > m || nby > FX_RES_MAX_CTAS) continue;
+        if ((X / 4) * (by / 2) > FX_REG_THREADS) break;
+        const int nbz = std::min(Z, std::min(m, FX_RES_MAX_CTAS) / nby);
+        FxResBox bx{by, (Z + nbz - 1) / nbz, nby, nbz, 0, {0, 0, 0}};
+        const long long smem = reg_smem(X, Y, Z, bx);
+        if (smem < 0 || smem > FX_RES_SMEM_MAX) continue;
+        const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, (nbz - 1) * nby);
+        // cycles of a sweep, roughly: the warps' issue slots or one warp's chain, and the faces
+        const double warps = (g.cols * g.parts + 31) / 32;
+        const double cost = std::max(warps * g.len * 2 * 25.0, g.len * 2 * 100.0) + 2.0 * (by + bx.bz) * (X / 4) / FX_REG_THREADS * 100.0;
+        if (!found || cost < best) {
+            found = true;
+            best = cost;
+            *out = bx;
+        }
+    }
+    return found;
+}
+constexpr int kRegVariant = 5;  // variant 4 with the pressure in registers
 bool res_box(int X, int Y, int Z, int m, int variant, FxResBox* out) {
+    if (variant == kRegVariant) return reg_box(X, Y, Z, m, out);
     const long long gx = X / 4;
     bool found = false;
     double best = 0;
@@ -284,7 +324,7 @@ bool res_box(int X, int Y, int Z, int m, int variant, FxResBox* out) {
         if (!found || cost < best) {
             found = true;
             best = cost;
-            *out = FxResBox{by, bz, nby, (Z + bz - 1) / bz};
+            *out = FxResBox{by, bz, nby, (Z + bz - 1) / bz, 0, {0, 0, 0}};
         }
     }
     return found;
@@ -332,7 +372,8 @@ bool res_assign(const std::vector<std::array<int, 3>>& dims, int cap, int varian
     *smem = 0;
     for (size_t i = 0; i < n; ++i) {
         res_box(dims[i][0], dims[i][1], dims[i][2], t[i], variant, &(*boxes)[i]);
-        *smem = std::max(*smem, (int)fx_res_smem_bytes(dims[i][0], (*boxes)[i].by, (*boxes)[i].bz));
+        *smem = std::max(*smem, (int)(variant == kRegVariant ? reg_smem(dims[i][0], dims[i][1], dims[i][2], (*boxes)[i])
+                                                   : fx_res_smem_bytes(dims[i][0], (*boxes)[i].by, (*boxes)[i].bz)));
     }
     return true;
 }
@@ -434,6 +475,91 @@ static TwoOpReciprocal two_op_reciprocal(int device, float d) {
     cache[{device, bits}] = r;
     return r;
 }
+
+// Exchange buffers of the resident Jacobi between batches: a step of a new handle would otherwise
+// pay for the allocation (0.3 ms at 64x96x64, more than the step). Holds at most kPoolBytes and
+// nothing once no batch is left; the buffers of a batch are free of work when they come back.
+namespace {
+constexpr size_t kPoolBytes = 64u << 20;
+struct ExchangePool {
+    struct Buffer {
+        int device;
+        unsigned* p;
+        size_t bytes;
+    };
+    std::mutex mu;
+    std::vector<Buffer> idle;
+    size_t held = 0;
+    int batches = 0;
+
+    // Takes a buffer of the current device of at least `need` bytes; *bytes is its size. NULL: none to be had.
+    unsigned* take(int device, size_t need, size_t* bytes) {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            size_t best = idle.size();
+            for (size_t i = 0; i < idle.size(); ++i)
+                if (idle[i].device == device && idle[i].bytes >= need && (best == idle.size() || idle[i].bytes < idle[best].bytes)) best = i;
+            if (best < idle.size()) {
+                const Buffer b = idle[best];
+                idle.erase(idle.begin() + best);
+                held -= b.bytes;
+                *bytes = b.bytes;
+                return b.p;
+            }
+        }
+        unsigned* p = nullptr;
+        if (cudaMalloc(&p, need) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        *bytes = need;
+        return p;
+    }
+    // Gives a buffer back; the caller has waited for the work that used it.
+    void give(int device, unsigned* p, size_t bytes) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (batches > 0 && held + bytes <= kPoolBytes) {
+                idle.push_back(Buffer{device, p, bytes});
+                held += bytes;
+                return;
+            }
+        }
+        cudaFree(p);
+    }
+    void enter() {
+        std::lock_guard<std::mutex> lock(mu);
+        ++batches;
+    }
+    void leave() {
+        std::vector<Buffer> last;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (--batches > 0) return;
+            last.swap(idle);
+            held = 0;
+        }
+        release(last);
+    }
+    void trim() {  // before an allocation that does not fit
+        std::vector<Buffer> all;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            all.swap(idle);
+            held = 0;
+        }
+        release(all);
+    }
+    static void release(const std::vector<Buffer>& v) {
+        for (const Buffer& b : v) {
+            DeviceGuard dg(b.device);
+            cudaFree(b.p);
+        }
+    }
+};
+ExchangePool g_exchange;
+}  // namespace
 
 // ---- one simulation ------------------------------------------------------------------------
 struct firex_sim {
@@ -676,8 +802,11 @@ struct firex_batch {
     int tableRes = -1;                               // whether resident boxes were requested
     std::vector<char> tableWater;                    // which members sprayed when the table was filled
     bool resOk = false;                              // ... and the batch fits one resident launch
-    int resVariant = 0;                              // ... of this kernel variant
+    FxResKernel resKernel{};                         // ... of this kernel
     int resSmem = 0;
+    unsigned* ex = nullptr;                          // variant 4's exchange buffer
+    size_t exBytes = 0;
+    bool counted = false;                            // among the pool's batches
     std::string err;
 
     // per-pass profiling (events between passes; graphs are bypassed while profiling)
@@ -700,6 +829,33 @@ struct firex_batch {
         tableDirty = true;
     }
 
+    // The exchange buffer of the resident Jacobi's variant 4 for these boxes, every tag cleared:
+    // kept by the batch and grown when a plan needs more (16 bytes a face cell, about 16 MB for a
+    // grid that fills the device). False when it cannot be had: another variant then runs.
+    bool ensure_exchange(const std::vector<std::array<int, 3>>& dims, std::vector<FxResBox>& boxes) {
+        size_t packets = 0;
+        int maxP = 0, maxR = 0;
+        for (size_t i = 0; i < boxes.size(); ++i) {
+            boxes[i].exOff = (int)packets;
+            packets += (size_t)boxes[i].nby * boxes[i].nbz * 2 * 2 * fx_reg_outbox_quads(dims[i][0], boxes[i]);
+            maxP = std::max(maxP, members[i]->h.P);
+            maxR = std::max(maxR, members[i]->h.R);
+        }
+        const size_t need = 128 + packets * 16;
+        if (need > exBytes) {
+            if (cudaStreamSynchronize(stream) != cudaSuccess) return false;
+            g_exchange.give(device, ex, exBytes);
+            exBytes = 0;
+            ex = g_exchange.take(device, need, &exBytes);
+            if (!ex) return false;
+        }
+        if (cudaMemsetAsync(ex, 0, need, stream) != cudaSuccess) return false;
+        h->ex = ex;
+        h->exPhase = maxP + 2;
+        h->exStep = maxP + maxR + 8;
+        return true;
+    }
+
     // Fills the brick prefix sums for the launch shape (k, zc); resident boxes when wanted,
     // of variant resForce when that is 0-4.
     void fill_table(int k, int zc, int zmZc, bool wantRes, int resForce, int simBy, bool tma) {
@@ -707,20 +863,22 @@ struct firex_batch {
         h->nsims = (int)members.size();
         std::vector<FxResBox> boxes;
         resOk = false;
+        h->ex = nullptr;
         if (wantRes && !members.empty()) {
             std::vector<std::array<int, 3>> dims;
             for (firex_sim* s : members) dims.push_back({s->X, s->Y, s->Z});
-            // the first variant every member fits: faces first with interior columns and a
-            // copy warp (FP32 pressure; 6.0 against 7.6 us per sweep at HD on B200), the same
-            // without the copy warp (long columns only), faces first (small-box instance
-            // first), then the column variant
-            for (int v : {4, 3, 2, 1, 0}) {
-                if (resForce >= 0 && v != resForce) continue;
-                if (v == 4 && members[0]->half) continue;  // the copy warp moves FP32 rows
-                const int cap = fx_res_capacity(members[0]->half, v);
+            // the first variant every member fits: pressure in registers (FP32, short columns), faces
+            // first with interior columns and a copy warp (FP32), the same without the copy warp
+            // (long columns only), faces first (small-box instance first), then the column variant
+            for (int v : {kRegVariant, 4, 3, 2, 1, 0}) {
+                const FxResKernel kernel{std::min(v, 4), members[0]->half, v == kRegVariant};
+                if (resForce >= 0 && kernel.variant != resForce) continue;
+                if (kernel.half && kernel.variant == 4) continue;  // FP32 rows only
+                const int cap = fx_res_capacity(kernel);
                 if (res_assign(dims, cap, v, &boxes, &resSmem)) {
+                    if (kernel.reg && !ensure_exchange(dims, boxes)) continue;
                     resOk = true;
-                    resVariant = v;
+                    resKernel = kernel;
                     break;
                 }
             }
@@ -871,14 +1029,15 @@ struct firex_batch {
         p.res = wantRes && resOk;
         if (p.res) {
             p.resSmem = resSmem;
-            p.resVariant = resVariant;
+            p.resVariant = resKernel.variant;
+            p.resReg = resKernel.reg;
             p.k = 1;
             p.fuseP = p.fuseR = false;
             p.tma = false;
             // the residual projection as variant 4's epilogue (unless the projection passes are
             // asked to run separately): every member runs residual sweeps, and every top box has
             // two rows or more (its top row projects the row below from the box)
-            bool epi = FX_PROJ_RES && resVariant == 4 && pf != FIREX_PROJECT_SEPARATE;
+            bool epi = FX_PROJ_RES && p.resVariant == 4 && pf != FIREX_PROJECT_SEPARATE;
             for (size_t i = 0; i < members.size() && epi; ++i) {
                 const FxResBox& bx = h->res[i];
                 epi = members[i]->h.R >= 1 && members[i]->Y - (bx.nby - 1) * bx.by >= 2;
@@ -1053,7 +1212,12 @@ struct firex_batch {
         for (cudaEvent_t e : evPool) cudaEventDestroy(e);
         evPool.clear();
         if (d) cudaFree(d);
+        g_exchange.give(device, ex, exBytes);
+        if (counted) g_exchange.leave();
+        counted = false;
         d = nullptr;
+        ex = nullptr;
+        exBytes = 0;
         delete h;
         h = nullptr;
         if (stream) cudaStreamDestroy(stream);
@@ -1075,6 +1239,8 @@ struct firex_batch {
             delete b;
             return nullptr;
         }
+        g_exchange.enter();
+        b->counted = true;
         b->rebuild_table();
         return b;
     }
@@ -1366,6 +1532,10 @@ int firex_create(const int32_t dims[3], const firex_options* opt, firex_sim** ou
     }
     size_t freeB = 0, totalB = 0;
     if (cudaMemGetInfo(&freeB, &totalB) == cudaSuccess && need > freeB) {
+        g_exchange.trim();
+        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) freeB = need;
+    }
+    if (totalB > 0 && need > freeB) {
         g_create_error = "grid needs " + std::to_string(need) + " device bytes, " + std::to_string(freeB) + " free";
         s->release();
         delete s;

@@ -38,13 +38,17 @@ void fx_launch_project(cudaStream_t s, bool half, const FxBatchDev* B, int brick
 void fx_launch_project_div(cudaStream_t s, bool half, const FxBatchDev* B, int bricks);
 // Every sweep of a phase in one cooperative launch of `ctas` CTAs with `smem` bytes of
 // dynamic shared memory (fx_jacobi_res.cuh; variant 0 column, 1 faces-first, 2 faces-first
-// for small boxes, 3 faces-first with interior columns, 4 variant 3 with a copy warp);
-// fx_res_capacity: the most CTAs of that variant one such launch can hold resident on this
-// device (0 when unavailable). epi (variant 4, residual phase): the launch also projects the
-// flow with the final correction (fx_res_project_epi), replacing fx_launch_project's phase 1.
-cudaError_t fx_launch_jacobi_res(cudaStream_t s, bool half, int variant, const FxBatchDev* B, int ctas, int phase,
-                                 int smem, bool epi);
-int fx_res_capacity(bool half, int variant);
+// for small boxes, 3 faces-first with interior columns, 4 with FP32 pressure: variant 3 with a
+// copy warp, or (reg) the pressure in registers for short columns, fx_jacobi_reg.cuh).
+// epi (variant 4, residual phase): the launch also projects the flow with the final correction,
+// replacing fx_launch_project's phase 1. two (reg): fx_launch_jacobi_two's.
+struct FxResKernel {
+    int variant;
+    bool half, reg;
+};
+int fx_res_capacity(const FxResKernel& k);  // the most CTAs one such launch can hold resident (0: none)
+cudaError_t fx_launch_jacobi_res(cudaStream_t s, const FxResKernel& k, const FxBatchDev* B, int ctas, int phase, int smem, bool epi,
+                                 bool two);
 
 // Single-simulation utilities.
 void fx_launch_init(cudaStream_t s, int storage, const FxSimDev* S, float tAmbient, float oxygen, float noise);

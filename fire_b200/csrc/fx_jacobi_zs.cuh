@@ -207,10 +207,15 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
             rare = rare || fx_jacobi_rare<TWO>(K, !stored || st[i] ? lo[i] : -1.0f, n[i]);
         }
         // numerators too small for the checked quotients, which only the fronts of a spreading
-        // solve have: through double precision
+        // solve have: through double precision (zeros, as everywhere in a fluid at rest, are not)
         if (__any_sync(0xffffffffu, rare)) {
+            bool tiny = !TWO;
 #pragma unroll
-            for (int i = 0; i < ROWS; ++i) q[i] = fx_jacobi_small<TWO>(K, n[i]);
+            for (int i = 0; i < ROWS; ++i) tiny = tiny || fx_jacobi_tiny(!stored || st[i] ? lo[i] : -1.0f, n[i]);
+            if (__any_sync(0xffffffffu, tiny)) {
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i) q[i] = fx_jacobi_small<TWO>(K, n[i]);
+            }
         }
 #pragma unroll
         for (int i = 0; i < ROWS; ++i)

@@ -15,6 +15,7 @@
 #include <mutex>
 
 #include "fx_internal.h"
+#include "fx_jacobi_reg.cuh"
 #include "fx_jacobi_res.cuh"
 #include "fx_sph.cuh"
 #include "fx_jacobi_zm.cuh"
@@ -51,6 +52,7 @@ __global__ void fxk_step_begin(FxBatchDev* __restrict__ B) {
 // Counters after the step (renderOfflineFrameInternal, FireXEngine.ts:681-682) and the
 // ping-pong parities of encodeSimulationStep (:2172-2275); copyFlow is a parity flip.
 __global__ void fxk_step_end(FxBatchDev* __restrict__ B) {
+    if (threadIdx.x == 0 && B->ex) B->ex[0] += (unsigned)B->exStep;
     for (int s = threadIdx.x; s < B->nsims; s += blockDim.x) {
         FxSimDev* S = B->sims[s];
         if (!S->active) continue;
@@ -780,6 +782,29 @@ __global__ void __launch_bounds__(FX_RES_THREADS, 1) fxk_jacobi_res(const FxBatc
     else fx_res_box_col<PT, sizeof(PT) == 2>(S, B->res[si], b, phase, sm);
 }
 
+// The same with the pressure in registers (fx_jacobi_reg.cuh). EPI (residual phase): the launch
+// also projects the flow with its result.
+template <bool EPI, bool TWO>
+__global__ void __launch_bounds__(FX_REG_THREADS, 1) fxk_jacobi_reg(const FxBatchDev* __restrict__ B, int phase) {
+    extern __shared__ float4 fx_res_smem[];
+    const int w = blockIdx.x;
+    if (w >= B->total[FX_SHAPE_RES]) return;
+    const int si = fx_find_sim(B->start[FX_SHAPE_RES], B->nsims, w);
+    const FxSimDev& S = *B->sims[si];
+    if (!S.active) return;
+    float* sm = reinterpret_cast<float*>(fx_res_smem);
+    const int b = w - B->start[FX_SHAPE_RES][si];
+    const FxResBox bx = B->res[si];
+    const FxRegGeom g = fx_reg_geom(S.X, S.Y, S.Z, bx, b);
+    static_assert(FX_REG_MAXZ == 4, "one instance per column length");
+    switch (g.len) {
+        case 1: return fx_reg_box<1, EPI, TWO>(S, B, bx, g, b, phase, sm);
+        case 2: return fx_reg_box<2, EPI, TWO>(S, B, bx, g, b, phase, sm);
+        case 3: return fx_reg_box<3, EPI, TWO>(S, B, bx, g, b, phase, sm);
+        default: return fx_reg_box<4, EPI, TWO>(S, B, bx, g, b, phase, sm);
+    }
+}
+
 __global__ void fxk_norm_final(const double* __restrict__ partial, int nblocks, double* __restrict__ out) {
     __shared__ double s_ss[256], s_mx[256];
     const int t = threadIdx.x;
@@ -977,46 +1002,50 @@ void fx_launch_jacobi_two(cudaStream_t s, bool half, const FxBatchDev* B, int br
     else launch_zs<float, false, false>(s, B, bricks, phase, launch, zc);
 }
 
-template <typename PT, int VARIANT>
-static const void* res_fn() {
-    return (const void*)fxk_jacobi_res<PT, VARIANT>;
-}
-static const void* res_kernel(bool half, int variant) {
+template <typename PT>
+static const void* res_variant(int variant) {
     switch (variant) {
-        case 4: return half ? nullptr : res_fn<float, 4>();
-        case 1: return half ? res_fn<__half, 1>() : res_fn<float, 1>();
-        case 2: return half ? res_fn<__half, 2>() : res_fn<float, 2>();
-        case 3: return half ? res_fn<__half, 3>() : res_fn<float, 3>();
-        default: return half ? res_fn<__half, 0>() : res_fn<float, 0>();
+        case 1: return (const void*)fxk_jacobi_res<PT, 1>;
+        case 2: return (const void*)fxk_jacobi_res<PT, 2>;
+        case 3: return (const void*)fxk_jacobi_res<PT, 3>;
+        default: return (const void*)fxk_jacobi_res<PT, 0>;
     }
 }
+static const void* res_kernel(const FxResKernel& k, bool epi, bool two) {
+    if (k.variant != 4) return k.half ? res_variant<__half>(k.variant) : res_variant<float>(k.variant);
+    if (k.half) return nullptr;
+    if (!k.reg) return epi ? (const void*)fxk_jacobi_res<float, 4, true> : (const void*)fxk_jacobi_res<float, 4>;
+    if (two) return epi ? (const void*)fxk_jacobi_reg<true, true> : (const void*)fxk_jacobi_reg<false, true>;
+    return epi ? (const void*)fxk_jacobi_reg<true, false> : (const void*)fxk_jacobi_reg<false, false>;
+}
+static int res_threads(const FxResKernel& k) { return k.reg ? FX_REG_THREADS : FX_RES_THREADS; }
 
-// Most CTAs of resident-Jacobi variant `variant` that one cooperative launch can keep
-// resident (0: the variant cannot run, e.g. variant 4 with FP16 pressure).
-int fx_res_capacity(bool half, int variant) {
-    const void* fn = res_kernel(half, variant);
+// Most CTAs of a resident Jacobi that one cooperative launch can keep resident (0: it cannot
+// run, e.g. variant 4 with FP16 pressure).
+int fx_res_capacity(const FxResKernel& k) {
+    const void* fn = res_kernel(k, false, false);
     if (!fn) return 0;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, FX_RES_SMEM_MAX) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, FX_RES_THREADS, FX_RES_SMEM_MAX) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, res_threads(k), FX_RES_SMEM_MAX) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     return per_sm * num_sms();
 }
 
-cudaError_t fx_launch_jacobi_res(cudaStream_t s, bool half, int variant, const FxBatchDev* B, int ctas, int phase,
-                                 int smem, bool epi) {
-    const void* fn = (epi && variant == 4 && !half) ? (const void*)fxk_jacobi_res<float, 4, true> : res_kernel(half, variant);
+cudaError_t fx_launch_jacobi_res(cudaStream_t s, const FxResKernel& k, const FxBatchDev* B, int ctas, int phase, int smem, bool epi,
+                                 bool two) {
+    const void* fn = res_kernel(k, epi, two);
     if (!fn) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, FX_RES_SMEM_MAX);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(FX_RES_THREADS);
+    cfg.blockDim = dim3((unsigned)res_threads(k));
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];

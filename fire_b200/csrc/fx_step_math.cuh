@@ -761,27 +761,23 @@ FXD bool fx_odd4(const FxQuad& n) {  // an infinity or NaN among them
     const float m = 3.402823466e38f;
     return !(fabsf(n.a.x) <= m && fabsf(n.a.y) <= m && fabsf(n.b.x) <= m && fabsf(n.b.y) <= m);
 }
-// Whether a numerator of n is outside the range its quotient was checked for (lo < 0: the
-// quad's result is not used).
+// Whether a numerator of n may be outside the range its quotient was checked for (lo < 0: the
+// quad's result is not used): one compare of the smallest magnitude, which zeros also fail.
+FXD float fx_jacobi_least(float m, const FxQuad& n) {
+    m = fminf(fminf(m, fabsf(n.a.x)), fabsf(n.a.y));
+    return fminf(fminf(m, fabsf(n.b.x)), fabsf(n.b.y));
+}
 template <bool TWO>
 FXD bool fx_jacobi_rare(const FxJacobiK<TWO>& K, float lo, const FxQuad& n) {
-    const float least = fminf(fminf(fabsf(n.a.x), fabsf(n.a.y)), fminf(fabsf(n.b.x), fabsf(n.b.y)));
-    bool bad = least < lo;
+    bool bad = fx_jacobi_least(INFINITY, n) < lo;
     if (!TWO) bad = bad || (lo > 0.0f && (!K.fast || fx_odd4(n)));
     return bad;
 }
-// The quotients of two quads, guarded by one warp-uniform test: numerators too small for the
-// checked operations, which only the fronts of a spreading solve have, take the quotient through
-// double precision.
-template <bool TWO>
-FXD void fx_jacobi_divide2(const FxJacobiK<TWO>& K, float lo1, float lo2, const FxQuad& n1, const FxQuad& n2, FxQuad& q1,
-                           FxQuad& q2) {
-    q1 = fx_jacobi_quotients<TWO>(K, n1);
-    q2 = fx_jacobi_quotients<TWO>(K, n2);
-    if (__any_sync(0xffffffffu, fx_jacobi_rare<TWO>(K, lo1, n1) || fx_jacobi_rare<TWO>(K, lo2, n2))) {
-        q1 = fx_jacobi_small<TWO>(K, n1);
-        q2 = fx_jacobi_small<TWO>(K, n2);
-    }
+// ... and whether one is: zeros pass through the two operations (not through Markstein's step,
+// which loses their sign).
+FXD bool fx_jacobi_tiny(float lo, const FxQuad& n) {
+    auto tiny = [&](float x) { return x != 0.0f && fabsf(x) < lo; };
+    return tiny(n.a.x) || tiny(n.a.y) || tiny(n.b.x) || tiny(n.b.y);
 }
 // One cell.
 template <bool TWO>

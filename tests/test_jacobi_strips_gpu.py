@@ -74,3 +74,57 @@ def test_auto_on_a_grid_beyond_the_chip_equals_single_sweeps_and_the_oracle():
     assert d["jacobi_kernel"] == A.JACOBI_FUSED and d["jacobi_staging"] == A.STAGING_TMA, d
     same(auto, one)
     same(auto, o)
+
+
+# ---- the resident variant with the pressure in registers (fx_jacobi_reg.cuh) -------------------
+
+@pytest.mark.parametrize("dims", [(4, 12, 8), (8, 28, 4), (36, 20, 44), (100, 36, 20), (128, 8, 148), (260, 12, 16), (64, 96, 64)])
+@pytest.mark.parametrize("P,R", [(1, 1), (7, 4)])
+def test_registers_equal_single_sweeps(dims, P, R):
+    """Rows of one group and of 25 and 65 (rows across warps), columns in overlapping parts, more boxes
+    than planes or rows, and the slots of one to seven sweeps over three steps."""
+    opts = sphere_options(dims, P=P, R=R)
+    one, reg = FireXSim(dims, opts), FireXSim(dims, opts)
+    one.set_jacobi("unblocked")
+    one.step(3, DT)
+    reg.step(3, DT)
+    d = reg.diagnostics
+    assert d["jacobi_kernel"] == A.JACOBI_RESIDENT and d["jacobi_variant"] == 4, d
+    same(one, reg)
+
+
+def test_registers_from_rest_and_cold():
+    dims = (48, 64, 48)
+    for mode in (A.PRESSURE_WARM_F32, A.PRESSURE_COLD_F32):
+        opts = sphere_options(dims, P=40, R=24, noise=0.0, pressure_mode=mode)
+        one, reg = FireXSim(dims, opts), FireXSim(dims, opts)
+        one.set_jacobi("unblocked")
+        one.step(2, DT)
+        reg.step(2, DT)
+        same(one, reg)
+
+
+def test_registers_survive_a_change_of_members():
+    """The exchange buffer is kept, regrown and cleared as the batch's members change."""
+    from fire_b200.sim import FireXBatch
+    dims = [(32, 48, 32), (48, 64, 48), (36, 44, 28)]
+    alone = [FireXSim(d, sphere_options(d, P=6, R=5, seed=i)) for i, d in enumerate(dims)]
+    sims = [FireXSim(d, sphere_options(d, P=6, R=5, seed=i)) for i, d in enumerate(dims)]
+    for s in alone:
+        s.set_jacobi("unblocked")
+        s.step(4, DT)
+    with FireXBatch() as b:
+        b.add(sims[0])
+        b.step(1, DT)
+        b.add(sims[1])
+        b.step(2, DT)
+        b.remove(sims[0])
+        b.add(sims[2])
+        b.step(1, DT)
+        b.remove(sims[1])
+        b.step(3, DT)
+        b.remove(sims[2])
+    for s in sims[:2]:  # the fourth step of these, alone
+        s.step(1, DT)
+    for a, m in zip(alone, sims):
+        same(a, m)
