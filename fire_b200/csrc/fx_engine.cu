@@ -145,11 +145,12 @@ struct StepPlan {
     bool resReg = false;      // ... with the pressure in registers (variant 4)
     int resSmem = 0;          // its dynamic shared memory per CTA
     bool projRes = false;     // the residual projection inside the resident launch (variant 4)
+    bool simTwo = false;      // the source pass divides by its fixed divisors in two operations
     bool simEarly = false;    // the source pass evaluates its neighbour terms before the advection
     int bricks[FX_NSHAPES] = {};
     auto key() const {
         return std::tie(storage, half, maxP, maxR, k, zc, zrun, zmZc, row4, fuseP, fuseR, pack, tma, two, simBy, projDiv, res,
-                        resVariant, resReg, resSmem, projRes, simEarly,
+                        resVariant, resReg, resSmem, projRes, simEarly, simTwo,
                         bricks[0],
                         bricks[1], bricks[2], bricks[3], bricks[4], bricks[5], bricks[6]);
     }
@@ -202,7 +203,7 @@ void enqueue_step_launches(cudaStream_t st, const StepPlan& pl, FxBatchDev* B) {
     fx_launch_step_begin(st, B);
     fx_launch_step_tables(st, B, pl.bricks[FX_SHAPE_TAB]);
     if (sph_launches(pl)) fx_launch_sph(st, B, pl.bricks[FX_SHAPE_ROW4], pl.bricks[FX_SHAPE_PART]);
-    fx_launch_simulate(st, pl.storage, pl.simBy, pl.simEarly, B, pl.bricks[FX_SHAPE_CELL]);
+    fx_launch_simulate(st, pl.storage, pl.simBy, pl.simEarly, pl.simTwo, B, pl.bricks[FX_SHAPE_CELL]);
     fx_launch_divergence(st, B, pl.bricks[FX_SHAPE_ROW4], 0);
     enqueue_jacobi_phase(st, pl, B, 0);
     if (pl.projDiv) {
@@ -561,6 +562,31 @@ struct ExchangePool {
 ExchangePool g_exchange;
 }  // namespace
 
+// Whether the fixed divisors of simulate have their two-operation quotients on this device
+// (fx_div_two_of), checked like the others, once per device.
+static bool fixed_divisors_ok(int device) {
+    static std::map<int, bool> cache;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(device);
+    if (it != cache.end()) return it->second;
+    unsigned long long bad = ~0ull, *dcount = nullptr;
+    cudaStream_t st = nullptr;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess && cudaMalloc(&dcount, sizeof(bad)) == cudaSuccess &&
+        cudaMemsetAsync(dcount, 0, sizeof(bad), st) == cudaSuccess) {
+        for (int k = 0; k < FX_DIV_TWO_COUNT; ++k) {
+            const FxDivTwo c = fx_div_two_of(k);
+            fx_launch_check_div_two(st, c.d, c.rh, c.rl, FX_DIV_TWO_LO, 1.0 / (double)c.d, dcount);
+        }
+        if (cudaMemcpyAsync(&bad, dcount, sizeof(bad), cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+            bad = ~0ull;
+    }
+    cudaGetLastError();
+    if (dcount) cudaFree(dcount);
+    if (st) cudaStreamDestroy(st);
+    return cache[device] = bad == 0;
+}
+
 // ---- one simulation ------------------------------------------------------------------------
 struct firex_sim {
     int X = 0, Y = 0, Z = 0;
@@ -717,6 +743,7 @@ struct firex_sim {
         const float divisors[DIVC_COUNT] = {
             6.0f, 0.78f - 0.30f, 1500.0f - 400.0f, 930.0f - 690.0f, 1650.0f - 520.0f, 1040.0f - 335.0f,
             0.48f - (-0.42f), 1500.0f, fmaxr(u[9], 0.001f), fmaxr(u[4], 0.0001f), 1005.0f * persistence};
+        h.simTwo = fixed_divisors_ok(device) ? 1 : 0;
         for (int k = 0; k < DIVC_COUNT; ++k) {
             FxDivc& c = h.divc[k];
             std::memset(&c, 0, sizeof(c));
@@ -1006,11 +1033,11 @@ struct firex_batch {
         // 0.118 against 0.125 ms)
         const int pf = this->projFuse != FIREX_PROJECT_AUTO ? this->projFuse : members[0]->projFuse;
         p.projDiv = pf == FIREX_PROJECT_FUSED || (pf == FIREX_PROJECT_AUTO && cells < (8LL << 20));
-        // the source pass's neighbour terms ahead of the advection below 12 Mi cells with FP32
-        // storage (measured on B200, ms per pass, early against reference order: HD 0.185 /
-        // 0.194, 160x240x160 0.353 / 0.361, 192x288x192 0.604 / 0.618; 256^3 1.010 / 0.964;
-        // mixed storage HD 0.181 / 0.174, 160x240x160 0.344 / 0.326)
-        p.simEarly = p.storage == FX_STORAGE_F32 && cells < FX_SIM_EARLY_CELLS;
+        // the source pass's neighbour terms ahead of the advection below 12 Mi cells (measured on
+        // B200, us per pass, early against reference order: HD 157 / 167, 160x240x160 298 / 307,
+        // mixed storage HD 154 / 158; 300x452x276 2565 / 2220, 508^3 8302 / 8012, twelve uneven grids
+        // of 38 M cells 1660 / 1530)
+        p.simEarly = cells < FX_SIM_EARLY_CELLS;
         // The two-sweep pass stages its planes by TMA (FP32 pressure, every member's tensor maps
         // built) when asked to, or when AUTO chose the pass with chunks that fill the device's
         // waves: tensor loads then cost a warp next to nothing (160x240x160: 2.14 against 2.56 ms
@@ -1022,7 +1049,11 @@ struct firex_batch {
         for (firex_sim* s : members) maps = maps && s->h.tmapOk;
         p.tma = p.k == 2 && maps;
         p.two = true;
-        for (firex_sim* s : members) p.two = p.two && s->h.jcTwo;
+        p.simTwo = true;
+        for (firex_sim* s : members) {
+            p.two = p.two && s->h.jcTwo;
+            p.simTwo = p.simTwo && s->h.simTwo;
+        }
         if (tableK != p.k || tableZc != p.zrun || tableZmZc != p.zmZc || tableRes != (wantRes ? 2 + resForce : 0) ||
             tableWater != water_signature() || tableSimBy != p.simBy || tableTma != p.tma)
             fill_table(p.k, p.zrun, p.zmZc, wantRes, resForce, p.simBy, p.tma);
@@ -1098,7 +1129,7 @@ struct firex_batch {
             fx_launch_sph(stream, d, pl.bricks[FX_SHAPE_ROW4], pl.bricks[FX_SHAPE_PART]);
             mark(FIREX_PASS_PARTICLES, sph_launches(pl));
         }
-        fx_launch_simulate(stream, pl.storage, pl.simBy, pl.simEarly, d, pl.bricks[FX_SHAPE_CELL]);
+        fx_launch_simulate(stream, pl.storage, pl.simBy, pl.simEarly, pl.simTwo, d, pl.bricks[FX_SHAPE_CELL]);
         mark(FIREX_PASS_SIMULATE, 1);
         fx_launch_divergence(stream, d, pl.bricks[FX_SHAPE_ROW4], 0);
         mark(FIREX_PASS_DIVERGENCE, 1);

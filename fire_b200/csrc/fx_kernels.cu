@@ -95,9 +95,14 @@ struct Acc {
 };
 
 // One thread per cell of a 32 x BY x (8 / BY) brick (BY = 2, 4 or 8: the tunable brick
-// shape; FX_CELL_BY, 4, by default).
-// EARLY: the neighbour terms before the advection (fx_simulate_cell).
-template <class St, int BY, bool EARLY>
+// shape; FX_CELL_BY, 4, by default). EARLY: the neighbour terms before the advection, TWO: the fixed
+// divisors in two operations and records in pairs (fx_simulate_cell).
+// Bound by the latency of its gathers and by issue slots (55 % busy; L1 data pipe 55-59 %): 955
+// instructions a warp and cell, 1292 before pairs, two-operation divisions, T^4 by two double
+// products and brick places by carries; 128x192x128 157 us a pass (186 before), 160x240x160 298
+// (350), 300x452x276 2.22 ms (2.67), 508^3 8.0 ms (8.98). Two CTAs per SM without spills: 508^3 7.7 ms,
+// but 128x192x128 178 us and twelve uneven grids 1.77 ms against 1.53; four at 64 registers: no faster.
+template <class St, int BY, bool EARLY, bool TWO>
 __global__ void __launch_bounds__(256, 3) fxk_simulate(const FxBatchDev* __restrict__ B) {
     constexpr int BX = FX_CELL_BX, BZ = 256 / (FX_CELL_BX * BY);
     // the simulation's parameter block, the uniform entries of its per-step table and its
@@ -106,7 +111,12 @@ __global__ void __launch_bounds__(256, 3) fxk_simulate(const FxBatchDev* __restr
     __shared__ FxParams sP;
     __shared__ float sUT[TU_COUNT];
     __shared__ FxDivc sDC[DIVC_COUNT];
+    __shared__ FxTabLayout sL;
     const FxSimDev* cur = nullptr;
+    // the brick's place in its simulation, and how far the CTA's next brick (gridDim.x on) is from
+    // it: found by division once per simulation, then advanced with carries (a division of each
+    // brick number by every thread cost 60 instructions per cell)
+    int bx = 0, by = 0, bz = 0, nbx = 1, nby = 1, dx = 0, dy = 0, dz = 0;
     fx_for_bricks<FX_SHAPE_CELL>(B, [&](const FxSimDev& S, int b) {
         if (&S != cur) {      // the same brick, so the same decision, in every thread
             __syncthreads();  // every read of the previous simulation's block is done
@@ -117,17 +127,37 @@ __global__ void __launch_bounds__(256, 3) fxk_simulate(const FxBatchDev* __restr
                 else if (i < nP + TU_COUNT) sUT[i - nP] = S.tab[i - nP];
                 else reinterpret_cast<uint32_t*>(sDC)[i - nP - TU_COUNT] = reinterpret_cast<const uint32_t*>(S.divc)[i - nP - TU_COUNT];
             }
+            if (threadIdx.x == 0) sL = fx_tab_layout(S.X, S.Y, S.Z);
             __syncthreads();
             cur = &S;
+            nbx = (S.X + BX - 1) / BX;
+            nby = (S.Y + BY - 1) / BY;
+            const int step = (int)gridDim.x;
+            bx = b % nbx;
+            by = (b / nbx) % nby;
+            bz = b / (nbx * nby);
+            dx = step % nbx;
+            dy = (step / nbx) % nby;
+            dz = step / (nbx * nby);
         }
-        const int nbx = (S.X + BX - 1) / BX, nby = (S.Y + BY - 1) / BY;
-        const int x = (b % nbx) * BX + threadIdx.x % BX;
-        const int y = ((b / nbx) % nby) * BY + (threadIdx.x / BX) % BY;
-        const int z = (b / (nbx * nby)) * BZ + threadIdx.x / (BX * BY);
+        const int x = bx * BX + threadIdx.x % BX;
+        const int y = by * BY + (threadIdx.x / BX) % BY;
+        const int z = bz * BZ + threadIdx.x / (BX * BY);
+        bx += dx;
+        by += dy;
+        bz += dz;
+        if (bx >= nbx) {
+            bx -= nbx;
+            ++by;
+        }
+        if (by >= nby) {
+            by -= nby;
+            ++bz;
+        }
         if (x >= S.X || y >= S.Y || z >= S.Z) return;
         const FxGrid g{S.X, S.Y, S.Z};
         Acc<St> a{S.flow[S.fi], S.species[S.si], S.liquid};
-        FxCellOut o = fx_simulate_cell<EARLY>(sP, g, x, y, z, a, S.tab, sUT, sDC);
+        const FxCellOut o = fx_simulate_cell<EARLY, TWO>(sP, g, x, y, z, a, S.tab, sL, sUT, sDC);
         const int id = x + S.X * (y + S.Y * z);
         fx_st_flow(S.flow[S.fi ^ 1], id, o.flow);
         St::st_species(S.species[S.si ^ 1], id, o.species);
@@ -872,25 +902,28 @@ void fx_launch_step_tables(cudaStream_t s, const FxBatchDev* B, int bricks) {
     fxk_step_tables<<<bricks > 0 ? bricks : 1, 256, 0, s>>>(B);
 }
 
-template <class St, int BY, bool EARLY>
+template <class St, int BY, bool EARLY, bool TWO>
 static void launch_simulate(cudaStream_t s, const FxBatchDev* B, int bricks) {
-    static int g = persistent_grid((const void*)fxk_simulate<St, BY, EARLY>, 256, 1 << 30);
-    fxk_simulate<St, BY, EARLY><<<bricks < g ? bricks : g, 256, 0, s>>>(B);
+    static int g = persistent_grid((const void*)fxk_simulate<St, BY, EARLY, TWO>, 256, 1 << 30);
+    fxk_simulate<St, BY, EARLY, TWO><<<bricks < g ? bricks : g, 256, 0, s>>>(B);
 }
 
-template <class St, bool EARLY>
+template <class St, bool EARLY, bool TWO>
 static void launch_simulate_shape(cudaStream_t s, int by, const FxBatchDev* B, int bricks) {
-    if (by == 2) launch_simulate<St, 2, EARLY>(s, B, bricks);
-    else if (by == 8) launch_simulate<St, 8, EARLY>(s, B, bricks);
-    else launch_simulate<St, 4, EARLY>(s, B, bricks);
+    if (by == 2) launch_simulate<St, 2, EARLY, TWO>(s, B, bricks);
+    else if (by == 8) launch_simulate<St, 8, EARLY, TWO>(s, B, bricks);
+    else launch_simulate<St, 4, EARLY, TWO>(s, B, bricks);
 }
 
-void fx_launch_simulate(cudaStream_t s, int storage, int by, bool early, const FxBatchDev* B, int bricks) {
-    if (storage == FX_STORAGE_MIXED) {  // the reference order only (measured faster for mixed storage)
-        launch_simulate_shape<StMixed, false>(s, by, B, bricks);
+void fx_launch_simulate(cudaStream_t s, int storage, int by, bool early, bool two, const FxBatchDev* B, int bricks) {
+    if (storage == FX_STORAGE_MIXED) {
+        if (!two) launch_simulate_shape<StMixed, false, false>(s, by, B, bricks);
+        else if (early) launch_simulate_shape<StMixed, true, true>(s, by, B, bricks);
+        else launch_simulate_shape<StMixed, false, true>(s, by, B, bricks);
     } else {
-        if (early) launch_simulate_shape<StF32, true>(s, by, B, bricks);
-        else launch_simulate_shape<StF32, false>(s, by, B, bricks);
+        if (!two) launch_simulate_shape<StF32, false, false>(s, by, B, bricks);
+        else if (early) launch_simulate_shape<StF32, true, true>(s, by, B, bricks);
+        else launch_simulate_shape<StF32, false, true>(s, by, B, bricks);
     }
 }
 

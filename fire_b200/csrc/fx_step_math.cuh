@@ -86,6 +86,80 @@ FXD float fx_smoothstep_c(float e0, float x, const FxDivc& c) {
     return t * t * (3.0f - 2.0f * t);
 }
 
+struct FxQuad {  // four values as two pairs: four consecutive x cells, or a cell's record
+    float2 a, b;
+};
+FXD FxQuad fx_quad(float4 v) { return FxQuad{make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
+FXD FxQuad fx_quad_zero() { return fx_quad(make_float4(0.0f, 0.0f, 0.0f, 0.0f)); }
+FXD float2 fx_bcast2(float v) { return make_float2(v, v); }
+
+// The fixed divisors of simulate in two operations: RN(x rh + RN(x rl)) with 1/d = rh + rl, rh
+// rounded down (fx_div_two below has the method), is x / d for every float x of magnitude 2^-100
+// and above, for zeros, infinities and NaN. The engine checks that on the device for every float
+// before the source pass uses them (FxSimDev::simTwo), else the pass divides by fx_divc.
+struct FxDivTwo {
+    float d, rh, rl;
+};
+#define FX_DIV_TWO_LO 7.888609052210118e-31f  // 2^-100
+#define FX_DIV_TWO_COUNT 8
+__host__ __device__ inline FxDivTwo fx_div_two_of(int slot) {
+    switch (slot) {
+        case DIVC_SIX: return {6.0f, 0x1.555554p-3f, 0x1.555556p-27f};
+        case DIVC_FUELCORE: return {0.78f - 0.30f, 0x1.0aaaacp+1f, 0x1.238e4ap-26f};
+        case DIVC_ENTRAIN_T: return {1500.0f - 400.0f, 0x1.dca01cp-11f, 0x1.ca01dcp-35f};
+        case DIVC_IGNITION: return {930.0f - 690.0f, 0x1.11111p-8f, 0x1.111112p-32f};
+        case DIVC_HOTPLUME: return {1650.0f - 520.0f, 0x1.cff8cp-11f, 0x1.cff8cp-39f};
+        case DIVC_EVAP: return {1040.0f - 335.0f, 0x1.73d5ep-10f, 0x1.8b133ep-35f};
+        case DIVC_LOBE: return {0.48f - (-0.42f), 0x1.1c71c6p+0f, 0x1.9add3cp-24f};
+        default: return {1500.0f, 0x1.5d867cp-11f, 0x1.f67152p-38f};  // DIVC_BUOYANCY
+    }
+}
+static_assert(DIVC_BUOYANCY == FX_DIV_TWO_COUNT - 1, "the fixed divisors come first");
+// x / d of slot SLOT without a range check, for an x that is 0 or no smaller than 2^-100: a
+// difference from a constant of at least 0.3, whose neighbouring floats are 2^-26 apart.
+template <int SLOT>
+FXD float fx_div_fixed(float x) {
+    const FxDivTwo c = fx_div_two_of(SLOT);
+    return __fmaf_rn(x, c.rh, __fmul_rn(x, c.rl));
+}
+// (x - e0) / d of slot SLOT by the two operations (TWO) or by fx_divc, and its smoothstep.
+template <bool TWO, int SLOT>
+FXD float fx_div_from(float e0, float x, const FxDivc* dc) {
+    return TWO ? fx_div_fixed<SLOT>(x - e0) : fx_divc(x - e0, dc[SLOT]);
+}
+template <bool TWO, int SLOT>
+FXD float fx_smoothstep_from(float e0, float x, const FxDivc* dc) {
+    const float t = fx_clamp(fx_div_from<TWO, SLOT>(e0, x, dc), 0.0f, 1.0f);
+    return t * t * (3.0f - 2.0f * t);
+}
+// A sixth of each of four sums (shaders.ts:177-187). TWO: two operations a pair, unless one of the
+// sums is too small for them, as at the faint edge of a diffusing field (zeros are not).
+FXD float4 fx_sixth(const float4& s, const FxDivc* dc) {
+    return make_float4(fx_divc(s.x, dc[DIVC_SIX]), fx_divc(s.y, dc[DIVC_SIX]), fx_divc(s.z, dc[DIVC_SIX]), fx_divc(s.w, dc[DIVC_SIX]));
+}
+FXD unsigned fx_mag(float x) { return 2u * __float_as_uint(x) - 1u; }  // ascends with |x|; zeros come last
+FXD float4 fx_sixth_two(const FxQuad& s, const FxDivc* dc) {
+    const FxDivTwo c = fx_div_two_of(DIVC_SIX);
+    const float2 rh = fx_bcast2(c.rh), rl = fx_bcast2(c.rl);
+    const float2 a = __ffma2_rn(s.a, rh, __fmul2_rn(s.a, rl)), b = __ffma2_rn(s.b, rh, __fmul2_rn(s.b, rl));
+    const unsigned least = min(min(fx_mag(s.a.x), fx_mag(s.a.y)), min(fx_mag(s.b.x), fx_mag(s.b.y)));
+    if (least < fx_mag(FX_DIV_TWO_LO)) return fx_sixth(make_float4(s.a.x, s.a.y, s.b.x, s.b.y), dc);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+FXD FxQuad fx_add4(const FxQuad& a, const FxQuad& b) { return FxQuad{__fadd2_rn(a.a, b.a), __fadd2_rn(a.b, b.b)}; }
+FXD float4 fx_f4(const FxQuad& q) { return make_float4(q.a.x, q.a.y, q.b.x, q.b.y); }
+// mix of two records: a (1 - t) + b t, every product rounded (nz: the run-time -0 of fx_jacobi4)
+FXD FxQuad fx_mix_two(const FxQuad& a, const FxQuad& b, float t, float nz) {
+    const float2 s2 = fx_bcast2(1.0f - t), t2 = fx_bcast2(t), z2 = fx_bcast2(nz);
+    return FxQuad{__fadd2_rn(__ffma2_rn(a.a, s2, z2), __ffma2_rn(b.a, t2, z2)), __fadd2_rn(__ffma2_rn(a.b, s2, z2), __ffma2_rn(b.b, t2, z2))};
+}
+// T^4 rounded once from the double product of exact squares: nearer to the exact power than
+// powf(T, 4) (two units in the last place) at a tenth of its instructions.
+FXD float fx_pow4(float t) {
+    const double s = (double)t * (double)t;
+    return (float)(s * s);
+}
+
 // trilinearFlow / trilinearSpecies (shaders.ts:61-95): 8-tap trilinear sample at
 // position - 0.5, clamped to [0, dims - 1.001]. The clamp bounds floor() to
 // [0, dims - 2], so base + 1 is always inside the grid and the reference's clamped tap
@@ -116,6 +190,16 @@ FXD float4 fx_trilinear(const FxGrid& g, const FxTri& t, Load load) {
     float4 z1 = fx_mix4(fx_mix4(c001, c101, t.fx), fx_mix4(c011, c111, t.fx), t.fy);
     return fx_mix4(z0, z1, t.fz);
 }
+template <class Load>
+FXD float4 fx_trilinear_two(const FxGrid& g, const FxTri& t, float nz, Load load) {
+    const int X = g.X, XY = g.X * g.Y, b = t.base;
+    auto plane = [&](int i) {
+        const FxQuad lo = fx_mix_two(fx_quad(load(i)), fx_quad(load(i + 1)), t.fx, nz);
+        return fx_mix_two(lo, fx_mix_two(fx_quad(load(i + X)), fx_quad(load(i + X + 1)), t.fx, nz), t.fy, nz);
+    };
+    const FxQuad z0 = plane(b);
+    return fx_f4(fx_mix_two(z0, plane(b + XY), t.fz, nz));
+}
 
 // ---- per-step tables ------------------------------------------------------------------------
 // Terms of simulate that depend only on time and on one or two coordinates are computed
@@ -140,6 +224,7 @@ enum {
     TU_LIFT, TU_ENTRAIN, TU_AMB_O2, TU_HEAT,       // clamped lift, entrainment, ambient O2, heat release
     TU_VORT_S, TU_TURB, TU_BUOY, TU_CINE,          // vorticity step, turbulence gain, clamped buoyancy, cinematic
     TU_SPRAY_X, TU_SPRAY_Y, TU_SPRAY_Z,            // unit spray direction
+    TU_NZ,                                         // -0 (fx_mix_two)
     TU_COUNT = 24
 };
 enum { TX_SWZ = 0, TX_CELL = 1, TX_LOBE = 2, TX_RAD = 3, TX_COUNT = 4 };
@@ -189,7 +274,7 @@ FXD float fx_table_entry(const float* u, int X, int Y, int Z, int i) {
         switch (i) {
             case TU_DECAY_Z: return expf(-dt * FC(0.075) / persistence);
             case TU_DECAY_W: return expf(-dt * FC(0.14) / persistence);
-            case TU_TAMB4: return powf(u[U_T_AMBIENT], 4.0f);
+            case TU_TAMB4: return fx_pow4(u[U_T_AMBIENT]);
             case TU_MX: return m.x;
             case TU_MY: return m.y;
             case TU_MZ: return m.z;
@@ -207,6 +292,7 @@ FXD float fx_table_entry(const float* u, int X, int Y, int Z, int i) {
             case TU_TURB: return FC(0.075) + FC(0.16) * u[U_VORTICITY];
             case TU_BUOY: return fx_clamp(u[U_BUOYANCY], 0.0f, 4.0f);
             case TU_CINE: return fx_clamp(u[U_CINEMATIC], 0.0f, 1.0f);
+            case TU_NZ: return -0.0f;
             default: break;
         }
         if (i >= TU_SPRAY_X && i <= TU_SPRAY_Z) {  // spray momentum direction (shaders.ts:293-297)
@@ -286,12 +372,12 @@ struct FxCellOut {
 // P, ut (the per-step table's uniform entries, TU_*) and dc are the same for every cell of a
 // simulation: the source pass stages them in shared memory; tab (the per-coordinate tables)
 // and the fields come from global memory.
-template <bool EARLY, class Acc>
+// TWO: the fixed divisors in two operations and the records in pairs.
+template <bool EARLY, bool TWO, class Acc>
 FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y, int z, const Acc& a,
-                               const float* __restrict__ tab, const float* ut, const FxDivc* dc) {
+                               const float* __restrict__ tab, const FxTabLayout& L, const float* ut, const FxDivc* dc) {
     const float* u = P.u;
     const int X = g.X, Y = g.Y, Z = g.Z;
-    const FxTabLayout L = fx_tab_layout(X, Y, Z);
     const int id = x + X * (y + Y * z);
     float picx = (float)x + 0.5f, picy = (float)y + 0.5f, picz = (float)z + 0.5f;
     float dt = u[U_DT];
@@ -303,24 +389,31 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     // temperature gradient of the vorticity confinement, each the reference's expression. EARLY
     // evaluates them before the advection, so that only these values, not the 12 neighbour
     // records, stay live through the update and the neighbour loads overlap the advection's
-    // dependent loads (faster up to about 10 M cells: HD 0.185 against 0.194 ms per pass,
-    // 192x288x192 0.604 against 0.618); otherwise they are evaluated where the reference does
-    // (256^3: 0.964 against 1.010 ms). The results are the same either way.
+    // dependent loads (faster up to about 10 M cells: 128x192x128 157 against 167 us per pass);
+    // otherwise they are evaluated where the reference does (508^3: 8.0 against 8.3 ms). The results
+    // are the same either way.
     // 6 neighbours with clamped (Neumann) addressing (shaders.ts:43-51)
     const int oL = x > 0 ? id - 1 : id, oR = x < X - 1 ? id + 1 : id;
     const int oB = y > 0 ? id - X : id, oT = y < Y - 1 ? id + X : id;
     const int oK = z > 0 ? id - X * Y : id, oF = z < Z - 1 ? id + X * Y : id;
-    float vax, vay, vaz, ta;  // shaders.ts:177-180
+    float4 va;                // velocity and temperature (shaders.ts:177-180)
     float cx, cy, cz;         // curl (shaders.ts:258-263)
     float gx, gy, gz;         // normalised grad(T) (shaders.ts:264-268)
     float4 avg;               // species diffusion (shaders.ts:182-187)
     float4 left, right, bottom, top, back, front;
+    const float nz = TWO ? ut[TU_NZ] : 0.0f;
+    auto sixth = [&](const float4& l, const float4& r, const float4& b, const float4& t, const float4& k, const float4& f) {
+        if constexpr (TWO) {
+            const FxQuad s = fx_add4(fx_add4(fx_add4(fx_add4(fx_add4(fx_quad(l), fx_quad(r)), fx_quad(b)), fx_quad(t)), fx_quad(k)), fx_quad(f));
+            return fx_sixth_two(s, dc);
+        } else {
+            return fx_sixth(make_float4(l.x + r.x + b.x + t.x + k.x + f.x, l.y + r.y + b.y + t.y + k.y + f.y,
+                                        l.z + r.z + b.z + t.z + k.z + f.z, l.w + r.w + b.w + t.w + k.w + f.w), dc);
+        }
+    };
     if constexpr (EARLY) {
         const float4 l = a.flow(oL), r = a.flow(oR), bo = a.flow(oB), t = a.flow(oT), k = a.flow(oK), f = a.flow(oF);
-        vax = fx_divc(l.x + r.x + bo.x + t.x + k.x + f.x, dc[DIVC_SIX]);
-        vay = fx_divc(l.y + r.y + bo.y + t.y + k.y + f.y, dc[DIVC_SIX]);
-        vaz = fx_divc(l.z + r.z + bo.z + t.z + k.z + f.z, dc[DIVC_SIX]);
-        ta = fx_divc(l.w + r.w + bo.w + t.w + k.w + f.w, dc[DIVC_SIX]);
+        va = sixth(l, r, bo, t, k, f);
         cx = 0.5f * ((t.z - bo.z) * metric.y - (f.y - k.y) * metric.z);
         cy = 0.5f * ((f.x - k.x) * metric.z - (r.z - l.z) * metric.x);
         cz = 0.5f * ((r.y - l.y) * metric.x - (t.x - bo.x) * metric.y);
@@ -331,21 +424,21 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         gx = gx / gl;
         gy = gy / gl;
         gz = gz / gl;
-        const float4 sl = a.species(oL), sr = a.species(oR);
-        const float4 sb = a.species(oB), st = a.species(oT);
-        const float4 sk = a.species(oK), sf = a.species(oF);
-        avg = make_float4(fx_divc(sl.x + sr.x + sb.x + st.x + sk.x + sf.x, dc[DIVC_SIX]),
-                          fx_divc(sl.y + sr.y + sb.y + st.y + sk.y + sf.y, dc[DIVC_SIX]),
-                          fx_divc(sl.z + sr.z + sb.z + st.z + sk.z + sf.z, dc[DIVC_SIX]),
-                          fx_divc(sl.w + sr.w + sb.w + st.w + sk.w + sf.w, dc[DIVC_SIX]));
+        avg = sixth(a.species(oL), a.species(oR), a.species(oB), a.species(oT), a.species(oK), a.species(oF));
     }
 
     float btx = picx - orig.x * dt * metric.x;
     float bty = picy - orig.y * dt * metric.y;
     float btz = picz - orig.z * dt * metric.z;
     const FxTri tri = fx_tri_setup(g, u, btx, bty, btz);
-    float4 flow = fx_trilinear(g, tri, [&](int i) { return a.flow(i); });
-    float4 species = fx_trilinear(g, tri, [&](int i) { return a.species(i); });
+    float4 flow, species;
+    if constexpr (TWO) {
+        flow = fx_trilinear_two(g, tri, nz, [&](int i) { return a.flow(i); });
+        species = fx_trilinear_two(g, tri, nz, [&](int i) { return a.species(i); });
+    } else {
+        flow = fx_trilinear(g, tri, [&](int i) { return a.flow(i); });
+        species = fx_trilinear(g, tri, [&](int i) { return a.species(i); });
+    }
     species = make_float4(fx_max(species.x, 0.0f), fx_max(species.y, 0.0f), fx_max(species.z, 0.0f),
                           fx_max(species.w, 0.0f));
 
@@ -358,29 +451,18 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         front = a.flow(oF);
     }
     {  // 6-neighbour diffusion of velocity and temperature (shaders.ts:177-180)
-        if constexpr (!EARLY) {
-            vax = fx_divc(left.x + right.x + bottom.x + top.x + back.x + front.x, dc[DIVC_SIX]);
-            vay = fx_divc(left.y + right.y + bottom.y + top.y + back.y + front.y, dc[DIVC_SIX]);
-            vaz = fx_divc(left.z + right.z + bottom.z + top.z + back.z + front.z, dc[DIVC_SIX]);
-        }
-        float vm = ut[TU_VMIX];
-        flow.x = fx_mix(flow.x, vax, vm);
-        flow.y = fx_mix(flow.y, vay, vm);
-        flow.z = fx_mix(flow.z, vaz, vm);
-        if constexpr (!EARLY) ta = fx_divc(left.w + right.w + bottom.w + top.w + back.w + front.w, dc[DIVC_SIX]);
-        flow.w = fx_mix(flow.w, ta, ut[TU_TMIX]);
+        if constexpr (!EARLY) va = sixth(left, right, bottom, top, back, front);
+        const float vm = ut[TU_VMIX];
+        flow.x = fx_mix(flow.x, va.x, vm);
+        flow.y = fx_mix(flow.y, va.y, vm);
+        flow.z = fx_mix(flow.z, va.z, vm);
+        flow.w = fx_mix(flow.w, va.w, ut[TU_TMIX]);
     }
     {  // species diffusion (shaders.ts:182-187)
-        if constexpr (!EARLY) {
-            float4 sl = a.species(oL), sr = a.species(oR);
-            float4 sb = a.species(oB), st = a.species(oT);
-            float4 sk = a.species(oK), sf = a.species(oF);
-            avg = make_float4(fx_divc(sl.x + sr.x + sb.x + st.x + sk.x + sf.x, dc[DIVC_SIX]),
-                              fx_divc(sl.y + sr.y + sb.y + st.y + sk.y + sf.y, dc[DIVC_SIX]),
-                              fx_divc(sl.z + sr.z + sb.z + st.z + sk.z + sf.z, dc[DIVC_SIX]),
-                              fx_divc(sl.w + sr.w + sb.w + st.w + sk.w + sf.w, dc[DIVC_SIX]));
-        }
-        species = fx_mix4(species, avg, ut[TU_SMIX]);
+        if constexpr (!EARLY)
+            avg = sixth(a.species(oL), a.species(oR), a.species(oB), a.species(oT), a.species(oK), a.species(oF));
+        if constexpr (TWO) species = fx_f4(fx_mix_two(fx_quad(species), fx_quad(avg), ut[TU_SMIX], nz));
+        else species = fx_mix4(species, avg, ut[TU_SMIX]);
     }
 
     // Source injection (shaders.ts:189-201); the sphere list replaces the burner.
@@ -403,7 +485,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         const float vertical = __ldg(tab + L.y + TY_VERT * Y + y);
         const float cellular = FC(0.76) + FC(0.24) * __ldg(tab + L.x + TX_CELL * X + x) * __ldg(tab + L.z + TZ_CELL * Z + z);
         const float lobeArg = __ldg(tab + L.x + TX_LOBE * X + x) * __ldg(tab + L.z + TZ_LOBE * Z + z);
-        const float lobes = fx_mix(FC(0.48), FC(1.18), fx_smoothstep_c(FC(-0.42), lobeArg, dc[DIVC_LOBE]));
+        const float lobes = fx_mix(FC(0.48), FC(1.18), fx_smoothstep_from<TWO, DIVC_LOBE>(FC(-0.42), lobeArg, dc));
         const float texture = fx_mix(cellular, cellular * lobes, ut[TU_CINE]);
         const float pulse = __ldg(tab + L.pulse + z * X + x);
         source = expf(-(radial + vertical)) * texture * pulse;
@@ -431,7 +513,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     const uint32_t liquidRaw = a.liquid(id);
     float water = fx_clamp((float)liquidRaw * (1.0f / 4096.0f) * FC(3.4), 0.0f, 5.0f);
     if (liquidRaw) {
-        float evaporation = water * fx_smoothstep_c(335.0f, flow.w, dc[DIVC_EVAP]) * dt * FC(13.5);
+        float evaporation = water * fx_smoothstep_from<TWO, DIVC_EVAP>(335.0f, flow.w, dc) * dt * FC(13.5);
         flow.w = fx_max(u[U_T_AMBIENT], flow.w - evaporation * 2080.0f - water * dt * 260.0f);
         species.w = fx_clamp(species.w + evaporation * FC(2.15), 0.0f, 3.0f);
     } else {
@@ -443,11 +525,11 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     const float entrainment = ut[TU_ENTRAIN];
     const float ambientOxygen = ut[TU_AMB_O2];
     float oxygenDeficit = fx_clamp(fx_divc(ambientOxygen - species.y, dc[DIVC_AMBIENT_O2]), 0.0f, 1.0f);
-    float fuelCore = fx_smoothstep_c(FC(0.30), species.x, dc[DIVC_FUELCORE]);
+    float fuelCore = fx_smoothstep_from<TWO, DIVC_FUELCORE>(FC(0.30), species.x, dc);
     float interfaceWeight = oxygenDeficit * fx_mix(1.0f, FC(0.18), fuelCore);
     float entrainmentMix = fx_clamp(dt * entrainment *
                                         (FC(0.12) + FC(0.28) * fx_length3(flow.x, flow.y, flow.z) +
-                                         FC(0.22) * fx_smoothstep_c(400.0f, flow.w, dc[DIVC_ENTRAIN_T])) *
+                                         FC(0.22) * fx_smoothstep_from<TWO, DIVC_ENTRAIN_T>(400.0f, flow.w, dc)) *
                                         interfaceWeight,
                                     0.0f, FC(0.08));
     species.y = fx_mix(species.y, ambientOxygen, entrainmentMix);
@@ -456,7 +538,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     float fuelBefore = fx_max(species.x, 0.0f);
     float oxygenBefore = fx_max(species.y, 0.0f);
     float availableFuel = fx_min(fuelBefore, oxygenBefore * FC(0.25));
-    float ignition = fx_smoothstep_c(690.0f, flow.w, dc[DIVC_IGNITION]);
+    float ignition = fx_smoothstep_from<TWO, DIVC_IGNITION>(690.0f, flow.w, dc);
     // 1 - exp(-arrhenius * ignition * dt). Below ignition (ignition == +0) the exponent is
     // -0 for any finite rate (the rate is clamped to [0, 80]) and the factor is exactly
     // +0, so the rate need not be evaluated; with no liquid exp(-water * 18) is exactly 1.
@@ -472,13 +554,19 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     float requestedBurn = availableFuel * growth;
     if (liquidRaw) requestedBurn = requestedBurn * expf(-water * 18.0f);
     float burn = fx_clamp(requestedBurn, 0.0f, availableFuel);
-    float richness = fx_clamp(1.0f - oxygenBefore / fx_max(fuelBefore * 4.0f, FC(0.00001)), 0.0f, 1.0f);
     species.x = fx_max(0.0f, fuelBefore - burn);
     species.y = fx_max(0.0f, oxygenBefore - burn * 4.0f);
-    species.z = fx_clamp(species.z + burn * (1.0f + richness * FC(1.8)), 0.0f, 3.0f);
+    // richness and the reaction rate only where something burns (burn == +0 elsewhere: the
+    // products below are then +0, whatever the richness, which is in [0, 1])
+    float fumes = 0.0f, reaction = 0.0f;
+    if (!(burn == 0.0f)) {
+        const float richness = fx_clamp(1.0f - oxygenBefore / fx_max(fuelBefore * 4.0f, FC(0.00001)), 0.0f, 1.0f);
+        fumes = burn * (1.0f + richness * FC(1.8));
+        reaction = fx_clamp(fx_divc(burn, dc[DIVC_DT]) * FC(0.22), 0.0f, 4.0f);
+    }
+    species.z = fx_clamp(species.z + fumes, 0.0f, 3.0f);
     species.w = fx_clamp(species.w + burn * FC(0.62), 0.0f, 3.0f);
     flow.w += burn * ut[TU_HEAT];
-    float reaction = fx_clamp(fx_divc(burn, dc[DIVC_DT]) * FC(0.22), 0.0f, 4.0f);
 
     {  // vorticity confinement: curl x grad(T) (shaders.ts:258-272)
         if constexpr (!EARLY) {
@@ -499,7 +587,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         flow.z = flow.z + (gx * cy - gy * cx) * vs;
     }
     {  // height-enveloped turbulence (shaders.ts:274-285)
-        float hotPlume = fx_smoothstep_c(520.0f, flow.w, dc[DIVC_HOTPLUME]);
+        float hotPlume = fx_smoothstep_from<TWO, DIVC_HOTPLUME>(520.0f, flow.w, dc);
         float heightEnvelope = __ldg(tab + L.y + TY_HE * Y + y);
         float ltx = __ldg(tab + L.ltx + z * Y + y);
         float lty = __ldg(tab + L.lty + z * X + x);
@@ -510,7 +598,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         flow.z = flow.z + ltz * ts;
     }
     {  // buoyancy (shaders.ts:287-288)
-        float buoyancy = fx_clamp(fx_divc(flow.w - u[U_T_AMBIENT], dc[DIVC_BUOYANCY]), FC(-0.1), FC(1.2));
+        float buoyancy = fx_clamp(fx_div_from<TWO, DIVC_BUOYANCY>(u[U_T_AMBIENT], flow.w, dc), FC(-0.1), FC(1.2));
         flow.y += buoyancy * dt * FC(0.72) * ut[TU_BUOY];
     }
     if (liquidRaw) species.z *= expf(-water * dt * FC(4.8));  // exp(-0) == 1 exactly otherwise
@@ -521,11 +609,9 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         flow.z = flow.z + dz * water * dt * FC(0.82);
     }
     // radiation and decay (shaders.ts:299-304); the decay factors come from the table
-    // pow(T, 4): cells at exactly the ambient temperature (every cold cell clamped to it
-    // above) take the per-step table value, which is the same powf of the same input
     const float tRad = fx_max(flow.w, 0.0f);
     const float tamb4 = ut[TU_TAMB4];
-    const float t4 = tRad == u[U_T_AMBIENT] ? tamb4 : powf(tRad, 4.0f);
+    const float t4 = fx_pow4(tRad);
     float radiation = fx_divc(FC(5.67e-8) * (tamb4 - t4), dc[DIVC_RADIATION]);
     flow.w = fx_max(u[U_T_AMBIENT], flow.w + dt * radiation);
     species.z *= ut[TU_DECAY_Z];
@@ -710,12 +796,6 @@ FXD FxJacobiK<TWO> fx_jacobi_k(const FxSimDev& S) {
     k.nz = -0.0f * fabsf(k.denom);  // a run-time -0 (see fx_jacobi4)
     return k;
 }
-struct FxQuad {  // four consecutive x cells as two pairs
-    float2 a, b;
-};
-FXD FxQuad fx_quad(float4 v) { return FxQuad{make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
-FXD FxQuad fx_quad_zero() { return fx_quad(make_float4(0.0f, 0.0f, 0.0f, 0.0f)); }
-FXD float2 fx_bcast2(float v) { return make_float2(v, v); }
 // Numerators of four consecutive cells of one sweep, the operations of fx_jacobi_numerator cell by
 // cell: c holds the cells, l and r their outer x neighbours, b/t/k/f the y-1, y+1, z-1, z+1
 // rows, d the divergence. The x sums are scalar (their operands straddle the pairs, which packed
