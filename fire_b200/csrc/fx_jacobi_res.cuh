@@ -713,7 +713,7 @@ static __device__ __noinline__ void fx_res_project_epi(const FxSimDev& S, const 
 // the neighbours and brings the halo rows in with bulk copies while the interior is computed;
 // the other FX_RES_COPY_TC threads run the sweep, synchronise on a named barrier, publish per
 // warp, and wait for the copies instead of waiting for flags and loading the halo themselves.
-template <typename PT, bool ROUND, bool COPY, bool EPI = false>
+template <typename PT, bool ROUND, bool COPY, bool EPI = false, bool TWO = false>
 FXD void fx_res_box_v3(const FxSimDev& S, const FxResBox& bx, int b, int phase, float* sm) {
     constexpr bool epi = EPI;
     __shared__ int s_flag;
@@ -773,7 +773,9 @@ FXD void fx_res_box_v3(const FxSimDev& S, const FxResBox& bx, int b, int phase, 
     const bool shflL = lane > 0 && q > 0 && col > 0 && part < P;
     const bool shflR = lane < 31 && q < gx - 1 && col < C - 1 && t + 1 < T && part < P;
     const long long gRow = (long long)(z0 + zs) * XY + (long long)y * X + x0;
-    const FxJacobiConst2 c2 = fx_jacobi_const2(FxJacobiConst{S.jc[0], S.jc[1], S.jc[2], S.jc[3]}, S.jcRcp, S.jcFastDiv != 0);
+    const FxJacobiConst2 c2 =
+        TWO ? fx_jacobi_const2_two(S)
+            : fx_jacobi_const2(FxJacobiConst{S.jc[0], S.jc[1], S.jc[2], S.jc[3]}, S.jcRcp, S.jcFastDiv != 0);
     // new value of face group g from the old values in shared memory
     auto update = [&](int g) {
         const int fq = g & 0x3ff, fly = (g >> 10) & 0x7ff, flz = g >> 21;
@@ -788,7 +790,7 @@ FXD void fx_res_box_v3(const FxSimDev& S, const FxResBox& bx, int b, int phase, 
         const float4 pkv = *reinterpret_cast<const float4*>((fz > 0 ? rowC - planeP : rowC) + fx0);
         const float4 pfv = *reinterpret_cast<const float4*>((fz < Z - 1 ? rowC + planeP : rowC) + fx0);
         const float4 d = *reinterpret_cast<const float4*>(sd + (flz * bx.by + fly) * X + fx0);
-        float4 o = fx_jacobi4<true, COPY>(c2, pl, pc, pr, pb, pt, pkv, pfv, d);
+        float4 o = fx_jacobi4<true, COPY, TWO>(c2, pl, pc, pr, pb, pt, pkv, pfv, d);
         if (ROUND) o = make_float4(PStore<__half>::round(o.x), PStore<__half>::round(o.y), PStore<__half>::round(o.z),
                                    PStore<__half>::round(o.w));
         return o;
@@ -878,7 +880,7 @@ FXD void fx_res_box_v3(const FxSimDev& S, const FxResBox& bx, int b, int phase, 
                     const float pl = shflL ? fromL : (hasL ? sp[off - 1] : pc.x);
                     const float pr = shflR ? fromR : (hasR ? sp[off + 4] : pc.w);
                     const float4 d = *reinterpret_cast<const float4*>(sd + offD + k * planeD);
-                    float4 o = fx_jacobi4<true, COPY>(c2, pl, pc, pr, pb, pt, pk, pfv, d);
+                    float4 o = fx_jacobi4<true, COPY, TWO>(c2, pl, pc, pr, pb, pt, pk, pfv, d);
                     if (ROUND) o = make_float4(PStore<__half>::round(o.x), PStore<__half>::round(o.y),
                                                PStore<__half>::round(o.z), PStore<__half>::round(o.w));
                     nv[k] = top ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : o;

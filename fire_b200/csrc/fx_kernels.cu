@@ -792,8 +792,9 @@ __global__ void __launch_bounds__(256) fxk_norm_partial(const FxSimDev* __restri
 // ---- every sweep of a Jacobi phase in one cooperative launch (fx_jacobi_res.cuh) --------
 // VARIANT: 0 column, 1 faces-first, 2 faces-first for small boxes, 3 faces-first with
 // interior columns, 4 variant 3 with a copy warp (FP32 pressure) (fx_jacobi_res.cuh).
-// EPI (variant 4, residual phase): the projection epilogue (fx_res_project_epi).
-template <typename PT, int VARIANT, bool EPI = false>
+// EPI (variant 4, residual phase): the projection epilogue (fx_res_project_epi). TWO (variant 4): the
+// two-operation quotient, where the members' denominators passed its check.
+template <typename PT, int VARIANT, bool EPI = false, bool TWO = false>
 __global__ void __launch_bounds__(FX_RES_THREADS, 1) fxk_jacobi_res(const FxBatchDev* __restrict__ B, int phase) {
     extern __shared__ float4 fx_res_smem[];
     const int w = blockIdx.x;
@@ -807,7 +808,7 @@ __global__ void __launch_bounds__(FX_RES_THREADS, 1) fxk_jacobi_res(const FxBatc
     else if (VARIANT == 2) fx_res_box_early<PT, sizeof(PT) == 2, FX_RES_MAXI_SMALL>(S, B->res[si], b, phase, sm);
     else if (VARIANT == 3) fx_res_box_v3<PT, sizeof(PT) == 2, false>(S, B->res[si], b, phase, sm);
     else if (VARIANT == 4) {
-        if constexpr (sizeof(PT) == 4) fx_res_box_v3<float, false, true, EPI>(S, B->res[si], b, phase, sm);
+        if constexpr (sizeof(PT) == 4) fx_res_box_v3<float, false, true, EPI, TWO>(S, B->res[si], b, phase, sm);
     }
     else fx_res_box_col<PT, sizeof(PT) == 2>(S, B->res[si], b, phase, sm);
 }
@@ -1047,6 +1048,7 @@ static const void* res_variant(int variant) {
 static const void* res_kernel(const FxResKernel& k, bool epi, bool two) {
     if (k.variant != 4) return k.half ? res_variant<__half>(k.variant) : res_variant<float>(k.variant);
     if (k.half) return nullptr;
+    if (!k.reg && two) return epi ? (const void*)fxk_jacobi_res<float, 4, true, true> : (const void*)fxk_jacobi_res<float, 4, false, true>;
     if (!k.reg) return epi ? (const void*)fxk_jacobi_res<float, 4, true> : (const void*)fxk_jacobi_res<float, 4>;
     if (two) return epi ? (const void*)fxk_jacobi_reg<true, true> : (const void*)fxk_jacobi_reg<false, true>;
     return epi ? (const void*)fxk_jacobi_reg<true, false> : (const void*)fxk_jacobi_reg<false, false>;

@@ -671,23 +671,47 @@ FXD float fx_jacobi_numerator(const FxJacobiConst& c, float l, float r, float b,
                                __fmul_rn(c.wz, __fadd_rn(k, f))),
                      div);
 }
+// RN(x / d) for any finite x through double precision: the product by rcp = RN(1/d) with one
+// correction step is the correctly rounded double quotient, whose rounding to float is x / d
+// (53 >= 2 * 24 + 2 bits). Zeros, infinities and NaN are returned as they are.
+FXD float fx_div_small(float x, double d, double rcp) {
+    const double q = __dmul_rn((double)x, rcp);
+    const float r = (float)__fma_rn(__fma_rn(-q, d, (double)x), rcp, q);
+    return x == 0.0f || !(fabsf(x) <= 3.402823466e38f) ? x : r;
+}
+
 // Jacobi constants as pairs, for fx_jacobi4.
 struct FxJacobiConst2 {
     fx_f2 rcp, negDenom;
     float wxS, wyS, wzS, denom, rcpS;
     bool fast;
+    float lo;                   // TWO: the smallest numerator the two operations are right for,
+    const volatile double* rcpD;  // and where RN(1 / denom) is (read in the rare path only)
 };
 FXD FxJacobiConst2 fx_jacobi_const2(const FxJacobiConst& c, float rcp, bool fast) {
-    return FxJacobiConst2{fx_pack2(rcp, rcp), fx_pack2(-c.denom, -c.denom), c.wx, c.wy, c.wz, c.denom, rcp, fast};
+    return FxJacobiConst2{fx_pack2(rcp, rcp), fx_pack2(-c.denom, -c.denom), c.wx, c.wy, c.wz, c.denom, rcp, fast, 0.0f, nullptr};
+}
+// ... for the two-operation quotient (rcp and negDenom hold the two parts of 1 / denom).
+FXD FxJacobiConst2 fx_jacobi_const2_two(const FxSimDev& S) {
+    return FxJacobiConst2{fx_pack2(S.jcRh, S.jcRh), fx_pack2(S.jcRl, S.jcRl), S.jc[0], S.jc[1], S.jc[2], S.jc[3], 0.0f, true,
+                          S.jcLo, &S.jcRcpD};
 }
 
 // The end of fx_jacobi4 from the six weighted pair sums: the numerators and the division.
-template <bool INLINE_RARE>
+template <bool INLINE_RARE, bool TWO>
 FXD float4 fx_jacobi4_finish(const FxJacobiConst2& c, fx_f2 x01, fx_f2 x23, fx_f2 y01, fx_f2 y23, fx_f2 z01, fx_f2 z23,
                              float4 d) {
     const fx_f2 n01 = fx_sub2(fx_add2(fx_add2(x01, y01), z01), fx_pack2(d.x, d.y));
     const fx_f2 n23 = fx_sub2(fx_add2(fx_add2(x23, y23), z23), fx_pack2(d.z, d.w));
     const float2 a = fx_unpack2(n01), b = fx_unpack2(n23);
+    if (TWO) {
+        const float2 u = fx_unpack2(fx_fma2(n01, c.rcp, fx_mul2(n01, c.negDenom)));
+        const float2 v = fx_unpack2(fx_fma2(n23, c.rcp, fx_mul2(n23, c.negDenom)));
+        const float least = fminf(fminf(fabsf(a.x), fabsf(a.y)), fminf(fabsf(b.x), fabsf(b.y)));
+        if (least >= c.lo) return make_float4(u.x, u.y, v.x, v.y);
+        const double D = c.denom, R = *c.rcpD;
+        return make_float4(fx_div_small(a.x, D, R), fx_div_small(a.y, D, R), fx_div_small(b.x, D, R), fx_div_small(b.y, D, R));
+    }
     if (!c.fast) return make_float4(__fdiv_rn(a.x, c.denom), __fdiv_rn(a.y, c.denom), __fdiv_rn(b.x, c.denom), __fdiv_rn(b.y, c.denom));
     // Markstein's step on both pairs: q = x rcp, e = fma(q, -d, x) = x - q d, q + e rcp
     const fx_f2 q01 = fx_mul2(n01, c.rcp), q23 = fx_mul2(n23, c.rcp);
@@ -713,17 +737,20 @@ FXD float4 fx_jacobi4_finish(const FxJacobiConst2& c, fx_f2 x01, fx_f2 x23, fx_f
 // A group with a numerator outside the checked range takes the IEEE division for its four
 // cells (the same quotients: inside the range the checked path equals it), through the
 // out-of-line rare path of fx_div_by_const, or inline (INLINE_RARE: no call in the caller's
-// loop; measured faster in the resident kernel at HD, 5.60 against 6.02 us per sweep, and
-// 1 % slower in the two-sweep kernel at 508^3).
+// loop; measured faster in the resident kernel at HD, 5.60 against 6.02 us per sweep).
 // A packed multiply feeding a packed add is contracted into a packed fma by the code
 // generator (measured on B200), which rounds once instead of twice, so the weight products
 // are either scalar multiplies (never contracted) or, with PACKED_W, packed fused
 // multiply-adds of -0: RN(w s + -0) = RN(w s) for every w and s, zeros' signs included, and
 // an fma feeding an add is not contracted. The -0 is computed from the run-time divisor
 // (finite), so the fma cannot be folded back into a multiply. PACKED_W measured 5.61
-// against 5.65 us per sweep in the resident kernel with the copy warp at HD, and 1 % slower
-// per step in the two-sweep kernel at 508^3.
-template <bool INLINE_RARE = false, bool PACKED_W = false>
+// against 5.65 us per sweep in the resident kernel with the copy warp at HD.
+// TWO: the two-operation quotient instead of Markstein's three and their IEEE fallback, one
+// compare of the smallest magnitude instead of eight, and double precision for a group with
+// a numerator below c.lo or a zero: 128x192x128, 200 sweeps, 1,115 against 1,124 us; the first
+// steps of a fluid at rest, whose fronts are zeros and tiny numerators, 128 sweeps, 1,210
+// against 3,345 us.
+template <bool INLINE_RARE = false, bool PACKED_W = false, bool TWO = false>
 FXD float4 fx_jacobi4(const FxJacobiConst2& c, float l, float4 pc, float r, float4 pb, float4 pt, float4 pk, float4 pf,
                       float4 d) {
     const fx_f2 mid = fx_pack2(pc.y, pc.z);
@@ -737,7 +764,7 @@ FXD float4 fx_jacobi4(const FxJacobiConst2& c, float l, float4 pc, float r, floa
         const float nzs = -0.0f * fabsf(c.denom);
         const fx_f2 nz = fx_pack2(nzs, nzs);
         const fx_f2 wx2 = fx_pack2(c.wxS, c.wxS), wy2 = fx_pack2(c.wyS, c.wyS), wz2 = fx_pack2(c.wzS, c.wzS);
-        return fx_jacobi4_finish<INLINE_RARE>(c, fx_fma2(wx2, lr01, nz), fx_fma2(wx2, lr23, nz), fx_fma2(wy2, bt01, nz),
+        return fx_jacobi4_finish<INLINE_RARE, TWO>(c, fx_fma2(wx2, lr01, nz), fx_fma2(wx2, lr23, nz), fx_fma2(wy2, bt01, nz),
                                               fx_fma2(wy2, bt23, nz), fx_fma2(wz2, kf01, nz), fx_fma2(wz2, kf23, nz), d);
     } else {
         const float2 s01 = fx_unpack2(lr01), s23 = fx_unpack2(lr23), u01 = fx_unpack2(bt01), u23 = fx_unpack2(bt23);
@@ -748,7 +775,7 @@ FXD float4 fx_jacobi4(const FxJacobiConst2& c, float l, float4 pc, float r, floa
         const fx_f2 y23 = fx_pack2(__fmul_rn(c.wyS, u23.x), __fmul_rn(c.wyS, u23.y));
         const fx_f2 z01 = fx_pack2(__fmul_rn(c.wzS, v01.x), __fmul_rn(c.wzS, v01.y));
         const fx_f2 z23 = fx_pack2(__fmul_rn(c.wzS, v23.x), __fmul_rn(c.wzS, v23.y));
-        return fx_jacobi4_finish<INLINE_RARE>(c, x01, x23, y01, y23, z01, z23, d);
+        return fx_jacobi4_finish<INLINE_RARE, TWO>(c, x01, x23, y01, y23, z01, z23, d);
     }
 }
 
@@ -759,15 +786,6 @@ FXD float4 fx_jacobi4(const FxJacobiConst2& c, float l, float4 pc, float r, floa
 // a d only after checking on the device that it equals x / d for every float x, with quotients
 // of 0 < |x| < lo taken by fx_div_small; of 1,450 denominators of grids tried it is exact for
 // 1,428 with one of five roundings of rl. rl > 0 keeps zeros' signs, infinities and NaN.
-//
-// RN(x / d) for any finite x through double precision: the product by rcp = RN(1/d) with one
-// correction step is the correctly rounded double quotient, whose rounding to float is x / d
-// (53 >= 2 * 24 + 2 bits). Zeros, infinities and NaN are returned as they are.
-FXD float fx_div_small(float x, double d, double rcp) {
-    const double q = __dmul_rn((double)x, rcp);
-    const float r = (float)__fma_rn(__fma_rn(-q, d, (double)x), rcp, q);
-    return x == 0.0f || !(fabsf(x) <= 3.402823466e38f) ? x : r;
-}
 FXD float fx_div_two(float x, float rh, float rl, float lo, double d, double rcp) {
     const float r = __fmaf_rn(x, rh, __fmul_rn(x, rl));
     return fabsf(x) < lo ? fx_div_small(x, d, rcp) : r;

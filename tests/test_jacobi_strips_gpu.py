@@ -128,3 +128,19 @@ def test_registers_survive_a_change_of_members():
         s.step(1, DT)
     for a, m in zip(alone, sims):
         same(a, m)
+
+
+# ---- the copy-warp kernel's two-operation quotient (fx_jacobi_res.cuh, long columns) ------------
+
+@pytest.mark.parametrize("P,R,noise,mode", [(40, 24, 0.0, A.PRESSURE_WARM_F32), (40, 24, 0.0, A.PRESSURE_COLD_F32),
+                                            (1, 2, 0.18, A.PRESSURE_WARM_F32)])
+def test_copy_warp_from_rest(P, R, noise, mode):
+    dims = (128, 192, 128)
+    opts = sphere_options(dims, P=P, R=R, noise=noise, pressure_mode=mode)
+    one, res = FireXSim(dims, opts), FireXSim(dims, opts)
+    one.set_jacobi("unblocked")
+    one.step(2, DT)
+    res.step(2, DT)
+    d = res.diagnostics
+    assert d["jacobi_kernel"] == A.JACOBI_RESIDENT and d["jacobi_variant"] == 4, d
+    same(one, res)
