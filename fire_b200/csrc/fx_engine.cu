@@ -1029,8 +1029,8 @@ struct firex_batch {
         p.simBy = by ? by : FX_CELL_BY;
         // the fused projection recomputes its backward neighbours from loads that hit L2 while
         // the batch's fields fit there; from 8 Mi cells they come from HBM and two passes are
-        // faster (measured on B200, 508^3: 2.84 + 0.66 ms fused against 1.95 + 1.32 ms; HD:
-        // 0.118 against 0.125 ms)
+        // faster (measured on B200, fused against a projection and a divergence pass: 160x240x160
+        // 82 / 83 us, 188x284x196 135 / 127, 508^3 1,660 / 1,430)
         const int pf = this->projFuse != FIREX_PROJECT_AUTO ? this->projFuse : members[0]->projFuse;
         p.projDiv = pf == FIREX_PROJECT_FUSED || (pf == FIREX_PROJECT_AUTO && cells < (8LL << 20));
         // the source pass's neighbour terms ahead of the advection below 12 Mi cells (measured on

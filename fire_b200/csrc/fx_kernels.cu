@@ -329,10 +329,13 @@ __global__ void __launch_bounds__(256) fxk_jacobi(const FxBatchDev* __restrict__
 // The solve's result sits in the buffer after its last launch; launch counts have the
 // parity of the sweep counts (the engine only fuses sweeps when they do), so the result
 // buffer is the reference's: p[(base + P) & 1] and corr[R & 1].
-// 8 CTAs per SM (32 registers, some spilled): 18 % faster than the 5 that 48 registers allow
-// at 508^3 (latency-bound: more loads in flight); the divergence kernel is fastest at 57.
+// Bound by HBM (36 bytes a cell; 508^3 738 us a pass, 97 % of the measured copy rate, against 994
+// when each cell was finished before the next one's loads): every load of the lane's four cells is
+// issued first, half pressures as stored (converted between the loads they kept them from being
+// batched: 412x616x412 844 us a pass against 579). 64 registers hold them; at five CTAs per SM some
+// spill (508^3 1,078 us), at three fewer loads are in flight (840).
 template <typename PT>
-__global__ void __launch_bounds__(256, 8) fxk_project(const FxBatchDev* __restrict__ B, int phase) {
+__global__ void __launch_bounds__(256, 4) fxk_project(const FxBatchDev* __restrict__ B, int phase) {
     fx_for_bricks<FX_SHAPE_ROW4>(B, [&](const FxSimDev& S, int b) {
         const Lane4 r = fx_lane4(S, b);
         if (r.n <= 0) return;
@@ -357,24 +360,35 @@ __global__ void __launch_bounds__(256, 8) fxk_project(const FxBatchDev* __restri
         const int X = S.X, XY = S.X * S.Y;
         int xs[4], ys[4], zs[4];
         fx_lane4_coords(S, r, xs, ys, zs);
+        float4 f[4];
+        typename PStore<PT>::Raw rc[4], rx[4], rt[4], rf[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            f[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            rc[i] = rx[i] = rt[i] = rf[i] = 0;
+            if (lane + 32 * i < r.n) {
+                const int c = r.c0 + 32 * i;
+                const int cs = (ys[i] == S.Y - 1) ? c - X : c;  // top row: the projected row below
+                f[i] = __ldg(flowIn + c);
+                if (!zeroP) {
+                    rc[i] = PStore<PT>::raw(p, cs);
+                    rx[i] = PStore<PT>::raw(p, xs[i] + 1 < X ? cs + 1 : cs);
+                    rt[i] = PStore<PT>::raw(p, cs + X);  // the row above the source row is in the grid
+                    rf[i] = PStore<PT>::raw(p, zs[i] < S.Z - 1 ? cs + XY : cs);
+                }
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (lane + 32 * i < r.n) {
                 const int c = r.c0 + 32 * i;
-                const int cs = (ys[i] == S.Y - 1) ? c - X : c;  // top row: the projected row below
-                const float4 f = __ldg(flowIn + c);
-                const float4 src = (cs == c) ? f : __ldg(flowIn + cs);
-                float pc = 0.0f, px = 0.0f, pt = 0.0f, pf = 0.0f;
-                if (!zeroP) {
-                    pc = PStore<PT>::ld(p, cs);
-                    px = xs[i] + 1 < X ? PStore<PT>::ld(p, cs + 1) : pc;
-                    pt = PStore<PT>::ld(p, cs + X);  // the row above the source row is in the grid
-                    pf = zs[i] < S.Z - 1 ? PStore<PT>::ld(p, cs + XY) : pc;
-                }
-                const float gx = (px - pc) * m.x;
-                const float gy = (pt - pc) * m.y;
-                const float gz = (pf - pc) * m.z;
-                float4 o = make_float4(src.x - gx, src.y - gy, src.z - gz, f.w);
+                float4 src = f[i];
+                if (ys[i] == S.Y - 1) src = __ldg(flowIn + c - X);
+                const float pc = PStore<PT>::of(rc[i]);
+                const float gx = (PStore<PT>::of(rx[i]) - pc) * m.x;
+                const float gy = (PStore<PT>::of(rt[i]) - pc) * m.y;
+                const float gz = (PStore<PT>::of(rf[i]) - pc) * m.z;
+                float4 o = make_float4(src.x - gx, src.y - gy, src.z - gz, f[i].w);
                 if (xs[i] == 0 || xs[i] == X - 1) o.x = 0.0f;
                 if (zs[i] == 0 || zs[i] == S.Z - 1) o.z = 0.0f;
                 if (ys[i] == 0) o.y = 0.0f;
@@ -397,44 +411,15 @@ __global__ void __launch_bounds__(256, 8) fxk_project(const FxBatchDev* __restri
 //   v of the row below:    the projection of (x, y - 1, z), never a top-row cell;
 //   w of the plane behind: the projection of (x, y, z - 1), from the row below when y is the
 //                          top row (the top row copies the projected row below).
-// The extra loads (one component of the flow and one pressure value per neighbour) hit
-// L1/L2: the rows and planes behind were read by the warps and CTAs before.
+// The extra loads (one component of the flow and one pressure value per neighbour; the other
+// pressure is the cell's own) hit L1/L2: the rows and planes behind were read by the warps and CTAs
+// before. Bound by L2 and latency: all loads of the lane's four cells are issued before the
+// arithmetic (100 registers, two CTAs per SM: 128x192x128 43 us with the residual's epilogue, 49
+// when each cell was finished by itself, 47 at 80 registers with some spilled; 32x48x32 8.4
+// against 12.9 us).
 #ifndef FX_PROJDIV_MINB
-#define FX_PROJDIV_MINB 6  // CTAs per SM the fused projection's registers are budgeted for
+#define FX_PROJDIV_MINB 2  // CTAs per SM the fused projection's registers are budgeted for
 #endif
-template <typename PT>
-struct ProjSrc {
-    const float4* __restrict__ flowIn;
-    const void* p;
-    bool zeroP;
-    int X, Y, Z, XY;
-    float3 m;
-    FXD float pr(int i) const { return zeroP ? 0.0f : PStore<PT>::ld(p, i); }
-    // u of cell c = (x, y, z), x in [1, X - 2] (the walls force u = 0 and need no load)
-    FXD float u(int c, int x, int y) const {
-        if (x == 0 || x == X - 1) return 0.0f;
-        const int cs = (y == Y - 1) ? c - X : c;
-        const float pc = pr(cs);
-        const float px = pr(cs + 1);
-        return __ldg(&flowIn[cs].x) - (px - pc) * m.x;
-    }
-    // v of cell c = (x, y, z) with y <= Y - 2
-    FXD float v(int c, int y) const {
-        if (y == 0) return 0.0f;
-        const float pc = pr(c);
-        const float pt = pr(c + X);
-        return __ldg(&flowIn[c].y) - (pt - pc) * m.y;
-    }
-    // w of cell c = (x, y, z) with z <= Z - 2
-    FXD float w(int c, int y, int z) const {
-        if (z == 0) return 0.0f;
-        const int cs = (y == Y - 1) ? c - X : c;
-        const float pc = pr(cs);
-        const float pf = pr(cs + XY);
-        return __ldg(&flowIn[cs].z) - (pf - pc) * m.z;
-    }
-};
-
 template <typename PT>
 __global__ void __launch_bounds__(256, FX_PROJDIV_MINB) fxk_project_div(const FxBatchDev* __restrict__ B) {
     fx_for_bricks<FX_SHAPE_ROW4>(B, [&](const FxSimDev& S, int b) {
@@ -442,49 +427,78 @@ __global__ void __launch_bounds__(256, FX_PROJDIV_MINB) fxk_project_div(const Fx
         if (r.n <= 0) return;  // warp-uniform
         const int lane = threadIdx.x & 31;
         const int base = (S.mode == FIREX_PRESSURE_COLD_F32) ? 0 : S.pi;
-        ProjSrc<PT> src{reinterpret_cast<const float4*>(S.flow[S.fi ^ 1]), S.p[(base + S.P) & 1],
-                        S.mode == FIREX_PRESSURE_COLD_F32 && S.P == 0, S.X, S.Y, S.Z, S.X * S.Y, fx_metric(S.prm.u)};
+        const float4* __restrict__ flowIn = reinterpret_cast<const float4*>(S.flow[S.fi ^ 1]);
+        const void* p = S.p[(base + S.P) & 1];
+        const bool zeroP = S.mode == FIREX_PRESSURE_COLD_F32 && S.P == 0;
+        const float3 m = fx_metric(S.prm.u);
         float4* __restrict__ flowOut = reinterpret_cast<float4*>(S.flow[S.fi]);
         const int X = S.X, XY = S.X * S.Y;
         int xs[4], ys[4], zs[4];
         fx_lane4_coords(S, r, xs, ys, zs);
         // u of the cell before lane 0's first cell (another warp's or brick's cell)
-        float prevU = (lane == 0 && xs[0] > 0) ? src.u(r.c0 - 1, xs[0] - 1, ys[0]) : 0.0f;
+        float prevU = 0.0f;  // (0 on a wall, at x = 0)
+        if (lane == 0 && xs[0] > 1) {
+            const int cs = r.c0 - 1 - (ys[0] == S.Y - 1 ? X : 0);
+            float pl = 0.0f, pr = 0.0f;
+            if (!zeroP) {
+                pl = PStore<PT>::ld(p, cs);
+                pr = PStore<PT>::ld(p, cs + 1);
+            }
+            prevU = __ldg(&flowIn[cs].x) - (pr - pl) * m.x;
+        }
+        float4 f[4];
+        float fy[4], fz[4];  // v of the row below and w of the plane behind, before their projection
+        typename PStore<PT>::Raw rc[4], rx[4], rt[4], rf[4], rb[4], rk[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            // each of the lane's cells is finished in its own iteration: only the u that the
-            // next group's first lane needs is carried (registers for more CTAs per SM)
-            const bool valid = lane + 32 * i < r.n;
+            f[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            fy[i] = fz[i] = 0.0f;
+            rc[i] = rx[i] = rt[i] = rf[i] = rb[i] = rk[i] = 0;
+            if (lane + 32 * i < r.n) {
+                const int c = r.c0 + 32 * i;
+                const int cs = (ys[i] == S.Y - 1) ? c - X : c;  // top row: the projected row below
+                f[i] = __ldg(flowIn + c);
+                if (ys[i] > 1) fy[i] = __ldg(&flowIn[c - X].y);
+                if (zs[i] > 1) fz[i] = __ldg(&flowIn[cs - XY].z);
+                if (!zeroP) {
+                    rc[i] = PStore<PT>::raw(p, cs);
+                    rx[i] = PStore<PT>::raw(p, xs[i] + 1 < X ? cs + 1 : cs);
+                    rt[i] = PStore<PT>::raw(p, cs + X);
+                    rf[i] = PStore<PT>::raw(p, zs[i] < S.Z - 1 ? cs + XY : cs);
+                    if (ys[i] > 1) rb[i] = PStore<PT>::raw(p, c - X);
+                    if (zs[i] > 1) rk[i] = PStore<PT>::raw(p, cs - XY);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool valid = lane + 32 * i < r.n, top = ys[i] == S.Y - 1;
             const int c = r.c0 + 32 * i;
             float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             float vb = 0.0f, wk = 0.0f;
             if (valid) {
-                const int cs = (ys[i] == S.Y - 1) ? c - X : c;  // top row: the projected row below
-                const float4 f = __ldg(src.flowIn + c);
-                const float4 s = (cs == c) ? f : __ldg(src.flowIn + cs);
-                float pc = 0.0f, px = 0.0f, pt = 0.0f, pf = 0.0f;
-                if (!src.zeroP) {
-                    pc = PStore<PT>::ld(src.p, cs);
-                    px = xs[i] + 1 < X ? PStore<PT>::ld(src.p, cs + 1) : pc;
-                    pt = PStore<PT>::ld(src.p, cs + X);
-                    pf = zs[i] < S.Z - 1 ? PStore<PT>::ld(src.p, cs + XY) : pc;
-                }
-                const float gx = (px - pc) * src.m.x;
-                const float gy = (pt - pc) * src.m.y;
-                const float gz = (pf - pc) * src.m.z;
-                q = make_float4(s.x - gx, s.y - gy, s.z - gz, f.w);
+                float4 s = f[i];
+                if (top) s = __ldg(flowIn + c - X);
+                const float pc = PStore<PT>::of(rc[i]), pt = PStore<PT>::of(rt[i]);
+                const float gx = (PStore<PT>::of(rx[i]) - pc) * m.x;
+                const float gy = (pt - pc) * m.y;
+                const float gz = (PStore<PT>::of(rf[i]) - pc) * m.z;
+                q = make_float4(s.x - gx, s.y - gy, s.z - gz, f[i].w);
                 if (xs[i] == 0 || xs[i] == X - 1) q.x = 0.0f;
                 if (zs[i] == 0 || zs[i] == S.Z - 1) q.z = 0.0f;
                 if (ys[i] == 0) q.y = 0.0f;
-                if (ys[i] == S.Y - 1) q.y = fx_max(0.0f, q.y);
+                if (top) q.y = fx_max(0.0f, q.y);
                 flowOut[c] = q;
-                vb = ys[i] > 0 ? src.v(c - X, ys[i] - 1) : q.y;
-                wk = zs[i] > 0 ? src.w(c - XY, ys[i], zs[i] - 1) : q.z;
+                // rows 0 and planes 0 are walls (0); a top cell's own pressure is pt, any other's pc
+                const float vp = ys[i] > 1 ? fy[i] - ((top ? pt : pc) - PStore<PT>::of(rb[i])) * m.y : 0.0f;
+                const float wp = zs[i] > 1 ? fz[i] - (pc - PStore<PT>::of(rk[i])) * m.z : 0.0f;
+                vb = ys[i] > 0 ? vp : q.y;
+                wk = zs[i] > 0 ? wp : q.z;
             }
             const float fromLeft = __shfl_up_sync(0xffffffffu, q.x, 1);
             const float ul = xs[i] == 0 ? q.x : (lane > 0 ? fromLeft : prevU);
             prevU = __shfl_sync(0xffffffffu, q.x, 31);
-            if (valid) S.div[c] = (q.x - ul) * src.m.x + (q.y - vb) * src.m.y + (q.z - wk) * src.m.z;
+            if (valid) S.div[c] = (q.x - ul) * m.x + (q.y - vb) * m.y + (q.z - wk) * m.z;
         }
     });
 }
@@ -675,16 +689,27 @@ FXD uint2 fx_half4(float a, float b, float c, float d) {
     r.y = *reinterpret_cast<const uint32_t*>(&hi);
     return r;
 }
-FXD void fx_pack_cell(const FxSimDev& S, int id, int x, int y, int z, bool view7, const float3& m) {
+struct FxPackIn {
+    float4 f, sr;
+    float reaction;
+    int liquid;
+};
+FXD FxPackIn fx_pack_load(const FxSimDev& S, int id) {
+    FxPackIn a;
+    a.f = __ldg(reinterpret_cast<const float4*>(S.flow[S.fi]) + id);
+    a.sr = S.storage == FX_STORAGE_MIXED ? StMixed::ld_species(S.species[S.si], id) : StF32::ld_species(S.species[S.si], id);
+    a.reaction = __ldg(S.reaction + id);
+    a.liquid = __ldg(S.liquid + id);
+    return a;
+}
+FXD void fx_pack_cell(const FxSimDev& S, const FxPackIn& a, int id, int x, int y, int z, bool view7, const float3& m) {
     const float4* flow = reinterpret_cast<const float4*>(S.flow[S.fi]);
-    const float4 f = __ldg(flow + id);
-    const float4 sr = S.storage == FX_STORAGE_MIXED ? StMixed::ld_species(S.species[S.si], id)
-                                                    : StF32::ld_species(S.species[S.si], id);
+    const float4 f = a.f, sr = a.sr;
     const float4 sp = make_float4(fx_max(sr.x, 0.0f), fx_max(sr.y, 0.0f), fx_max(sr.z, 0.0f), fx_max(sr.w, 0.0f));
-    const float reaction = fx_clamp(__ldg(S.reaction + id), 0.0f, 4.0f);
+    const float reaction = fx_clamp(a.reaction, 0.0f, 4.0f);
     const float richness = fx_clamp(sp.x / fx_max(sp.x + sp.y * 0.25f, FC(0.0001)), 0.0f, 1.0f);
     const float soot = sp.z * fx_smoothstep(0.25f, FC(0.82), richness);
-    const float liq = (float)__ldg(S.liquid + id) * FC(3.4 / 4096.0);
+    const float liq = (float)a.liquid * FC(3.4 / 4096.0);
     float disp = fx_max(fx_max(reaction, soot), fx_max(liq, fx_max(sp.w, fx_smoothstep(420.0f, 700.0f, f.w))));
     if (view7) {
         const bool shell = x == 0 || y == 0 || z == 0 || x + 1 >= S.X || y + 1 >= S.Y || z + 1 >= S.Z;
@@ -711,12 +736,14 @@ __global__ void fxk_pack_sim(const FxSimDev* __restrict__ Sp) {
     const bool v7 = fx_view7(S.prm.u);
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
         const int x = id % S.X, t = id / S.X, y = t % S.Y, z = t / S.Y;
-        fx_pack_cell(S, id, x, y, z, v7, m);
+        fx_pack_cell(S, fx_pack_load(S, id), id, x, y, z, v7, m);
     }
 }
 
-// Every member that packs each step, after the step's end (canonical buffers current).
-__global__ void __launch_bounds__(256) fxk_pack_batch(const FxBatchDev* __restrict__ B) {
+// Every member that packs each step, after the step's end (canonical buffers current). Bound by HBM
+// (64 bytes a cell with FP32 records): the lane's four cells are loaded before the first is packed,
+// 508^3 2.01 -> 1.53 ms, 300x452x276 0.58 -> 0.44 (80 registers; at 64 0.51, at 128 0.55).
+__global__ void __launch_bounds__(256, 3) fxk_pack_batch(const FxBatchDev* __restrict__ B) {
     fx_for_bricks<FX_SHAPE_ROW4>(B, [&](const FxSimDev& S, int b) {
         if (!S.renderPack) return;
         const Lane4 r = fx_lane4(S, b);
@@ -726,9 +753,13 @@ __global__ void __launch_bounds__(256) fxk_pack_batch(const FxBatchDev* __restri
         const bool v7 = fx_view7(S.prm.u);
         int xs[4], ys[4], zs[4];
         fx_lane4_coords(S, r, xs, ys, zs);
+        FxPackIn a[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            if (lane + 32 * i < r.n) fx_pack_cell(S, r.c0 + 32 * i, xs[i], ys[i], zs[i], v7, m);
+            if (lane + 32 * i < r.n) a[i] = fx_pack_load(S, r.c0 + 32 * i);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (lane + 32 * i < r.n) fx_pack_cell(S, a[i], r.c0 + 32 * i, xs[i], ys[i], zs[i], v7, m);
     });
 }
 

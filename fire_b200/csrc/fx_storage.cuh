@@ -43,6 +43,10 @@ struct PStore;
 template <>
 struct PStore<float> {
     FXD static float ld(const void* b, long long i) { return __ldg(reinterpret_cast<const float*>(b) + i); }
+    // an element as stored, to be converted once every load is issued
+    using Raw = float;
+    FXD static Raw raw(const void* b, long long i) { return ld(b, i); }
+    FXD static float of(Raw r) { return r; }
     FXD static float4 ld4(const void* b, long long i) { return __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(b) + i)); }
     FXD static void st4(void* b, long long i, float4 v) { *reinterpret_cast<float4*>(reinterpret_cast<float*>(b) + i) = v; }
     FXD static float round(float v) { return v; }
@@ -50,6 +54,9 @@ struct PStore<float> {
 template <>
 struct PStore<__half> {
     FXD static float ld(const void* b, long long i) { return __half2float(__ldg(reinterpret_cast<const __half*>(b) + i)); }
+    using Raw = unsigned short;
+    FXD static Raw raw(const void* b, long long i) { return __ldg(reinterpret_cast<const unsigned short*>(b) + i); }
+    FXD static float of(Raw r) { return __half2float(__ushort_as_half(r)); }
     FXD static float4 ld4(const void* b, long long i) {
         uint2 r = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(b) + i));
         float2 a = __half22float2(*reinterpret_cast<__half2*>(&r.x));
