@@ -80,12 +80,6 @@ FXD float fx_divc(float x, const FxDivc& c) {
     return fx_div_range(x, v.x, v.y, v.z, v.w);
 }
 
-// smoothstep with its constant denominator e1 - e0 held in c.
-FXD float fx_smoothstep_c(float e0, float x, const FxDivc& c) {
-    float t = fx_clamp(fx_divc(x - e0, c), 0.0f, 1.0f);
-    return t * t * (3.0f - 2.0f * t);
-}
-
 struct FxQuad {  // four values as two pairs: four consecutive x cells, or a cell's record
     float2 a, b;
 };
@@ -883,11 +877,5 @@ FXD float fx_jacobi_cell(const FxJacobiK<TWO>& K, float l, float r, float b, flo
     const float n = fx_jacobi_numerator(FxJacobiConst{K.wx, K.wy, K.wz, K.denom}, l, r, b, t, k, f, div);
     if (TWO) return fx_div_two(n, K.rh, K.rl, K.lo, K.denom, K.rcpD);
     return fx_div_small(n, K.denom, K.rcpD);
-}
-
-// One cell of fx_jacobi4 (the same numerator; the checked constant division when enabled).
-FXD float fx_jacobi1(const FxJacobiConst2& c, float l, float r, float b, float t, float k, float f, float div) {
-    const float n = fx_jacobi_numerator(FxJacobiConst{c.wxS, c.wyS, c.wzS, c.denom}, l, r, b, t, k, f, div);
-    return c.fast ? fx_div_by_const(n, c.denom, c.rcpS) : __fdiv_rn(n, c.denom);
 }
 
