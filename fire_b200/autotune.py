@@ -33,7 +33,7 @@ class Candidate:
     kernel: str
     block: int = 0
     zchunk: int = 0
-    staging: int = A.STAGING_AUTO  # two-sweep pass: cp.async (AUTO) or TMA (FP32 pressure)
+    staging: int = A.STAGING_AUTO  # two-sweep pass: cp.async or TMA (FP32 pressure)
     simulate_by: int = 0           # source-pass bricks: 32 x by x (8 / by); 0 = default
     project: int = A.PROJECT_AUTO  # primary projection fused with the residual divergence or not
 

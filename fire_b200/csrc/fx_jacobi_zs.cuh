@@ -24,7 +24,7 @@
 // Measured on B200: bound by the latency of a step at 16 warps per SM (issue slots 44 % busy,
 // shared memory 64 %) and, at 508^3, by the power cap; 508^3 31.4 ms of Jacobi per step of 96 + 96
 // sweeps against 45.2 for the former 32 x 30 tiles of one row to a thread, whose every neighbour
-// came from shared memory (39 instructions per cell and sweep; 17 here); 160x240x160 2.14 ms
+// came from shared memory (39 instructions per cell and sweep; 20 here); 160x240x160 2.14 ms
 // against 3.95 for single sweeps from L2. Small CTAs because the step barrier is what the warps
 // wait for: 508^3 with cp.async 36.0 ms with 8 warps and 64 columns, 33.5 with 4, 35.3 with 2 and 32
 // columns; twelve uneven grids 17.2, 14.8 and 13.8. One row to a thread at 80 registers and 24

@@ -36,7 +36,7 @@ def main() -> None:
     ap.add_argument("--profile", action="store_true", help="per-pass device times (no graph replay)")
     ap.add_argument("--time", type=int, default=0, help="then time this many steps (graph replay)")
     ap.add_argument("--staging", default="auto", choices=["auto", "cpasync", "tma"],
-                    help="plane staging of the two-sweep pass (auto: cp.async)")
+                    help="plane staging of the two-sweep pass (auto: tma where auto chose the pass, FP32)")
     ap.add_argument("--project", default="auto", choices=["auto", "fused", "separate"],
                     help="primary projection and residual divergence in one pass or two")
     ap.add_argument("--simulate-by", type=int, default=0, choices=[0, 2, 4, 8], help="source-pass brick height")

@@ -38,8 +38,9 @@ from .sim import FireXBatch, FireXSim, make_options, planned_device_bytes
 DEFAULT_BUDGET = 150 * 10**9
 DEFAULT_TICK_MS = 40.0
 # Device cost of one member step outside the Jacobi sweeps (simulate, divergence, both
-# projections), in Jacobi cell-sweep equivalents; measured on B200 at 508^3: simulate 8.7 ms,
-# divergence and projections 3.3 ms against 1.79 ns per cell-sweep of the two-sweep pass.
+# projections), in Jacobi cell-sweep equivalents; measured on B200 at 508^3: simulate 8.0 ms,
+# divergence and projections 2.8 ms against 1.25 ps per cell-sweep of the two-sweep pass (66; on small
+# grids 30 to 60).
 FIXED_SWEEP_EQUIVALENTS = 50
 
 
