@@ -39,8 +39,8 @@ DEFAULT_BUDGET = 150 * 10**9
 DEFAULT_TICK_MS = 40.0
 # Device cost of one member step outside the Jacobi sweeps (simulate, divergence, both
 # projections), in Jacobi cell-sweep equivalents; measured on B200 at 508^3: simulate 8.0 ms,
-# divergence and projections 2.8 ms against 1.25 ps per cell-sweep of the two-sweep pass (66; on small
-# grids 30 to 60).
+# divergence and projections 2.8 ms against 1.25 ps per cell-sweep of the two-sweep pass (66; 39 at
+# 128x192x128, 41 at 160x240x160).
 FIXED_SWEEP_EQUIVALENTS = 50
 
 
