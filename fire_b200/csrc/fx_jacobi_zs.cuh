@@ -33,6 +33,7 @@
 
 #include "fx_async.cuh"
 #include "fx_jacobi_zm.cuh"  // cp.async helpers
+#include "fx_plan.h"
 #include "fx_step_math.cuh"
 #include "fx_storage.cuh"
 
@@ -104,10 +105,9 @@ FXD void fx_zs_tensor(void* dst, const CUtensorMap* map, int x, int y, int z, un
 FXD void fx_zs_map_acquire(const CUtensorMap* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
 }
-// Index of a plane or row outside 0 .. n - 1 reflected into it (-1 is 0, n is n - 1). The update adds the
-// two neighbours of an axis, so the sweep-1 value of a reflected plane or row is that of its
+// Planes and rows outside the grid are reflected into it (fx_zs_reflect, fx_zs_input_row). The update
+// adds the two neighbours of an axis, so the sweep-1 value of a reflected plane or row is that of its
 // image, which is what sweep 2's clamped neighbour is: the walls need no code of their own.
-FXD int fx_zs_reflect(int q, int n) { return q < 0 ? -1 - q : (q >= n ? 2 * n - 1 - q : q); }
 
 // Two sweeps of planes [z0, z1) of the tile at (x0, y0): pin -> pout. TOP: the tile holds rows at
 // or above the open top.
@@ -124,7 +124,7 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
 #pragma unroll
     for (int k = 0; k < H::KP; ++k) {
         const int i = t + k * FX_ZS_THREADS, row = i / H::SEGS, gx = min(max(x0 - 4 + 4 * (i - row * H::SEGS), 0), X - 4);
-        gP[k] = min(fx_zs_reflect(y0 - 2 + row, Y + 2), Y - 1) * X + gx;
+        gP[k] = fx_zs_input_row(y0 - 2 + row, Y) * X + gx;
     }
 #pragma unroll
     for (int k = 0; k < H::KD; ++k) {

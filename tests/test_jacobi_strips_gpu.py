@@ -144,3 +144,18 @@ def test_copy_warp_from_rest(P, R, noise, mode):
     d = res.diagnostics
     assert d["jacobi_kernel"] == A.JACOBI_RESIDENT and d["jacobi_variant"] == 4, d
     same(one, res)
+
+
+# ---- the flattest grids: a tile's rows reach far above the top --------------------------------
+
+@pytest.mark.parametrize("staging", [A.STAGING_CPASYNC, A.STAGING_TMA])
+@pytest.mark.parametrize("dims", [(4, 4, 4), (36, 4, 12), (64, 4, 20), (36, 8, 12)])
+def test_flat_grids(dims, staging):
+    for zc in (1, 7, 64):
+        pair(dims, zc=zc, staging=staging, P=8, R=8)
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4), (36, 4, 12), (64, 8, 20)])
+def test_flat_grids_fp16_pressure(dims):
+    for zc in (1, 7):
+        pair(dims, zc=zc, P=8, R=8, pressure_mode=A.PRESSURE_F16)
