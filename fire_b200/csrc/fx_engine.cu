@@ -649,14 +649,15 @@ struct firex_sim {
     }
 
     // After a stream synchronisation: whether a bounded device wait of this simulation
-    // expired (the resident Jacobi's group barrier). The fields are then incomplete.
+    // expired (the resident Jacobi's faces, the two-sweep pass's tensor loads). The fields are
+    // then incomplete.
     int check_device_waits() {
         unsigned word = 0;
         cudaError_t e = cudaMemcpy(&word, h.sync + 2, sizeof(word), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "error word");
         if (word != 0) {
             poisoned = true;
-            err = "a bounded device wait expired (resident Jacobi barrier); the step did not complete";
+            err = "a bounded device wait of the Jacobi expired; the step did not complete";
             return FIREX_ERR_TIMEOUT;
         }
         return FIREX_OK;

@@ -13,7 +13,8 @@
 // columns are kept cell by cell, one on a thread.
 //
 // The planes are brought by tensor loads that one thread issues (TMA) or by cp.async, one 4-cell
-// segment to a thread and turn. Waits on the tensor loads are bounded.
+// segment to a thread and turn. Waits on the tensor loads are bounded; a tile whose wait runs out waits
+// once more, so that its loads have landed before the CTA ends, and reports it.
 //
 // The update is fx_jacobi_numerators and the two-operation quotient: each sweep computes the single
 // sweep's FP32 operations, rounds to FP16 as a stored sweep where the pressure is stored so, and
@@ -32,7 +33,8 @@
 #pragma once
 
 #include "fx_async.cuh"
-#include "fx_jacobi_zm.cuh"  // cp.async helpers
+#include "fx_jacobi_res.cuh"  // the words of FxSimDev::sync
+#include "fx_jacobi_zm.cuh"   // cp.async helpers
 #include "fx_plan.h"
 #include "fx_step_math.cuh"
 #include "fx_storage.cuh"
@@ -105,15 +107,22 @@ FXD void fx_zs_tensor(void* dst, const CUtensorMap* map, int x, int y, int z, un
 FXD void fx_zs_map_acquire(const CUtensorMap* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
 }
+// Bounded wait for the phase of bar with the given parity; the limit is read once the first poll has failed.
+FXD bool fx_zs_wait(const FxSimDev& S, unsigned long long* bar, unsigned parity) {
+    if (fx_mbar_try_wait(bar, parity)) return true;
+    const unsigned own = S.sync[FX_SYNC_SPIN];
+    return fx_mbar_wait(bar, parity, own ? own : FX_ZS_WAIT_LIMIT);
+}
 // Planes and rows outside the grid are reflected into it (fx_zs_reflect, fx_zs_input_row). The update
 // adds the two neighbours of an axis, so the sweep-1 value of a reflected plane or row is that of its
 // image, which is what sweep 2's clamped neighbour is: the walls need no code of their own.
 
 // Two sweeps of planes [z0, z1) of the tile at (x0, y0): pin -> pout. TOP: the tile holds rows at
-// or above the open top.
+// or above the open top. held (a test's, firex_test_hold_face): the first planes are waited for with
+// bytes that nothing brings. False when a bounded wait ran out.
 template <typename PT, int TXG, bool ZERO_IN, bool ROUND, bool TWO, bool TOP, bool TMA>
 FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restrict__ pout, int x0, int y0, int z0, int z1,
-                    FxZsSmem<PT, TXG>& sm, const CUtensorMap* mapP, const CUtensorMap* mapD, unsigned& parity) {
+                    FxZsSmem<PT, TXG>& sm, const CUtensorMap* mapP, const CUtensorMap* mapD, unsigned& parity, bool held) {
     using H = FxZsShape<TXG>;
     constexpr int COLS = H::COLS;
     const int X = S.X, Y = S.Y, Z = S.Z, XY = X * Y, t = threadIdx.x;
@@ -157,9 +166,9 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         for (int k = 0; k < H::KD; ++k)
             if (k < H::KD - 1 || lastD) fx_cp_async16(dst + 4 * k * FX_ZS_THREADS, src + gD[k]);
     };
-    // nP input planes and one divergence plane complete the next phase of sm.bar
-    auto expect = [&](int nP) {
-        if (TMA && t == 0) fx_mbar_expect_tx(&sm.bar, (ZERO_IN ? 0 : nP) * BP + BD);
+    // nP input planes, one divergence plane and `more` bytes complete the next phase of sm.bar
+    auto expect = [&](int nP, unsigned more) {
+        if (TMA && t == 0) fx_mbar_expect_tx(&sm.bar, (ZERO_IN ? 0 : nP) * BP + BD + more);
     };
     // the copies requested last have landed, for every thread; false when a bounded wait ran out
     auto landed = [&](bool requested) {
@@ -168,9 +177,11 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
             __syncthreads();
             return true;
         }
-        const bool late = requested && !fx_mbar_wait(&sm.bar, parity, FX_ZS_WAIT_LIMIT);
+        const bool late = requested && !fx_zs_wait(S, &sm.bar, parity);
         if (requested) parity ^= 1u;
-        return !fx_bar_or(0, FX_ZS_THREADS, late);
+        if (!fx_bar_or(0, FX_ZS_THREADS, late)) return true;
+        if (t == 0) fx_zs_wait(S, &sm.bar, parity ^ 1u);  // the one phase in flight
+        return false;
     };
     const FxJacobiK<TWO> K = fx_jacobi_k<TWO>(S);
     constexpr int ROWS = H::ROWS;
@@ -249,7 +260,7 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         constexpr int C = decltype(slot)::value, N = (C + 1) % 3, M = (C + 2) % 3;
         if (!landed(z != zs)) return false;  // planes up to z + 1 are here; plane z - 1's input and z - 2's other slots are free
         if (z < z1) {
-            expect(1);
+            expect(1, 0);
             issueP(z + 2, M);
             issueD(z + 1, N);
             if (!TMA) fx_cp_commit();
@@ -297,7 +308,7 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         return true;
     };
     // slots: plane z in slot (z - zs) mod 3, plane zs - 1 in slot 2 until step zs
-    expect(3);
+    expect(3, held ? 16 : 0);
     issueP(zs - 1, 2);
     issueP(zs, 0);
     issueP(zs + 1, 1);

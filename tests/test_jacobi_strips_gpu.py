@@ -159,3 +159,39 @@ def test_flat_grids(dims, staging):
 def test_flat_grids_fp16_pressure(dims):
     for zc in (1, 7):
         pair(dims, zc=zc, P=8, R=8, pressure_mode=A.PRESSURE_F16)
+
+
+# ---- a wait on tensor loads that runs out -------------------------------------------------------
+
+def test_unfinished_tensor_loads_expire_the_wait():
+    """Chunk 0 waits for bytes that nothing brings, with a short limit: its CTA waits once more for its
+    loads, reports and returns, the host answers with a timeout, and a fresh handle steps exactly."""
+    from fire_b200.sim import FireXError
+    dims = (36, 32, 20)
+    opts = sphere_options(dims, P=4, R=4)
+
+    def handle():
+        s = FireXSim(dims, opts)
+        s.set_jacobi("fused", 2, 7)
+        s.set_staging(A.STAGING_TMA)
+        return s
+
+    g = handle()
+    g.step(1, DT)
+    g.sync()
+    assert g.diagnostics["jacobi_staging"] == A.STAGING_TMA
+    g.set_wait_limit(16)
+    g.test_hold_face(0, 1)
+    g.step(1, DT)
+    with pytest.raises(FireXError) as e:
+        g.sync()
+    assert e.value.code == A.ERR_TIMEOUT
+    with pytest.raises(FireXError) as e:
+        g.step(1, DT)
+    assert e.value.code == A.ERR_STATE
+    g.close()
+    h, o = handle(), OracleSim(dims, opts)
+    h.step(2, 0.0)
+    o.step(2, 0.0)
+    same(h, o)
+    h.close()
