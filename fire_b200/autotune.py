@@ -5,9 +5,10 @@ real steps on the device.
 Every Jacobi kernel of the library computes each sweep with the same FP32 operations in
 the same order (the GPU tests hold them bit-identical), so the steps taken while tuning are
 ordinary steps of the run: the trajectory is the same whichever candidate ran them. The
-candidates are the resident kernel in each box variant that fits, the single-sweep kernels
-(unblocked, and z-marching with 8, 16 or 32 planes per CTA) and the two-sweep pass with 16-,
-32- or 64-plane chunks, its planes staged by TMA or by cp.async. With the fastest Jacobi
+candidates are the resident kernel as the planner lays it out and in each box variant that fits,
+the single-sweep kernels (unblocked, and z-marching with 8, 16 or 32 planes per CTA) and the
+two-sweep pass with chunks fitted to the device or of 16, 32 or 64 planes, its planes staged by
+TMA or by cp.async: whatever AUTO would run is among them. With the fastest Jacobi
 applied, the source pass's bricks (32 x 4 x 2, 32 x 2 x 4, 32 x 8 x 1 cells), each with the
 primary projection fused with the residual divergence or run as two passes, are timed the same
 way; every choice computes each cell with the same operations. The winner is applied
@@ -42,10 +43,10 @@ class Candidate:
 
 
 def default_candidates() -> list:
-    out = [Candidate("resident", v + 1) for v in (4, 3, 2, 1, 0)]
+    out = [Candidate("resident")] + [Candidate("resident", v + 1) for v in (4, 3, 2, 1, 0)]
     out += [Candidate("unblocked")]
     out += [Candidate("zmarch", 0, zc) for zc in (8, 16, 32)]
-    out += [Candidate("fused", 2, zc, st) for zc in (16, 32, 64) for st in (A.STAGING_CPASYNC, A.STAGING_TMA)]
+    out += [Candidate("fused", 2, zc, st) for zc in (0, 16, 32, 64) for st in (A.STAGING_CPASYNC, A.STAGING_TMA)]
     return out
 
 

@@ -65,6 +65,41 @@ def test_cached_choice_is_applied_without_stepping(tmp_path):
     assert stub.applied == [("fused", 2, 32), ("staging", A.STAGING_CPASYNC), ("tiles", 8, A.PROJECT_SEPARATE)]
 
 
+def test_candidates_cover_what_auto_runs():
+    """AUTO runs the resident kernel in the planner's variant, the two-sweep pass with chunks fitted to
+    the device in either staging, or the unblocked kernel: a tuned workload is no slower than AUTO's."""
+    c = default_candidates()
+    for want in (Candidate("resident"), Candidate("unblocked"), Candidate("fused", 2, 0, A.STAGING_CPASYNC),
+                 Candidate("fused", 2, 0, A.STAGING_TMA)):
+        assert want in c
+    assert len(c) == len(set(c))
+
+
+@pytest.mark.gpu
+def test_auto_beyond_the_chip_is_timed_by_the_tuner():
+    """What AUTO launches on a grid beyond the chip is one of the timed candidates."""
+    from fire_b200.sim import FireXSim
+
+    dims = (192, 200, 136)
+    opts = sphere_options(dims, P=8, R=8)
+    auto, tuned = FireXSim(dims, opts), FireXSim(dims, opts)
+    auto.step(1, DT)
+    auto.sync()
+    t = JacobiTuner(steps=1, warmup=1)
+    t.tune(tuned, DT)
+    want = auto.diagnostics
+    seen = []
+    for key in t.last_timings:
+        c = Candidate(*json.loads(key))
+        JacobiTuner.apply(tuned, c)
+        tuned.step(1, DT)
+        tuned.sync()
+        seen.append(tuple(tuned.diagnostics[k] for k in ("jacobi_kernel", "jacobi_block", "jacobi_zrun", "jacobi_staging")))
+    assert tuple(want[k] for k in ("jacobi_kernel", "jacobi_block", "jacobi_zrun", "jacobi_staging")) in seen
+    auto.close()
+    tuned.close()
+
+
 @pytest.mark.gpu
 def test_tuning_steps_are_ordinary_steps(tmp_path):
     from fire_b200.sim import FireXSim
