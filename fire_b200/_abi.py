@@ -158,7 +158,8 @@ class Diagnostics(C.Structure):
         ("project_fused", C.c_int32),
         ("project_resident", C.c_int32),
         ("jacobi_zrun", C.c_int32),
-        ("reserved", C.c_int32 * 4),
+        ("jacobi_registers", C.c_int32),
+        ("reserved", C.c_int32 * 3),
     ]
 
 

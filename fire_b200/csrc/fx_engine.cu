@@ -900,7 +900,7 @@ struct firex_batch {
             // (long columns only), faces first (small-box instance first), then the column variant
             for (int v : {kRegVariant, 4, 3, 2, 1, 0}) {
                 const FxResKernel kernel{std::min(v, 4), members[0]->half, v == kRegVariant};
-                if (resForce >= 0 && kernel.variant != resForce) continue;
+                if (resForce >= 0 && v != resForce) continue;  // variant 4 by number: the copy warp
                 if (kernel.half && kernel.variant == 4) continue;  // FP32 rows only
                 const int cap = fx_res_capacity(kernel);
                 if (res_assign(dims, cap, v, &boxes, &resSmem)) {
@@ -2006,6 +2006,7 @@ int firex_get_diagnostics(const firex_sim* s, firex_diagnostics* out) {
     out->simulate_by = p.simBy;
     out->project_fused = p.projDiv ? 1 : 0;
     out->project_resident = p.projRes ? 1 : 0;
+    out->jacobi_registers = p.res && p.resReg ? 1 : 0;
     return FIREX_OK;
 }
 

@@ -356,9 +356,10 @@ int firex_set_graphs(firex_sim* sim, int32_t on);
  * memory (only box faces cross L2 between sweeps); used by AUTO whenever the batch fits
  * on chip, else the single-sweep default runs. With RESIDENT, `block` 1-5 restricts the
  * box plan to variant block - 1 (0 columns, 1 faces first, 2 faces first for small
- * boxes, 3 faces first with interior columns, 4 with FP32 pressure only: the pressure in
- * registers for boxes of short columns, else variant 3 with a copy warp that brings the
- * halo rows in by bulk asynchronous copies); 0 lets the planner choose. */
+ * boxes, 3 faces first with interior columns, 4 with FP32 pressure only: variant 3 with a
+ * copy warp that brings the halo rows in by bulk asynchronous copies); 0 lets the planner
+ * choose, among these and, for boxes of short columns with FP32 pressure, variant 4 with the
+ * pressure in registers (firex_diagnostics.jacobi_registers). */
 #define FIREX_JACOBI_RESIDENT 4
 int firex_set_jacobi(firex_sim* sim, int32_t kernel, int32_t block, int32_t zchunk);
 int firex_batch_set_jacobi(firex_batch* batch, int32_t kernel, int32_t block, int32_t zchunk);
@@ -407,7 +408,8 @@ typedef struct firex_diagnostics {
     int32_t project_fused;    /* 1: the primary projection and the residual divergence ran as one pass */
     int32_t project_resident; /* 1: the residual projection ran inside the resident Jacobi's launch */
     int32_t jacobi_zrun;      /* z planes per CTA the two-sweep launches took (AUTO fits them to the device) */
-    int32_t reserved[4];
+    int32_t jacobi_registers; /* 1: the resident Jacobi held the pressure in registers (variant 4) */
+    int32_t reserved[3];
 } firex_diagnostics;
 int firex_get_diagnostics(const firex_sim* sim, firex_diagnostics* out);
 
