@@ -15,6 +15,7 @@
 #include <cuda_fp16.h>
 
 #include "../../include/firex.h"
+#include "fx_plan.h"
 
 // Constant divisors of simulate. Each slot holds d > 0, rcp = RN(1/d) and the range
 // [lo, hi] of |x| where Markstein's correction step (fx_div_checked) reproduces IEEE
@@ -202,13 +203,6 @@ enum FxShape {
     FX_NSHAPES = 7
 };
 
-// Box decomposition of one simulation for the resident Jacobi: boxes of by x bz rows of
-// full x rows, nby x nbz of them (CTA b owns box (b % nby, b / nby)).
-struct FxResBox {
-    int by, bz, nby, nbz;
-    int exOff;  // variant 4: the member's first packet (16 bytes) in the batch's exchange buffer
-    int pad[3];
-};
 // CELL: 32 x BY x (8 / BY) cells, one thread per cell (simulate); BY = FX_CELL_BY unless
 //       the plan tunes it (firex_set_tiles).
 // ROW4: 256 groups of 4 consecutive x cells in memory order (stencils).

@@ -131,7 +131,7 @@ struct StepPlan {
     bool half = false;
     int maxP = 0, maxR = 0;
     int k = 1, zc = 16;       // fused sweeps per Jacobi launch, z planes per CTA asked for
-    int zrun = 16;            // ... and those the launches take (zs_run)
+    int zrun = 16;            // ... and those the launches take (fx_zs_run)
     int zmZc = 16;            // z planes per CTA of the single-sweep (z-marching) kernel
     bool row4 = false;        // single sweeps by the unblocked kernel instead
     bool fuseP = false, fuseR = false;
@@ -216,167 +216,6 @@ void enqueue_step_launches(cudaStream_t st, const StepPlan& pl, FxBatchDev* B) {
     if (!pl.projRes) fx_launch_project(st, pl.half, B, pl.bricks[FX_SHAPE_ROW4], 1);
     fx_launch_step_end(st, B);
     if (pl.pack) fx_launch_pack_batch(st, B, pl.bricks[FX_SHAPE_ROW4]);
-}
-
-// Jacobi kernel when the caller did not choose one (measured on B200, 96+96 sweeps): below 2 Mi
-// cells per batch the unblocked kernel; from there two sweeps per pass by z-marching strips
-// (160x240x160: 2.14 ms of Jacobi per step against 3.95 unblocked; 508^3: 31.6 against 56.5
-// for one sweep per pass), in chunks of 16 planes, or 64 from 16 Mi cells, stretched or shortened
-// to fill the device's waves (zs_run). fire_b200/autotune.py refines this per workload.
-void default_jacobi(long long cells, int* kernel, int* k, int* zc) {
-    const bool fused = cells >= (2LL << 20);
-    *kernel = fused ? FIREX_JACOBI_FUSED : FIREX_JACOBI_UNBLOCKED;
-    *k = fused ? 2 : 1;
-    *zc = cells >= (16LL << 20) ? 64 : 16;
-}
-
-// Box decomposition of an X x Y x Z grid over at most m CTAs for the resident Jacobi
-// (boxes of by x bz full x rows; G = by * bz * X / 4 groups of 4 cells per box). Cost per
-// sweep: the groups a thread computes plus the halo traffic per thread (faces written and
-// halo rows read, 2 (by + bz) rows of X / 4 groups, both ways).
-//   variants 1, 2 (faces-first): face groups and interior groups dealt out separately,
-//     within FX_RES_MAXF and FX_RES_MAXI (variant 2: FX_RES_MAXI_SMALL) per thread;
-//   variant 0 (columns): thread columns of (x group, row), by * X / 4 <= T, each split into
-//     parts along z; at most FX_RES_MAXG planes per column part.
-// False when no box fits one CTA's shared memory and registers.
-//   variant 4 (registers): boxes of strips of four rows, their columns split along z
-//     (fx_reg_geom), at most FX_REG_MAXZ planes to a thread.
-long long reg_smem(int X, int Y, int Z, const FxResBox& bx) {
-    long long most = 0;
-    for (int iz = 0; iz < bx.nbz; ++iz)
-        for (int iy : {0, bx.nby - 1}) {
-            const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, iz * bx.nby + iy);
-            if (g.cols > FX_REG_THREADS || g.len > FX_REG_MAXZ || g.cols * g.parts > FX_REG_THREADS) return -1;
-            if (2 * (g.ny + g.nz) * (X / 4) > FX_REG_MAXH * FX_REG_THREADS) return -1;
-            most = std::max(most, fx_reg_smem_bytes(X, g));
-        }
-    return most;
-}
-bool reg_box(int X, int Y, int Z, int m, FxResBox* out) {
-    bool found = false;
-    double best = 0;
-    for (int by = 2; by <= Y; by += 2) {
-        const int nby = (Y + by - 1) / by;
-        if (nby > m || nby > FX_RES_MAX_CTAS) continue;
-        if ((X / 4) * (by / 2) > FX_REG_THREADS) break;
-        const int nbz = std::min(Z, std::min(m, FX_RES_MAX_CTAS) / nby);
-        FxResBox bx{by, (Z + nbz - 1) / nbz, nby, nbz, 0, {0, 0, 0}};
-        const long long smem = reg_smem(X, Y, Z, bx);
-        if (smem < 0 || smem > FX_RES_SMEM_MAX) continue;
-        const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, (nbz - 1) * nby);
-        // cycles of a sweep, roughly: the warps' issue slots or one warp's chain, and the faces
-        const double warps = (g.cols * g.parts + 31) / 32;
-        const double cost = std::max(warps * g.len * 2 * 25.0, g.len * 2 * 100.0) + 2.0 * (by + bx.bz) * (X / 4) / FX_REG_THREADS * 100.0;
-        if (!found || cost < best) {
-            found = true;
-            best = cost;
-            *out = bx;
-        }
-    }
-    return found;
-}
-constexpr int kRegVariant = 5;  // variant 4 with the pressure in registers
-bool res_box(int X, int Y, int Z, int m, int variant, FxResBox* out) {
-    if (variant == kRegVariant) return reg_box(X, Y, Z, m, out);
-    const long long gx = X / 4;
-    bool found = false;
-    double best = 0;
-    for (int by = 1; by <= Y && by <= 2047; ++by) {
-        const int nby = (Y + by - 1) / by;
-        if (nby > m || nby > FX_RES_MAX_CTAS) continue;
-        const int maxNbz = m / nby;
-        const int bz = (Z + maxNbz - 1) / maxNbz;
-        if (bz > 1023) continue;
-        if (fx_res_smem_bytes(X, by, bz) > FX_RES_SMEM_MAX) continue;
-        const long long G = (long long)by * bz * gx;
-        double work;
-        if (variant == 3 || variant == 4) {
-            // faces dealt out; interior columns (rows off the y faces x groups) one per
-            // thread, split along z when there are fewer columns than threads (variant 4:
-            // the threads but the copy warp)
-            const long long T = variant == 4 ? FX_RES_COPY_TC : FX_RES_THREADS;
-            if (2LL * (by + bz) * gx > (long long)FX_RES_MAXF * T) continue;
-            // the most interior rows and planes a box can have: a box with a neighbour on
-            // one side only keeps all but one row (plane) off its faces
-            const int nbzHere = (Z + bz - 1) / bz;
-            const long long rowsI = nby == 1 ? by : by - 1, planesI = nbzHere == 1 ? bz : bz - 1;
-            const long long Cmax = rowsI * gx;
-            if (Cmax > T) continue;
-            const long long parts = std::max(1LL, T / std::max(1LL, Cmax));
-            const long long zlen = (planesI + parts - 1) / parts;
-            if (zlen > FX_RES_MAXZ) continue;
-            if (zlen < 4) continue;  // short columns: the faces-first variants do better (measured)
-            const long long F = 2LL * (by + bz) * gx;
-            work = (double)zlen + (double)((F + T - 1) / T);
-        } else if (variant != 0) {
-            // faces (at most 2 (by + bz) rows of groups) and interior dealt out separately
-            const int maxi = variant == 2 ? FX_RES_MAXI_SMALL : FX_RES_MAXI;
-            if (2LL * (by + bz) * gx > (long long)FX_RES_MAXF * FX_RES_THREADS) continue;
-            if (G > (long long)maxi * FX_RES_THREADS) continue;
-            work = (double)((G + FX_RES_THREADS - 1) / FX_RES_THREADS);
-        } else {
-            if (by * gx > FX_RES_THREADS) continue;
-            const int parts = (int)(FX_RES_THREADS / (by * gx));
-            const int zlen = (bz + parts - 1) / parts;
-            if (zlen > FX_RES_MAXG) continue;
-            work = zlen;
-        }
-        const double cost = work + 4.0 * (by + bz) * gx / FX_RES_THREADS;
-        if (!found || cost < best) {
-            found = true;
-            best = cost;
-            *out = FxResBox{by, bz, nby, (Z + bz - 1) / bz, 0, {0, 0, 0}};
-        }
-    }
-    return found;
-}
-
-// CTAs for every simulation of a batch within `cap` (one launch of one variant): each gets
-// at least the fewest CTAs its grid fits in, the rest in proportion to cells. False when
-// the batch does not fit.
-bool res_assign(const std::vector<std::array<int, 3>>& dims, int cap, int variant, std::vector<FxResBox>* boxes,
-                int* smem) {
-    const size_t n = dims.size();
-    if (n == 0 || cap <= 0) return false;
-    std::vector<int> mins(n), t(n);
-    long long sumMin = 0;
-    double cells = 0;
-    FxResBox tmp;
-    for (size_t i = 0; i < n; ++i) {
-        const auto& d = dims[i];
-        if (!res_box(d[0], d[1], d[2], cap, variant, &tmp)) return false;
-        int lo = 1, hi = cap;
-        while (lo < hi) {
-            const int mid = (lo + hi) / 2;
-            if (res_box(d[0], d[1], d[2], mid, variant, &tmp)) hi = mid;
-            else lo = mid + 1;
-        }
-        mins[i] = lo;
-        sumMin += lo;
-        cells += (double)d[0] * d[1] * d[2];
-    }
-    if (sumMin > cap) return false;
-    long long sum = 0;
-    for (size_t i = 0; i < n; ++i) {
-        const double share = (double)dims[i][0] * dims[i][1] * dims[i][2] / cells;
-        t[i] = std::max(mins[i], (int)std::floor(share * cap));
-        sum += t[i];
-    }
-    while (sum > cap) {  // give back CTAs from the member with the most to spare
-        size_t j = 0;
-        for (size_t i = 1; i < n; ++i)
-            if (t[i] - mins[i] > t[j] - mins[j]) j = i;
-        --t[j];
-        --sum;
-    }
-    boxes->resize(n);
-    *smem = 0;
-    for (size_t i = 0; i < n; ++i) {
-        res_box(dims[i][0], dims[i][1], dims[i][2], t[i], variant, &(*boxes)[i]);
-        *smem = std::max(*smem, (int)(variant == kRegVariant ? reg_smem(dims[i][0], dims[i][1], dims[i][2], (*boxes)[i])
-                                                   : fx_res_smem_bytes(dims[i][0], (*boxes)[i].by, (*boxes)[i].bz)));
-    }
-    return true;
 }
 
 // z chunk of the z-marching kernel when not chosen: the largest of 32, 16, 8 planes that
@@ -893,17 +732,16 @@ struct firex_batch {
         resOk = false;
         h->ex = nullptr;
         if (wantRes && !members.empty()) {
-            std::vector<std::array<int, 3>> dims;
-            for (firex_sim* s : members) dims.push_back({s->X, s->Y, s->Z});
+            const std::vector<std::array<int, 3>> dims = this->dims();
             // the first variant every member fits: pressure in registers (FP32, short columns), faces
             // first with interior columns and a copy warp (FP32), the same without the copy warp
             // (long columns only), faces first (small-box instance first), then the column variant
-            for (int v : {kRegVariant, 4, 3, 2, 1, 0}) {
-                const FxResKernel kernel{std::min(v, 4), members[0]->half, v == kRegVariant};
+            for (int v : {FX_RES_REGISTERS, 4, 3, 2, 1, 0}) {
+                const FxResKernel kernel{std::min(v, 4), members[0]->half, v == FX_RES_REGISTERS};
                 if (resForce >= 0 && v != resForce) continue;  // variant 4 by number: the copy warp
                 if (kernel.half && kernel.variant == 4) continue;  // FP32 rows only
                 const int cap = fx_res_capacity(kernel);
-                if (res_assign(dims, cap, v, &boxes, &resSmem)) {
+                if (fx_res_assign(dims, cap, v, &boxes, &resSmem)) {
                     if (kernel.reg && !ensure_exchange(dims, boxes)) continue;
                     resOk = true;
                     resKernel = kernel;
@@ -946,34 +784,10 @@ struct firex_batch {
         tableDirty = true;
     }
 
-    // z planes per CTA of the two-sweep pass when the caller did not ask for a number: the chunk
-    // length that takes the fewest plane steps, counting a chunk's own planes, the one beside it
-    // at each end and the time its first planes take to arrive (about two steps more), over the
-    // waves of CTAs its bricks make on the device.
-    static int zs_run(const std::vector<firex_sim*>& members, int k) {
-        if (k != 2) return 16;
-        const int slots = fx_zs_capacity(members[0]->half);
-        int best = 16, maxZ = 0;
-        double least = 0;
-        for (firex_sim* s : members) maxZ = std::max(maxZ, s->Z);
-        if (members[0]->half) maxZ = std::min(maxZ, 64);  // FP16 rows: 412x616x412 17.0 ms at 52 planes, 18.0 at 206
-        for (int zc = std::min(4, maxZ); zc <= maxZ; ++zc) {
-            long long bricks = 0, steps = 0;
-            for (firex_sim* s : members) {
-                const long long n = fx_zs_bricks(s->X, s->Y, s->Z, zc, FX_ZS_TXG);
-                const int chunks = (s->Z + zc - 1) / zc;
-                bricks += n;
-                steps += n / chunks * (s->Z + 4LL * chunks);
-            }
-            const double waves = (double)((bricks + slots - 1) / slots);
-            // uneven members fill a wave's end with short chunks: never below the mean load
-            const double cost = std::max(std::min(waves * (zc + 4.0), steps / (double)slots + zc + 4.0), steps / (double)slots);
-            if (least == 0 || cost < least * 0.999) {
-                least = cost;
-                best = zc;
-            }
-        }
-        return best;
+    std::vector<std::array<int, 3>> dims() const {
+        std::vector<std::array<int, 3>> v;
+        for (const firex_sim* s : members) v.push_back({s->X, s->Y, s->Z});
+        return v;
     }
 
     std::vector<char> water_signature() const {
@@ -1008,7 +822,7 @@ struct firex_batch {
         const bool autoKernel = wantRes, zcOwn = zc > 0;
         if (autoKernel) {
             int dk = 1, dzc = 32;
-            default_jacobi(cells, &kernel, &dk, &dzc);
+            fx_default_jacobi(cells, &kernel, &dk, &dzc);
             k = dk;
             if (zc <= 0) zc = dzc;
         }
@@ -1020,7 +834,7 @@ struct firex_batch {
         }
         p.k = k;
         p.zc = zc > 0 ? zc : 16;
-        p.zrun = zcOwn ? p.zc : zs_run(members, k);
+        p.zrun = zcOwn ? p.zc : (k == 2 ? fx_zs_run(dims(), p.half, fx_zs_capacity(p.half)) : 16);
         p.fuseP = k == 2 && uniformP && fused_pairs(p.maxP) > 0;
         p.fuseR = k == 2 && uniformR && fused_pairs(p.maxR) > 0;
         if (!p.fuseP && !p.fuseR) p.k = 1;

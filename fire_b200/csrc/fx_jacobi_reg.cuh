@@ -34,39 +34,6 @@
 #include "fx_step_math.cuh"
 #include "fx_storage.cuh"
 
-#define FX_REG_THREADS 384
-#define FX_REG_MAXZ 4  // planes of a thread's column part
-#define FX_REG_MAXH 4  // halo quads a thread receives per sweep
-
-// Geometry of box b of a plan: rows y0 .. y0 + ny - 1 (strips of two), planes z0 .. z0 + nz - 1 dealt
-// evenly over the nbz boxes, each column of strips split into `parts` runs of `len` planes, which
-// overlap where nz is not a multiple of len.
-struct FxRegGeom {
-    int y0, ny, z0, nz, ns, cols, parts, len;
-};
-__host__ __device__ inline FxRegGeom fx_reg_geom(int X, int Y, int Z, const FxResBox& bx, int b) {
-    FxRegGeom g;
-    const int iy = b % bx.nby, iz = b / bx.nby;
-    g.y0 = iy * bx.by;
-    g.ny = Y - g.y0 < bx.by ? Y - g.y0 : bx.by;
-    g.z0 = (int)((long long)iz * Z / bx.nbz);
-    g.nz = (int)((long long)(iz + 1) * Z / bx.nbz) - g.z0;
-    g.ns = g.ny / 2;
-    g.cols = (X / 4) * g.ns;
-    const int most = FX_REG_THREADS / (g.cols > 0 ? g.cols : 1);
-    g.len = most > 0 ? (g.nz + most - 1) / most : g.nz;
-    g.parts = (g.nz + g.len - 1) / g.len;
-    return g;
-}
-// Shared memory: the box's pressure with a halo row or plane on each side, and each thread's
-// divergence.
-__host__ __device__ inline int fx_reg_pressure_floats(int X, const FxRegGeom& g) { return (g.nz + 2) * (g.ny + 2) * X; }
-__host__ __device__ inline long long fx_reg_smem_bytes(int X, const FxRegGeom& g) {
-    return 4LL * fx_reg_pressure_floats(X, g) + 32LL * g.len * FX_REG_THREADS;
-}
-// Quads a box sends per sweep: sections y low, y high (bz rows), z low, z high (by rows).
-__host__ __device__ inline int fx_reg_outbox_quads(int X, const FxResBox& bx) { return 2 * (bx.by + bx.bz) * (X / 4); }
-
 // Faces travel as packets of {value, tag} in 64-bit words, stored and loaded relaxed: a word is
 // one access, so a receiver that sees the sweep's tag has the sweep's value, and needs no flag,
 // fence or second round trip.

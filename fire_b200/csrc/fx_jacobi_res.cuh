@@ -31,19 +31,11 @@
 #pragma once
 
 #include "fx_async.cuh"
+#include "fx_plan.h"
 #include "fx_step_math.cuh"
 #include "fx_storage.cuh"
 
-#define FX_RES_THREADS 512
-#define FX_RES_COPY_TC (FX_RES_THREADS - 32)  // compute threads of variant 4 (the last warp copies)
-#define FX_RES_MAXG 12                // groups of 4 cells per thread, column variant
-#define FX_RES_MAXF 4                 // face groups per thread, faces-first variant
-#define FX_RES_MAXI 11                // interior groups per thread, faces-first variant
-#define FX_RES_MAXI_SMALL 7           // ... its instance for small boxes (fewer registers)
-#define FX_RES_MAXZ 10                // interior planes per thread column, faces-first column variant
-#define FX_RES_SMEM_MAX (226 * 1024)  // dynamic shared memory per CTA (227 KB opt-in less static)
 #define FX_RES_SPIN_LIMIT (1u << 24)  // polls of a neighbour's flag (well over a second with back-off)
-#define FX_RES_MAX_CTAS 1024          // boxes per simulation and phase (flag slots)
 #define FX_RES_FLAGS 16               // offset of the flag slots in FxSimDev::sync
 #define FX_RES_SYNC_WORDS (FX_RES_FLAGS + 2 * FX_RES_MAX_CTAS)
 // Words of FxSimDev::sync after the error word [2], set from the host (firex_set_wait_limit,
@@ -55,11 +47,6 @@
 #define FX_SYNC_SPIN 3
 #define FX_SYNC_HOLD_BOX 4
 #define FX_SYNC_HOLD_SWEEP 5
-
-// Shared-memory bytes of a box: pressure with halo rows + divergence.
-__host__ __device__ inline long long fx_res_smem_bytes(int X, int by, int bz) {
-    return ((long long)(by + 2) * (bz + 2) + (long long)by * bz) * X * 4;
-}
 
 FXD unsigned fx_ld_acquire_u32(const unsigned* p) {
     unsigned v;

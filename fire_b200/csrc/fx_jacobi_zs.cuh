@@ -39,12 +39,9 @@
 #include "fx_step_math.cuh"
 #include "fx_storage.cuh"
 
-#define FX_ZS_THREADS 64
 #define FX_ZS_MINB 8  // CTAs per SM the registers are budgeted for
 #define FX_ZS_SLOTS 3
 #define FX_ZS_WAIT_LIMIT (1u << 22)  // polls of a step's copies
-#define FX_ZS_ROWS 2                 // rows of a thread's strip
-#define FX_ZS_TXG 8   // 4-cell groups of a tile row
 
 template <int TXG>
 struct FxZsShape {
@@ -71,11 +68,6 @@ template <int I>
 struct FxZsInt {
     static constexpr int value = I;
 };
-
-__host__ __device__ inline int fx_zs_bricks(int X, int Y, int Z, int zc, int txg) {
-    const int tx = 4 * txg, ty = FX_ZS_ROWS * (FX_ZS_THREADS / txg) - 2;
-    return ((X + tx - 1) / tx) * ((Y + ty - 1) / ty) * ((Z + zc - 1) / zc);
-}
 
 // Tensor maps of a simulation (FxSimDev::tmap): pressure pair, correction pair, divergence.
 enum { FX_TM_P0 = 0, FX_TM_P1 = 1, FX_TM_C0 = 2, FX_TM_C1 = 3, FX_TM_DIV = 4, FX_TM_COUNT = 5 };

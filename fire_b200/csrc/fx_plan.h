@@ -2,11 +2,23 @@
 // and compiled by the host compiler alone in the CPU tests.
 #pragma once
 
+#include <algorithm>
+#include <array>
+#include <cmath>
+#include <vector>
+
+#include "../../include/firex.h"
+
 #ifdef __CUDACC__
 #define FX_HOST_DEVICE __host__ __device__ inline
 #else
 #define FX_HOST_DEVICE inline
 #endif
+
+// ---- the two-sweep pass by strips (fx_jacobi_zs.cuh) ---------------------------------------------
+#define FX_ZS_THREADS 64
+#define FX_ZS_ROWS 2  // rows of a thread's strip
+#define FX_ZS_TXG 8   // 4-cell groups of a tile row
 
 // Index of a plane or row outside 0 .. n - 1 reflected into it (-1 is 0, n is n - 1), for an index
 // less than n outside.
@@ -16,3 +28,255 @@ FX_HOST_DEVICE int fx_zs_reflect(int q, int n) { return q < 0 ? -1 - q : (q >= n
 // floor are reflected, rows above the open top (q >= Y, whose values reach no stored cell) are
 // the top row. q is -2 or more; a tile of few rows reaches far above the top of a flat grid.
 FX_HOST_DEVICE int fx_zs_input_row(int q, int Y) { return q < 0 ? -1 - q : (q < Y ? q : Y - 1); }
+
+FX_HOST_DEVICE int fx_zs_bricks(int X, int Y, int Z, int zc, int txg) {
+    const int tx = 4 * txg, ty = FX_ZS_ROWS * (FX_ZS_THREADS / txg) - 2;
+    return ((X + tx - 1) / tx) * ((Y + ty - 1) / ty) * ((Z + zc - 1) / zc);
+}
+
+// ---- the resident Jacobi (fx_jacobi_res.cuh, fx_jacobi_reg.cuh) -----------------------------------
+#define FX_RES_THREADS 512
+#define FX_RES_COPY_TC (FX_RES_THREADS - 32)  // compute threads of variant 4 (the last warp copies)
+#define FX_RES_MAXG 12                // groups of 4 cells per thread, column variant
+#define FX_RES_MAXF 4                 // face groups per thread, faces-first variant
+#define FX_RES_MAXI 11                // interior groups per thread, faces-first variant
+#define FX_RES_MAXI_SMALL 7           // ... its instance for small boxes (fewer registers)
+#define FX_RES_MAXZ 10                // interior planes per thread column, faces-first column variant
+#define FX_RES_SMEM_MAX (226 * 1024)  // dynamic shared memory per CTA (227 KB opt-in less static)
+#define FX_RES_MAX_CTAS 1024          // boxes per simulation and phase (flag slots)
+
+#define FX_REG_THREADS 384
+#define FX_REG_MAXZ 4  // planes of a thread's column part
+#define FX_REG_MAXH 4  // halo quads a thread receives per sweep
+
+// Box decomposition of one simulation for the resident Jacobi: boxes of by x bz rows of
+// full x rows, nby x nbz of them (CTA b owns box (b % nby, b / nby)).
+struct FxResBox {
+    int by, bz, nby, nbz;
+    int exOff;  // variant 4: the member's first packet (16 bytes) in the batch's exchange buffer
+    int pad[3];
+};
+
+// Shared-memory bytes of a box: pressure with halo rows + divergence.
+FX_HOST_DEVICE long long fx_res_smem_bytes(int X, int by, int bz) {
+    return ((long long)(by + 2) * (bz + 2) + (long long)by * bz) * X * 4;
+}
+
+// Geometry of box b of a plan: rows y0 .. y0 + ny - 1 (strips of two), planes z0 .. z0 + nz - 1 dealt
+// evenly over the nbz boxes, each column of strips split into `parts` runs of `len` planes, which
+// overlap where nz is not a multiple of len.
+struct FxRegGeom {
+    int y0, ny, z0, nz, ns, cols, parts, len;
+};
+FX_HOST_DEVICE FxRegGeom fx_reg_geom(int X, int Y, int Z, const FxResBox& bx, int b) {
+    FxRegGeom g;
+    const int iy = b % bx.nby, iz = b / bx.nby;
+    g.y0 = iy * bx.by;
+    g.ny = Y - g.y0 < bx.by ? Y - g.y0 : bx.by;
+    g.z0 = (int)((long long)iz * Z / bx.nbz);
+    g.nz = (int)((long long)(iz + 1) * Z / bx.nbz) - g.z0;
+    g.ns = g.ny / 2;
+    g.cols = (X / 4) * g.ns;
+    const int most = FX_REG_THREADS / (g.cols > 0 ? g.cols : 1);
+    g.len = most > 0 ? (g.nz + most - 1) / most : g.nz;
+    g.parts = (g.nz + g.len - 1) / g.len;
+    return g;
+}
+// Shared memory: the box's pressure with a halo row or plane on each side, and each thread's
+// divergence.
+FX_HOST_DEVICE int fx_reg_pressure_floats(int X, const FxRegGeom& g) { return (g.nz + 2) * (g.ny + 2) * X; }
+FX_HOST_DEVICE long long fx_reg_smem_bytes(int X, const FxRegGeom& g) {
+    return 4LL * fx_reg_pressure_floats(X, g) + 32LL * g.len * FX_REG_THREADS;
+}
+// Quads a box sends per sweep: sections y low, y high (bz rows), z low, z high (by rows).
+FX_HOST_DEVICE int fx_reg_outbox_quads(int X, const FxResBox& bx) { return 2 * (bx.by + bx.bz) * (X / 4); }
+
+// ---- plans (host) ---------------------------------------------------------------------------------
+// Jacobi kernel when the caller did not choose one (measured on B200, 96+96 sweeps): below 2 Mi
+// cells per batch the unblocked kernel; from there two sweeps per pass by z-marching strips
+// (160x240x160: 2.14 ms of Jacobi per step against 3.95 unblocked; 508^3: 31.6 against 56.5
+// for one sweep per pass), in chunks of 16 planes, or 64 from 16 Mi cells, stretched or shortened
+// to fill the device's waves (fx_zs_run). fire_b200/autotune.py refines this per workload.
+inline void fx_default_jacobi(long long cells, int* kernel, int* k, int* zc) {
+    const bool fused = cells >= (2LL << 20);
+    *kernel = fused ? FIREX_JACOBI_FUSED : FIREX_JACOBI_UNBLOCKED;
+    *k = fused ? 2 : 1;
+    *zc = cells >= (16LL << 20) ? 64 : 16;
+}
+
+// z planes per CTA of the two-sweep pass when the caller did not ask for a number: the chunk
+// length that takes the fewest plane steps, counting a chunk's own planes, the one beside it
+// at each end and the time its first planes take to arrive (about two steps more), over the
+// waves that its bricks make of the `slots` CTAs the device holds at once.
+inline int fx_zs_run(const std::vector<std::array<int, 3>>& dims, bool half, int slots) {
+    int best = 16, maxZ = 0;
+    double least = 0;
+    for (const auto& d : dims) maxZ = std::max(maxZ, d[2]);
+    if (half) maxZ = std::min(maxZ, 64);  // FP16 rows: 412x616x412 17.0 ms at 52 planes, 18.0 at 206
+    for (int zc = std::min(4, maxZ); zc <= maxZ; ++zc) {
+        long long bricks = 0, steps = 0;
+        for (const auto& d : dims) {
+            const long long n = fx_zs_bricks(d[0], d[1], d[2], zc, FX_ZS_TXG);
+            const int chunks = (d[2] + zc - 1) / zc;
+            bricks += n;
+            steps += n / chunks * (d[2] + 4LL * chunks);
+        }
+        const double waves = (double)((bricks + slots - 1) / slots);
+        // uneven members fill a wave's end with short chunks: never below the mean load
+        const double cost = std::max(std::min(waves * (zc + 4.0), steps / (double)slots + zc + 4.0), steps / (double)slots);
+        if (least == 0 || cost < least * 0.999) {
+            least = cost;
+            best = zc;
+        }
+    }
+    return best;
+}
+
+// Box decomposition of an X x Y x Z grid over at most m CTAs for the resident Jacobi
+// (boxes of by x bz full x rows; G = by * bz * X / 4 groups of 4 cells per box). Cost per
+// sweep: the groups a thread computes plus the halo traffic per thread (faces written and
+// halo rows read, 2 (by + bz) rows of X / 4 groups, both ways).
+//   variants 1, 2 (faces-first): face groups and interior groups dealt out separately,
+//     within FX_RES_MAXF and FX_RES_MAXI (variant 2: FX_RES_MAXI_SMALL) per thread;
+//   variant 0 (columns): thread columns of (x group, row), by * X / 4 <= T, each split into
+//     parts along z; at most FX_RES_MAXG planes per column part.
+// False when no box fits one CTA's shared memory and registers.
+//   variant 4 (registers): boxes of strips of four rows, their columns split along z
+//     (fx_reg_geom), at most FX_REG_MAXZ planes to a thread.
+inline long long fx_reg_smem(int X, int Y, int Z, const FxResBox& bx) {
+    long long most = 0;
+    for (int iz = 0; iz < bx.nbz; ++iz)
+        for (int iy : {0, bx.nby - 1}) {
+            const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, iz * bx.nby + iy);
+            if (g.cols > FX_REG_THREADS || g.len > FX_REG_MAXZ || g.cols * g.parts > FX_REG_THREADS) return -1;
+            if (2 * (g.ny + g.nz) * (X / 4) > FX_REG_MAXH * FX_REG_THREADS) return -1;
+            most = std::max(most, fx_reg_smem_bytes(X, g));
+        }
+    return most;
+}
+inline bool fx_reg_box(int X, int Y, int Z, int m, FxResBox* out) {
+    bool found = false;
+    double best = 0;
+    for (int by = 2; by <= Y; by += 2) {
+        const int nby = (Y + by - 1) / by;
+        if (nby > m || nby > FX_RES_MAX_CTAS) continue;
+        if ((X / 4) * (by / 2) > FX_REG_THREADS) break;
+        const int nbz = std::min(Z, std::min(m, FX_RES_MAX_CTAS) / nby);
+        FxResBox bx{by, (Z + nbz - 1) / nbz, nby, nbz, 0, {0, 0, 0}};
+        const long long smem = fx_reg_smem(X, Y, Z, bx);
+        if (smem < 0 || smem > FX_RES_SMEM_MAX) continue;
+        const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, (nbz - 1) * nby);
+        // cycles of a sweep, roughly: the warps' issue slots or one warp's chain, and the faces
+        const double warps = (g.cols * g.parts + 31) / 32;
+        const double cost = std::max(warps * g.len * 2 * 25.0, g.len * 2 * 100.0) + 2.0 * (by + bx.bz) * (X / 4) / FX_REG_THREADS * 100.0;
+        if (!found || cost < best) {
+            found = true;
+            best = cost;
+            *out = bx;
+        }
+    }
+    return found;
+}
+constexpr int FX_RES_REGISTERS = 5;  // variant 4 with the pressure in registers
+inline bool fx_res_box(int X, int Y, int Z, int m, int variant, FxResBox* out) {
+    if (variant == FX_RES_REGISTERS) return fx_reg_box(X, Y, Z, m, out);
+    const long long gx = X / 4;
+    bool found = false;
+    double best = 0;
+    for (int by = 1; by <= Y && by <= 2047; ++by) {
+        const int nby = (Y + by - 1) / by;
+        if (nby > m || nby > FX_RES_MAX_CTAS) continue;
+        const int maxNbz = m / nby;
+        const int bz = (Z + maxNbz - 1) / maxNbz;
+        if (bz > 1023) continue;
+        if (fx_res_smem_bytes(X, by, bz) > FX_RES_SMEM_MAX) continue;
+        const long long G = (long long)by * bz * gx;
+        double work;
+        if (variant == 3 || variant == 4) {
+            // faces dealt out; interior columns (rows off the y faces x groups) one per
+            // thread, split along z when there are fewer columns than threads (variant 4:
+            // the threads but the copy warp)
+            const long long T = variant == 4 ? FX_RES_COPY_TC : FX_RES_THREADS;
+            if (2LL * (by + bz) * gx > (long long)FX_RES_MAXF * T) continue;
+            // the most interior rows and planes a box can have: a box with a neighbour on
+            // one side only keeps all but one row (plane) off its faces
+            const int nbzHere = (Z + bz - 1) / bz;
+            const long long rowsI = nby == 1 ? by : by - 1, planesI = nbzHere == 1 ? bz : bz - 1;
+            const long long Cmax = rowsI * gx;
+            if (Cmax > T) continue;
+            const long long parts = std::max(1LL, T / std::max(1LL, Cmax));
+            const long long zlen = (planesI + parts - 1) / parts;
+            if (zlen > FX_RES_MAXZ) continue;
+            if (zlen < 4) continue;  // short columns: the faces-first variants do better (measured)
+            const long long F = 2LL * (by + bz) * gx;
+            work = (double)zlen + (double)((F + T - 1) / T);
+        } else if (variant != 0) {
+            // faces (at most 2 (by + bz) rows of groups) and interior dealt out separately
+            const int maxi = variant == 2 ? FX_RES_MAXI_SMALL : FX_RES_MAXI;
+            if (2LL * (by + bz) * gx > (long long)FX_RES_MAXF * FX_RES_THREADS) continue;
+            if (G > (long long)maxi * FX_RES_THREADS) continue;
+            work = (double)((G + FX_RES_THREADS - 1) / FX_RES_THREADS);
+        } else {
+            if (by * gx > FX_RES_THREADS) continue;
+            const int parts = (int)(FX_RES_THREADS / (by * gx));
+            const int zlen = (bz + parts - 1) / parts;
+            if (zlen > FX_RES_MAXG) continue;
+            work = zlen;
+        }
+        const double cost = work + 4.0 * (by + bz) * gx / FX_RES_THREADS;
+        if (!found || cost < best) {
+            found = true;
+            best = cost;
+            *out = FxResBox{by, bz, nby, (Z + bz - 1) / bz, 0, {0, 0, 0}};
+        }
+    }
+    return found;
+}
+
+// CTAs for every simulation of a batch within `cap` (one launch of one variant): each gets
+// at least the fewest CTAs its grid fits in, the rest in proportion to cells. False when
+// the batch does not fit.
+inline bool fx_res_assign(const std::vector<std::array<int, 3>>& dims, int cap, int variant, std::vector<FxResBox>* boxes,
+                          int* smem) {
+    const size_t n = dims.size();
+    if (n == 0 || cap <= 0) return false;
+    std::vector<int> mins(n), t(n);
+    long long sumMin = 0;
+    double cells = 0;
+    FxResBox tmp;
+    for (size_t i = 0; i < n; ++i) {
+        const auto& d = dims[i];
+        if (!fx_res_box(d[0], d[1], d[2], cap, variant, &tmp)) return false;
+        int lo = 1, hi = cap;
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (fx_res_box(d[0], d[1], d[2], mid, variant, &tmp)) hi = mid;
+            else lo = mid + 1;
+        }
+        mins[i] = lo;
+        sumMin += lo;
+        cells += (double)d[0] * d[1] * d[2];
+    }
+    if (sumMin > cap) return false;
+    long long sum = 0;
+    for (size_t i = 0; i < n; ++i) {
+        const double share = (double)dims[i][0] * dims[i][1] * dims[i][2] / cells;
+        t[i] = std::max(mins[i], (int)std::floor(share * cap));
+        sum += t[i];
+    }
+    while (sum > cap) {  // give back CTAs from the member with the most to spare
+        size_t j = 0;
+        for (size_t i = 1; i < n; ++i)
+            if (t[i] - mins[i] > t[j] - mins[j]) j = i;
+        --t[j];
+        --sum;
+    }
+    boxes->resize(n);
+    *smem = 0;
+    for (size_t i = 0; i < n; ++i) {
+        fx_res_box(dims[i][0], dims[i][1], dims[i][2], t[i], variant, &(*boxes)[i]);
+        *smem = std::max(*smem, (int)(variant == FX_RES_REGISTERS ? fx_reg_smem(dims[i][0], dims[i][1], dims[i][2], (*boxes)[i])
+                                                        : fx_res_smem_bytes(dims[i][0], (*boxes)[i].by, (*boxes)[i].bz)));
+    }
+    return true;
+}
