@@ -822,7 +822,7 @@ struct firex_batch {
         const bool autoKernel = wantRes, zcOwn = zc > 0;
         if (autoKernel) {
             int dk = 1, dzc = 32;
-            fx_default_jacobi(cells, &kernel, &dk, &dzc);
+            fx_default_jacobi(cells, fx_zs_fill(dims()), p.half, &kernel, &dk, &dzc);
             k = dk;
             if (zc <= 0) zc = dzc;
         }

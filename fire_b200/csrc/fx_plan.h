@@ -92,13 +92,29 @@ FX_HOST_DEVICE long long fx_reg_smem_bytes(int X, const FxRegGeom& g) {
 FX_HOST_DEVICE int fx_reg_outbox_quads(int X, const FxResBox& bx) { return 2 * (bx.by + bx.bz) * (X / 4); }
 
 // ---- plans (host) ---------------------------------------------------------------------------------
+// Cells of these grids over the cells of the strip tiles that cover them: 1 where 32 x 14 tiles fit.
+inline double fx_zs_fill(const std::vector<std::array<int, 3>>& dims) {
+    double cells = 0, tiled = 0;
+    for (const auto& d : dims) {
+        cells += (double)d[0] * d[1] * d[2];
+        tiled += (double)fx_zs_bricks(d[0], d[1], 1, 1, FX_ZS_TXG) * (4 * FX_ZS_TXG) * (FX_ZS_ROWS * (FX_ZS_THREADS / FX_ZS_TXG) - 2) * d[2];
+    }
+    return tiled > 0 ? cells / tiled : 1.0;
+}
+
 // Jacobi kernel when the caller did not choose one (measured on B200, 96+96 sweeps): below 2 Mi
 // cells per batch the unblocked kernel; from there two sweeps per pass by z-marching strips
 // (160x240x160: 2.14 ms of Jacobi per step against 3.95 unblocked; 508^3: 31.6 against 56.5
 // for one sweep per pass), in chunks of 16 planes, or 64 from 16 Mi cells, stretched or shortened
 // to fill the device's waves (fx_zs_run). fire_b200/autotune.py refines this per workload.
-inline void fx_default_jacobi(long long cells, int* kernel, int* k, int* zc) {
-    const bool fused = cells >= (2LL << 20);
+// Narrow and flat grids leave the tiles empty: below a fill of 0.42 the unblocked kernel is the faster
+// at any size (us per sweep, strips and unblocked: 4x1024x1024, fill 0.12, 37.9 and 14.8;
+// 8x512x1024, 0.25, 21.6 and 15.1; 200 grids of 36x16x36, 0.32, 30.4 and 21.7; 128 of 36x44x28, 0.44,
+// 24.5 and 27.9; 16x512x512, 0.49, 13.3 and 15.1). FP16 pressure gains less from strips while it
+// stays in L2: below 8 Mi cells the line is at 0.56 (60 grids of 36x60x36, 0.48, 23.6 and 21.6;
+// 36x400x300, 0.55, 16.2 and 16.0; 512x8x1024, 0.57, 13.5 and 14.4).
+inline void fx_default_jacobi(long long cells, double fill, bool half, int* kernel, int* k, int* zc) {
+    const bool fused = cells >= (2LL << 20) && fill >= (half && cells < (8LL << 20) ? 0.56 : 0.42);
     *kernel = fused ? FIREX_JACOBI_FUSED : FIREX_JACOBI_UNBLOCKED;
     *k = fused ? 2 : 1;
     *zc = cells >= (16LL << 20) ? 64 : 16;
@@ -140,9 +156,9 @@ inline int fx_zs_run(const std::vector<std::array<int, 3>>& dims, bool half, int
 //     within FX_RES_MAXF and FX_RES_MAXI (variant 2: FX_RES_MAXI_SMALL) per thread;
 //   variant 0 (columns): thread columns of (x group, row), by * X / 4 <= T, each split into
 //     parts along z; at most FX_RES_MAXG planes per column part.
+//   FX_RES_REGISTERS: boxes of strips of two rows, their columns split along z (fx_reg_geom), at
+//     most FX_REG_MAXZ planes to a thread.
 // False when no box fits one CTA's shared memory and registers.
-//   variant 4 (registers): boxes of strips of four rows, their columns split along z
-//     (fx_reg_geom), at most FX_REG_MAXZ planes to a thread.
 inline long long fx_reg_smem(int X, int Y, int Z, const FxResBox& bx) {
     long long most = 0;
     for (int iz = 0; iz < bx.nbz; ++iz)

@@ -346,8 +346,8 @@ int firex_set_graphs(firex_sim* sim, int32_t on);
  *               sweeps leave it in.
  * `zchunk`: z planes per CTA for ZMARCH and FUSED (0 = auto: FUSED fits them to the device,
  * firex_diagnostics.jacobi_zrun). AUTO takes RESIDENT when the batch fits on chip, else by its
- * cell count: UNBLOCKED below 2 Mi cells, FUSED with block 2 and 16-plane chunks below 16 Mi,
- * FUSED with block 2 and 64-plane chunks from 16 Mi. */
+ * cell count: UNBLOCKED below 2 Mi cells and for grids so narrow or flat that 32 x 14 tiles stay
+ * largely empty, else FUSED with block 2. */
 #define FIREX_JACOBI_AUTO 0
 #define FIREX_JACOBI_UNBLOCKED 1
 #define FIREX_JACOBI_ZMARCH 2
