@@ -838,7 +838,10 @@ struct firex_batch {
         p.fuseP = k == 2 && uniformP && fused_pairs(p.maxP) > 0;
         p.fuseR = k == 2 && uniformR && fused_pairs(p.maxR) > 0;
         if (!p.fuseP && !p.fuseR) p.k = 1;
-        p.row4 = kernel == FIREX_JACOBI_UNBLOCKED;
+        // single sweeps of a phase that does not fuse, or is left over: unblocked while AUTO's batch stays
+        // in L2 (us per sweep, unblocked and z-marching: 144x216x136 15.7 and 18.5, 160x240x160 21.0 and
+        // 22.3, with FP16 pressure 22.6 and 34.9, 64 grids of 36x44x28 15.5 and 20.5; 184x272x168 30.4 and 27.3)
+        p.row4 = kernel == FIREX_JACOBI_UNBLOCKED || (autoKernel && cells < (8LL << 20));
         p.zmZc = (kernel == FIREX_JACOBI_ZMARCH && zc > 0) ? zc : zm_chunk(zm32, zm16);
         const int by = this->simBy ? this->simBy : members[0]->simBy;
         p.simBy = by ? by : FX_CELL_BY;

@@ -195,3 +195,29 @@ def test_unfinished_tensor_loads_expire_the_wait():
     o.step(2, 0.0)
     same(h, o)
     h.close()
+
+
+# ---- phases that AUTO does not fuse ----------------------------------------------------------------
+
+def test_auto_runs_unblocked_sweeps_where_no_phase_fuses():
+    """Beyond the chip and within L2: fewer than four sweeps, and members of different sweep counts."""
+    from fire_b200.sim import FireXBatch
+    s = FireXSim((160, 240, 160), sphere_options((160, 240, 160), P=2, R=3))
+    s.step(1, DT)
+    s.sync()
+    assert s.diagnostics["jacobi_kernel"] == A.JACOBI_UNBLOCKED, s.diagnostics
+    s.close()
+    dims = (96, 144, 96)
+    alone = [FireXSim(dims, sphere_options(dims, P=6 + i, R=9 - i, seed=i)) for i in range(4)]
+    members = [FireXSim(dims, sphere_options(dims, P=6 + i, R=9 - i, seed=i)) for i in range(4)]
+    for a in alone:
+        a.set_jacobi("unblocked")
+        a.step(2, DT)
+    with FireXBatch() as b:
+        for m in members:
+            b.add(m)
+        b.step(2, DT)
+        b.sync()
+        assert members[0].diagnostics["jacobi_kernel"] == A.JACOBI_UNBLOCKED, members[0].diagnostics
+    for a, m in zip(alone, members):
+        same(a, m)
