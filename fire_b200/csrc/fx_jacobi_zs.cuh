@@ -105,16 +105,21 @@ FXD bool fx_zs_wait(const FxSimDev& S, unsigned long long* bar, unsigned parity)
     const unsigned own = S.sync[FX_SYNC_SPIN];
     return fx_mbar_wait(bar, parity, own ? own : FX_ZS_WAIT_LIMIT);
 }
+// firex_test_hold_face: whether a test holds this brick. Read while the first planes are on their way (read
+// before they were asked for it cost 0.9 % of a step at 160x240x160).
+FXD bool fx_zs_held(const FxSimDev& S, int brick, int launch) {
+    return S.sync[FX_SYNC_HOLD_BOX] == (unsigned)brick + 1u && (unsigned)launch >= S.sync[FX_SYNC_HOLD_SWEEP];
+}
 // Planes and rows outside the grid are reflected into it (fx_zs_reflect, fx_zs_input_row). The update
 // adds the two neighbours of an axis, so the sweep-1 value of a reflected plane or row is that of its
 // image, which is what sweep 2's clamped neighbour is: the walls need no code of their own.
 
 // Two sweeps of planes [z0, z1) of the tile at (x0, y0): pin -> pout. TOP: the tile holds rows at
-// or above the open top. held (a test's, firex_test_hold_face): the first planes are waited for with
-// bytes that nothing brings. False when a bounded wait ran out.
+// or above the open top; brick and launch: its place for a test that holds it (fx_zs_held). False when
+// a bounded wait ran out.
 template <typename PT, int TXG, bool ZERO_IN, bool ROUND, bool TWO, bool TOP, bool TMA>
 FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restrict__ pout, int x0, int y0, int z0, int z1,
-                    FxZsSmem<PT, TXG>& sm, const CUtensorMap* mapP, const CUtensorMap* mapD, unsigned& parity, bool held) {
+                    FxZsSmem<PT, TXG>& sm, const CUtensorMap* mapP, const CUtensorMap* mapD, unsigned& parity, int brick, int launch) {
     using H = FxZsShape<TXG>;
     constexpr int COLS = H::COLS;
     const int X = S.X, Y = S.Y, Z = S.Z, XY = X * Y, t = threadIdx.x;
@@ -158,9 +163,9 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         for (int k = 0; k < H::KD; ++k)
             if (k < H::KD - 1 || lastD) fx_cp_async16(dst + 4 * k * FX_ZS_THREADS, src + gD[k]);
     };
-    // nP input planes, one divergence plane and `more` bytes complete the next phase of sm.bar
-    auto expect = [&](int nP, unsigned more) {
-        if (TMA && t == 0) fx_mbar_expect_tx(&sm.bar, (ZERO_IN ? 0 : nP) * BP + BD + more);
+    // nP input planes and one divergence plane complete the next phase of sm.bar
+    auto expect = [&](int nP) {
+        if (TMA && t == 0) fx_mbar_expect_tx(&sm.bar, (ZERO_IN ? 0 : nP) * BP + BD);
     };
     // the copies requested last have landed, for every thread; false when a bounded wait ran out
     auto landed = [&](bool requested) {
@@ -252,7 +257,7 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         constexpr int C = decltype(slot)::value, N = (C + 1) % 3, M = (C + 2) % 3;
         if (!landed(z != zs)) return false;  // planes up to z + 1 are here; plane z - 1's input and z - 2's other slots are free
         if (z < z1) {
-            expect(1, 0);
+            expect(1);
             issueP(z + 2, M);
             issueD(z + 1, N);
             if (!TMA) fx_cp_commit();
@@ -300,12 +305,13 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         return true;
     };
     // slots: plane z in slot (z - zs) mod 3, plane zs - 1 in slot 2 until step zs
-    expect(3, held ? 16 : 0);
+    expect(3);
     issueP(zs - 1, 2);
     issueP(zs, 0);
     issueP(zs + 1, 1);
     issueD(zs, 0);
     if (!TMA) fx_cp_commit();
+    else if (t == 0 && fx_zs_held(S, brick, launch)) fx_mbar_expect_more(&sm.bar, 16);  // bytes that nothing brings
     if (!landed(true)) return false;
     FxQuad p0[FX_ZS_ROWS], p1[FX_ZS_ROWS], p2[FX_ZS_ROWS], s0[FX_ZS_ROWS], s1[FX_ZS_ROWS], s2[FX_ZS_ROWS];
 #pragma unroll

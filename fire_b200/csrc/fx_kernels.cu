@@ -561,17 +561,16 @@ __global__ void __launch_bounds__(FX_ZS_THREADS, FX_ZS_MINB) fxk_jacobi_zs(const
         const CUtensorMap* mapP = TMA ? fx_zs_map_of(S, bufs.pin) : nullptr;
         const CUtensorMap* mapD = &S.tmap[FX_TM_DIV];
         const bool top = y0 + H::TY >= S.Y - 1;  // the tile or its ring reaches the open top
-        const bool held = TMA && S.sync[FX_SYNC_HOLD_BOX] == (unsigned)b + 1u && (unsigned)launch >= S.sync[FX_SYNC_HOLD_SWEEP];
         if (TMA && threadIdx.x == 0) {  // the thread that issues the tensor loads
             if (!bufs.zeroIn) fx_zs_map_acquire(mapP);
             fx_zs_map_acquire(mapD);
         }
         if (bufs.zeroIn) {
-            ok = top ? fx_zs_tile<PT, TXG, true, ROUND, TWO, true, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, held)
-                     : fx_zs_tile<PT, TXG, true, ROUND, TWO, false, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, held);
+            ok = top ? fx_zs_tile<PT, TXG, true, ROUND, TWO, true, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, b, launch)
+                     : fx_zs_tile<PT, TXG, true, ROUND, TWO, false, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, b, launch);
         } else {
-            ok = top ? fx_zs_tile<PT, TXG, false, ROUND, TWO, true, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, held)
-                     : fx_zs_tile<PT, TXG, false, ROUND, TWO, false, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, held);
+            ok = top ? fx_zs_tile<PT, TXG, false, ROUND, TWO, true, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, b, launch)
+                     : fx_zs_tile<PT, TXG, false, ROUND, TWO, false, TMA>(S, pin, pout, x0, y0, z0, z1, sm, mapP, mapD, parity, b, launch);
         }
         if (!ok && threadIdx.x == 0) atomicExch(S.sync + 2, 1u);
     });
