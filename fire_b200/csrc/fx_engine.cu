@@ -135,6 +135,7 @@ struct StepPlan {
     int zmZc = 16;            // z planes per CTA of the single-sweep (z-marching) kernel
     bool row4 = false;        // single sweeps by the unblocked kernel instead
     bool fuseP = false, fuseR = false;
+    bool bothR = false;       // the residual solve leaves its last two sweeps in the buffers (fused_pairs)
     bool pack = false;        // a member packs its render volumes at the end of every step
     bool tma = false;         // the two-sweep pass stages its planes by TMA
     bool two = false;         // every member's denominator has a checked two-operation quotient
@@ -149,7 +150,7 @@ struct StepPlan {
     bool simEarly = false;    // the source pass evaluates its neighbour terms before the advection
     int bricks[FX_NSHAPES] = {};
     auto key() const {
-        return std::tie(storage, half, maxP, maxR, k, zc, zrun, zmZc, row4, fuseP, fuseR, pack, tma, two, simBy, projDiv, res,
+        return std::tie(storage, half, maxP, maxR, k, zc, zrun, zmZc, row4, fuseP, fuseR, bothR, pack, tma, two, simBy, projDiv, res,
                         resVariant, resReg, resSmem, projRes, simEarly, simTwo,
                         bricks[0],
                         bricks[1], bricks[2], bricks[3], bricks[4], bricks[5], bricks[6]);
@@ -166,14 +167,18 @@ struct StepPlan {
 
 // Two-sweep launches of a phase of n sweeps: an even number, the rest (up to three) as single
 // sweeps, so the launch count has the parity of n and the result lands in the buffer the
-// reference's ping-pong leaves it in.
-int fused_pairs(int n) { return (n / 2) & ~1; }
+// reference's ping-pong leaves it in. both: the other buffer of the pair is observable and has to
+// hold the sweep before the last, so the phase ends with single sweeps.
+int fused_pairs(int n, bool both = false) { return ((n / 2) & ~1) - (both && n % 4 == 0 && n > 0 ? 2 : 0); }
+
+int phase_pairs(const StepPlan& pl, int phase) {
+    return phase == 0 ? (pl.fuseP ? fused_pairs(pl.maxP) : 0) : (pl.fuseR ? fused_pairs(pl.maxR, pl.bothR) : 0);
+}
 
 int jacobi_phase_launches(const StepPlan& pl, int phase) {
     const int n = phase == 0 ? pl.maxP : pl.maxR;
     if (pl.res) return n > 0 ? 1 : 0;
-    const bool fuse = phase == 0 ? pl.fuseP : pl.fuseR;
-    return fuse ? n - fused_pairs(n) : n;
+    return n - phase_pairs(pl, phase);
 }
 
 void enqueue_jacobi_phase(cudaStream_t st, const StepPlan& pl, FxBatchDev* B, int phase) {
@@ -184,12 +189,9 @@ void enqueue_jacobi_phase(cudaStream_t st, const StepPlan& pl, FxBatchDev* B, in
                                  phase == 1 && pl.projRes, pl.two);
         return;
     }
-    const bool fuse = phase == 0 ? pl.fuseP : pl.fuseR;
     int launch = 0, sweep = 0;
-    if (fuse) {
-        for (; launch < fused_pairs(n); sweep += 2, ++launch)
-            fx_launch_jacobi_two(st, pl.half, B, pl.bricks[FX_SHAPE_COL], phase, launch, pl.zrun, pl.tma, pl.two);
-    }
+    for (; launch < phase_pairs(pl, phase); sweep += 2, ++launch)
+        fx_launch_jacobi_two(st, pl.half, B, pl.bricks[FX_SHAPE_COL], phase, launch, pl.zrun, pl.tma, pl.two);
     for (; sweep < n; ++sweep, ++launch) {
         if (pl.row4) fx_launch_jacobi(st, pl.half, B, pl.bricks[FX_SHAPE_ROW4], phase, launch, sweep);
         else fx_launch_jacobi_zm(st, pl.half, B, pl.bricks[FX_SHAPE_ZM], phase, launch, sweep, pl.zmZc);
@@ -836,7 +838,11 @@ struct firex_batch {
         p.zc = zc > 0 ? zc : 16;
         p.zrun = zcOwn ? p.zc : (k == 2 ? fx_zs_run(dims(), p.half, fx_zs_capacity(p.half)) : 16);
         p.fuseP = k == 2 && uniformP && fused_pairs(p.maxP) > 0;
-        p.fuseR = k == 2 && uniformR && fused_pairs(p.maxR) > 0;
+        // a cold start's two solves share their buffers, and the pressure is read from p[P & 1]: with P
+        // and R of different parity that is the residual solve's other buffer
+        for (firex_sim* s : members)
+            p.bothR = p.bothR || (s->mode == FIREX_PRESSURE_COLD_F32 && ((s->h.P ^ s->h.R) & 1));
+        p.fuseR = k == 2 && uniformR && fused_pairs(p.maxR, p.bothR) > 0;
         if (!p.fuseP && !p.fuseR) p.k = 1;
         // single sweeps of a phase that does not fuse, or is left over: unblocked while AUTO's batch stays
         // in L2 (us per sweep, unblocked and z-marching: 144x216x136 15.7 and 18.5, 160x240x160 21.0 and

@@ -343,7 +343,8 @@ int firex_set_graphs(firex_sim* sim, int32_t on);
  *               (with FP16 pressure storage the first sweep is rounded as a stored one). A
  *               phase runs an even number of fused launches and its last sweeps, up to three,
  *               one by one, so that its result lands in the buffer of the pair that single
- *               sweeps leave it in.
+ *               sweeps leave it in (four where the other buffer is observable, as after a cold
+ *               start with sweep counts of different parity).
  * `zchunk`: z planes per CTA for ZMARCH and FUSED (0 = auto: FUSED fits them to the device,
  * firex_diagnostics.jacobi_zrun). AUTO takes RESIDENT when the batch fits on chip, else by its
  * cell count: UNBLOCKED below 2 Mi cells and for grids so narrow or flat that 32 x 14 tiles stay

@@ -221,3 +221,24 @@ def test_auto_runs_unblocked_sweeps_where_no_phase_fuses():
         assert members[0].diagnostics["jacobi_kernel"] == A.JACOBI_UNBLOCKED, members[0].diagnostics
     for a, m in zip(alone, members):
         same(a, m)
+
+
+# ---- a cold start's shared buffers -----------------------------------------------------------------
+
+@pytest.mark.parametrize("P,R", [(13, 8), (5, 4), (7, 12), (8, 9), (6, 11), (13, 10), (8, 8)])
+@pytest.mark.parametrize("staging", [A.STAGING_CPASYNC, A.STAGING_TMA])
+def test_cold_start_leaves_the_last_two_sweeps(P, R, staging):
+    """The pressure is read from buffer P mod 2, which both solves of a cold start share: with R of the
+    other parity it holds the residual solve's last sweep but one."""
+    pair((36, 32, 20), P=P, R=R, staging=staging, pressure_mode=A.PRESSURE_COLD_F32)
+
+
+def test_auto_with_a_cold_start_beyond_the_chip():
+    dims = (160, 216, 152)
+    opts = sphere_options(dims, P=5, R=8, pressure_mode=A.PRESSURE_COLD_F32)
+    auto, one = FireXSim(dims, opts), FireXSim(dims, opts)
+    one.set_jacobi("unblocked")
+    auto.step(2, DT)
+    one.step(2, DT)
+    assert auto.diagnostics["jacobi_kernel"] == A.JACOBI_FUSED
+    same(auto, one)
