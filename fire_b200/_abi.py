@@ -159,7 +159,8 @@ class Diagnostics(C.Structure):
         ("project_resident", C.c_int32),
         ("jacobi_zrun", C.c_int32),
         ("jacobi_registers", C.c_int32),
-        ("reserved", C.c_int32 * 3),
+        ("jacobi_two_op", C.c_int32),
+        ("reserved", C.c_int32 * 2),
     ]
 
 

@@ -156,12 +156,11 @@ struct __align__(16) FxSimDev {
     float jc[4];           // Jacobi wx, wy, wz, 2(wx+wy+wz) (shaders.ts:386-389), f32
     float jcRcp;           // RN(1 / jc[3])
     int jcFastDiv;         // 1: x / jc[3] may use fx_div_by_const (checked exhaustively)
-    int jcTwo;             // 1: x / jc[3] may use the two-operation quotient (checked exhaustively)
+    int jcTwo;             // 1: x / jc[3] may use the two-operation quotient (checked on the device)
     float jcRh, jcRl;      // its reciprocal 1 / jc[3] as a sum of two floats, jcRl > 0
     float jcLo;            // smallest |x| it was checked for
     double jcRcpD;         // RN(1 / jc[3]) in double: the quotients below jcLo
-    int simTwo;            // 1: the fixed divisors of simulate may use their two operations (fx_div_two_of)
-    int pad2[11];
+    int pad2[12];
     void* flow[2];         // float4 records (both storages)
     void* species[2];      // float4 (F32) or 4 x half (MIXED)
     void* p[2];            // primary pressure: float (F32 / COLD) or half (F16 / MIXED)

@@ -146,12 +146,11 @@ struct StepPlan {
     bool resReg = false;      // ... with the pressure in registers (variant 4)
     int resSmem = 0;          // its dynamic shared memory per CTA
     bool projRes = false;     // the residual projection inside the resident launch (variant 4)
-    bool simTwo = false;      // the source pass divides by its fixed divisors in two operations
     bool simEarly = false;    // the source pass evaluates its neighbour terms before the advection
     int bricks[FX_NSHAPES] = {};
     auto key() const {
         return std::tie(storage, half, maxP, maxR, k, zc, zrun, zmZc, row4, fuseP, fuseR, bothR, pack, tma, two, simBy, projDiv, res,
-                        resVariant, resReg, resSmem, projRes, simEarly, simTwo,
+                        resVariant, resReg, resSmem, projRes, simEarly,
                         bricks[0],
                         bricks[1], bricks[2], bricks[3], bricks[4], bricks[5], bricks[6]);
     }
@@ -205,7 +204,7 @@ void enqueue_step_launches(cudaStream_t st, const StepPlan& pl, FxBatchDev* B) {
     fx_launch_step_begin(st, B);
     fx_launch_step_tables(st, B, pl.bricks[FX_SHAPE_TAB]);
     if (sph_launches(pl)) fx_launch_sph(st, B, pl.bricks[FX_SHAPE_ROW4], pl.bricks[FX_SHAPE_PART]);
-    fx_launch_simulate(st, pl.storage, pl.simBy, pl.simEarly, pl.simTwo, B, pl.bricks[FX_SHAPE_CELL]);
+    fx_launch_simulate(st, pl.storage, pl.simBy, pl.simEarly, B, pl.bricks[FX_SHAPE_CELL]);
     fx_launch_divergence(st, B, pl.bricks[FX_SHAPE_ROW4], 0);
     enqueue_jacobi_phase(st, pl, B, 0);
     if (pl.projDiv) {
@@ -268,9 +267,9 @@ static bool fast_division_ok(int device, float d, float rcp, float lo = 1.262177
     return ok;
 }
 
-// The reciprocal 1/d = rh + rl (rh rounded down, so rl > 0) with which fx_div_two equals IEEE
-// x / d for every float x on this device, checked like fast_division_ok: rl rounded to nearest,
-// or one or two steps beside it (that rounding decides the few quotients next to a midpoint).
+// The reciprocal with which fx_div_two equals IEEE x / d for every float x: the first candidate of
+// fx_two_op_candidates that passes on this device over a binade of x. Checks are kept by divisor; a
+// call that fails is not an answer and is not kept.
 struct TwoOpReciprocal {
     bool ok = false;
     float rh = 0, rl = 0, lo = 0;
@@ -285,35 +284,28 @@ static TwoOpReciprocal two_op_reciprocal(int device, float d) {
     std::memcpy(&bits, &d, 4);
     auto it = cache.find({device, bits});
     if (it != cache.end()) return it->second;
-    const double rcp = 1.0 / (double)d;
-    r.rh = (float)rcp;
-    if ((double)r.rh > rcp) r.rh = std::nextafter(r.rh, 0.0f);
-    float rl = (float)(rcp - (double)r.rh);
-    if (rl == 0.0f) rl = std::ldexp(r.rh, -60);  // a power of two: any tiny positive term rounds away
-    r.lo = std::ldexp(1.0f, -60 + std::ilogb(d));
-    const float up = std::nextafter(rl, INFINITY), down = std::nextafter(rl, 0.0f);
-    const float tries[5] = {rl, up, down, std::nextafter(up, INFINITY), std::nextafter(down, 0.0f)};
-    unsigned long long* dcount = nullptr;
+    const FxTwoOp two = fx_two_op_candidates(d);
+    unsigned bad[5], *dcount = nullptr;
     cudaStream_t st = nullptr;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
-        cudaMalloc(&dcount, sizeof(unsigned long long)) == cudaSuccess) {
-        for (float t : tries) {
-            unsigned long long bad = ~0ull;
-            if (cudaMemsetAsync(dcount, 0, sizeof(bad), st) != cudaSuccess) break;
-            fx_launch_check_div_two(st, d, r.rh, t, r.lo, rcp, dcount);
-            if (cudaMemcpyAsync(&bad, dcount, sizeof(bad), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess)
-                break;
-            if (bad == 0) {
-                r.ok = true;
-                r.rl = t;
-                break;
-            }
-        }
+    bool done = false;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess && cudaMalloc(&dcount, sizeof(bad)) == cudaSuccess &&
+        cudaMemsetAsync(dcount, 0, sizeof(bad), st) == cudaSuccess) {
+        fx_launch_check_div_two(st, d, two, dcount);
+        done = cudaGetLastError() == cudaSuccess &&
+               cudaMemcpyAsync(bad, dcount, sizeof(bad), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+               cudaStreamSynchronize(st) == cudaSuccess;
     }
     cudaGetLastError();
     if (dcount) cudaFree(dcount);
     if (st) cudaStreamDestroy(st);
+    if (!done) return r;
+    r.rh = two.rh;
+    r.lo = two.lo;
+    for (int k = 0; k < 5 && !r.ok; ++k)
+        if (bad[k] == 0) {
+            r.ok = true;
+            r.rl = two.rl[k];
+        }
     cache[{device, bits}] = r;
     return r;
 }
@@ -402,31 +394,6 @@ struct ExchangePool {
 };
 ExchangePool g_exchange;
 }  // namespace
-
-// Whether the fixed divisors of simulate have their two-operation quotients on this device
-// (fx_div_two_of), checked like the others, once per device.
-static bool fixed_divisors_ok(int device) {
-    static std::map<int, bool> cache;
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(device);
-    if (it != cache.end()) return it->second;
-    unsigned long long bad = ~0ull, *dcount = nullptr;
-    cudaStream_t st = nullptr;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess && cudaMalloc(&dcount, sizeof(bad)) == cudaSuccess &&
-        cudaMemsetAsync(dcount, 0, sizeof(bad), st) == cudaSuccess) {
-        for (int k = 0; k < FX_DIV_TWO_COUNT; ++k) {
-            const FxDivTwo c = fx_div_two_of(k);
-            fx_launch_check_div_two(st, c.d, c.rh, c.rl, FX_DIV_TWO_LO, 1.0 / (double)c.d, dcount);
-        }
-        if (cudaMemcpyAsync(&bad, dcount, sizeof(bad), cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
-            bad = ~0ull;
-    }
-    cudaGetLastError();
-    if (dcount) cudaFree(dcount);
-    if (st) cudaStreamDestroy(st);
-    return cache[device] = bad == 0;
-}
 
 // ---- one simulation ------------------------------------------------------------------------
 struct firex_sim {
@@ -585,7 +552,6 @@ struct firex_sim {
         const float divisors[DIVC_COUNT] = {
             6.0f, 0.78f - 0.30f, 1500.0f - 400.0f, 930.0f - 690.0f, 1650.0f - 520.0f, 1040.0f - 335.0f,
             0.48f - (-0.42f), 1500.0f, fmaxr(u[9], 0.001f), fmaxr(u[4], 0.0001f), 1005.0f * persistence};
-        h.simTwo = fixed_divisors_ok(device) ? 1 : 0;
         for (int k = 0; k < DIVC_COUNT; ++k) {
             FxDivc& c = h.divc[k];
             std::memset(&c, 0, sizeof(c));
@@ -595,7 +561,9 @@ struct firex_sim {
             c.hi = (float)std::min(3.4028234663852886e38, 3.4028234663852886e38 * std::min(1.0, (double)c.d) * 0.5);
             // dt may change every call: its divisor keeps the IEEE division rather than
             // paying the device check per new value
-            c.ok = (k != DIVC_DT && c.d > 0.0f && c.d < 1073741824.0f && fast_division_ok(device, c.d, c.rcp, c.lo, c.hi)) ? 1 : 0;
+            // the fixed divisors past the sixth divide in two operations and are not read from here
+            const bool read = k == DIVC_SIX || k >= FX_DIV_TWO_COUNT;
+            c.ok = (read && k != DIVC_DT && c.d > 0.0f && c.d < 1073741824.0f && fast_division_ok(device, c.d, c.rcp, c.lo, c.hi)) ? 1 : 0;
             // not enabled: an empty fast range sends every x to the IEEE division (fx_divc)
             if (!c.ok) c.lo = INFINITY;
         }
@@ -873,10 +841,8 @@ struct firex_batch {
         for (firex_sim* s : members) maps = maps && s->h.tmapOk;
         p.tma = p.k == 2 && maps;
         p.two = true;
-        p.simTwo = true;
         for (firex_sim* s : members) {
             p.two = p.two && s->h.jcTwo;
-            p.simTwo = p.simTwo && s->h.simTwo;
         }
         if (tableK != p.k || tableZc != p.zrun || tableZmZc != p.zmZc || tableRes != (wantRes ? 2 + resForce : 0) ||
             tableWater != water_signature() || tableSimBy != p.simBy || tableTma != p.tma)
@@ -953,7 +919,7 @@ struct firex_batch {
             fx_launch_sph(stream, d, pl.bricks[FX_SHAPE_ROW4], pl.bricks[FX_SHAPE_PART]);
             mark(FIREX_PASS_PARTICLES, sph_launches(pl));
         }
-        fx_launch_simulate(stream, pl.storage, pl.simBy, pl.simEarly, pl.simTwo, d, pl.bricks[FX_SHAPE_CELL]);
+        fx_launch_simulate(stream, pl.storage, pl.simBy, pl.simEarly, d, pl.bricks[FX_SHAPE_CELL]);
         mark(FIREX_PASS_SIMULATE, 1);
         fx_launch_divergence(stream, d, pl.bricks[FX_SHAPE_ROW4], 0);
         mark(FIREX_PASS_DIVERGENCE, 1);
@@ -1830,6 +1796,7 @@ int firex_get_diagnostics(const firex_sim* s, firex_diagnostics* out) {
     out->project_fused = p.projDiv ? 1 : 0;
     out->project_resident = p.projRes ? 1 : 0;
     out->jacobi_registers = p.res && p.resReg ? 1 : 0;
+    out->jacobi_two_op = p.two ? 1 : 0;
     return FIREX_OK;
 }
 

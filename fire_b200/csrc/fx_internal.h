@@ -16,8 +16,7 @@ void fx_launch_step_end(cudaStream_t s, FxBatchDev* B);
 void fx_launch_step_tables(cudaStream_t s, const FxBatchDev* B, int bricks);
 // The source pass with bricks of 32 x by x (8 / by) cells (by = 2, 4 or 8).
 // early: the neighbour terms before the advection (fx_simulate_cell<EARLY>; same results).
-// two: the fixed divisors by their checked two operations (FxSimDev::simTwo of every member).
-void fx_launch_simulate(cudaStream_t s, int storage, int by, bool early, bool two, const FxBatchDev* B, int bricks);
+void fx_launch_simulate(cudaStream_t s, int storage, int by, bool early, const FxBatchDev* B, int bricks);
 void fx_launch_divergence(cudaStream_t s, const FxBatchDev* B, int bricks, int phase);
 void fx_launch_jacobi(cudaStream_t s, bool half, const FxBatchDev* B, int bricks, int phase, int launch, int sweep);
 // One sweep by z-marching tiles of zc planes (fx_jacobi_zm.cuh).
@@ -68,8 +67,8 @@ void fx_launch_upload_batch(cudaStream_t s, const FxBatchDev& host, FxBatchDev* 
 // Exhaustive check of fx_div_by_const against IEEE division for one denominator.
 void fx_launch_check_div(cudaStream_t s, float d, float rcp, float lo, float hi, unsigned long long* mismatches);
 
-// The same for fx_div_two with the reciprocal rh + rl and the small-operand bound lo.
-void fx_launch_check_div_two(cudaStream_t s, float d, float rh, float rl, float lo, double rcp, unsigned long long* mismatches);
+// fx_div_two against IEEE division over one binade of x, for each of the five candidates.
+void fx_launch_check_div_two(cudaStream_t s, float d, const FxTwoOp& two, unsigned* mismatches);
 
 // Sets the text that firex_last_error(NULL) returns on the calling thread (fx_engine.cu).
 void fx_set_thread_error(const std::string& msg);

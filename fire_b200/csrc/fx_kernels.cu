@@ -95,14 +95,13 @@ struct Acc {
 };
 
 // One thread per cell of a 32 x BY x (8 / BY) brick (BY = 2, 4 or 8: the tunable brick
-// shape; FX_CELL_BY, 4, by default). EARLY: the neighbour terms before the advection, TWO: the fixed
-// divisors in two operations and records in pairs (fx_simulate_cell).
+// shape; FX_CELL_BY, 4, by default). EARLY: the neighbour terms before the advection (fx_simulate_cell).
 // Bound by the latency of its gathers and by issue slots (55 % busy; L1 data pipe 55-59 %): 955
 // instructions a warp and cell, 1292 before pairs, two-operation divisions, T^4 by two double
 // products and brick places by carries; 128x192x128 157 us a pass (186 before), 160x240x160 298
 // (350), 300x452x276 2.22 ms (2.67), 508^3 8.0 ms (8.98). Two CTAs per SM without spills: 508^3 7.7 ms,
 // but 128x192x128 178 us and twelve uneven grids 1.77 ms against 1.53; four at 64 registers: no faster.
-template <class St, int BY, bool EARLY, bool TWO>
+template <class St, int BY, bool EARLY>
 __global__ void __launch_bounds__(256, 3) fxk_simulate(const FxBatchDev* __restrict__ B) {
     constexpr int BX = FX_CELL_BX, BZ = 256 / (FX_CELL_BX * BY);
     // the simulation's parameter block, the uniform entries of its per-step table and its
@@ -157,7 +156,7 @@ __global__ void __launch_bounds__(256, 3) fxk_simulate(const FxBatchDev* __restr
         if (x >= S.X || y >= S.Y || z >= S.Z) return;
         const FxGrid g{S.X, S.Y, S.Z};
         Acc<St> a{S.flow[S.fi], S.species[S.si], S.liquid};
-        const FxCellOut o = fx_simulate_cell<EARLY, TWO>(sP, g, x, y, z, a, S.tab, sL, sUT, sDC);
+        const FxCellOut o = fx_simulate_cell<EARLY>(sP, g, x, y, z, a, S.tab, sL, sUT, sDC);
         const int id = x + S.X * (y + S.Y * z);
         fx_st_flow(S.flow[S.fi ^ 1], id, o.flow);
         St::st_species(S.species[S.si ^ 1], id, o.species);
@@ -590,17 +589,16 @@ __global__ void fxk_check_div(float d, float rcp, float lo, float hi, unsigned l
     if (bad) atomicAdd(mismatches, bad);
 }
 
-// The same for fx_div_two.
-__global__ void fxk_check_div_two(float d, float rh, float rl, float lo, double rcp, unsigned long long* __restrict__ mismatches) {
-    unsigned long long bad = 0;
-    const unsigned long long n = 1ull << 32;
-    for (unsigned long long b = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; b < n;
-         b += (unsigned long long)gridDim.x * blockDim.x) {
-        const float x = __uint_as_float((unsigned)b);
-        const float a = fx_div_two(x, rh, rl, lo, d, rcp), e = __fdiv_rn(x, d);
-        bad += (__float_as_uint(a) != __float_as_uint(e)) && !(a != a && e != e);
+// Counts the floats x of [1, 2) for which the two operations differ from the IEEE quotient, for the
+// candidate blockIdx.y. A new denominator costs 0.2 ms so; every float took 4 ms a candidate.
+__global__ void fxk_check_div_two(float d, FxTwoOp two, unsigned* __restrict__ mismatches) {
+    const float rl = two.rl[blockIdx.y];
+    unsigned bad = 0;
+    for (unsigned m = blockIdx.x * blockDim.x + threadIdx.x; m < 1u << 23; m += gridDim.x * blockDim.x) {
+        const float x = __uint_as_float(0x3f800000u | m);
+        bad += __fmaf_rn(x, two.rh, __fmul_rn(x, rl)) != __fdiv_rn(x, d);
     }
-    if (bad) atomicAdd(mismatches, bad);
+    if (bad) atomicAdd(mismatches + blockIdx.y, bad);
 }
 
 // ---- single-simulation utilities -----------------------------------------------------------
@@ -934,28 +932,26 @@ void fx_launch_step_tables(cudaStream_t s, const FxBatchDev* B, int bricks) {
     fxk_step_tables<<<bricks > 0 ? bricks : 1, 256, 0, s>>>(B);
 }
 
-template <class St, int BY, bool EARLY, bool TWO>
+template <class St, int BY, bool EARLY>
 static void launch_simulate(cudaStream_t s, const FxBatchDev* B, int bricks) {
-    static int g = persistent_grid((const void*)fxk_simulate<St, BY, EARLY, TWO>, 256, 1 << 30);
-    fxk_simulate<St, BY, EARLY, TWO><<<bricks < g ? bricks : g, 256, 0, s>>>(B);
+    static int g = persistent_grid((const void*)fxk_simulate<St, BY, EARLY>, 256, 1 << 30);
+    fxk_simulate<St, BY, EARLY><<<bricks < g ? bricks : g, 256, 0, s>>>(B);
 }
 
-template <class St, bool EARLY, bool TWO>
+template <class St, bool EARLY>
 static void launch_simulate_shape(cudaStream_t s, int by, const FxBatchDev* B, int bricks) {
-    if (by == 2) launch_simulate<St, 2, EARLY, TWO>(s, B, bricks);
-    else if (by == 8) launch_simulate<St, 8, EARLY, TWO>(s, B, bricks);
-    else launch_simulate<St, 4, EARLY, TWO>(s, B, bricks);
+    if (by == 2) launch_simulate<St, 2, EARLY>(s, B, bricks);
+    else if (by == 8) launch_simulate<St, 8, EARLY>(s, B, bricks);
+    else launch_simulate<St, 4, EARLY>(s, B, bricks);
 }
 
-void fx_launch_simulate(cudaStream_t s, int storage, int by, bool early, bool two, const FxBatchDev* B, int bricks) {
+void fx_launch_simulate(cudaStream_t s, int storage, int by, bool early, const FxBatchDev* B, int bricks) {
     if (storage == FX_STORAGE_MIXED) {
-        if (!two) launch_simulate_shape<StMixed, false, false>(s, by, B, bricks);
-        else if (early) launch_simulate_shape<StMixed, true, true>(s, by, B, bricks);
-        else launch_simulate_shape<StMixed, false, true>(s, by, B, bricks);
+        if (early) launch_simulate_shape<StMixed, true>(s, by, B, bricks);
+        else launch_simulate_shape<StMixed, false>(s, by, B, bricks);
     } else {
-        if (!two) launch_simulate_shape<StF32, false, false>(s, by, B, bricks);
-        else if (early) launch_simulate_shape<StF32, true, true>(s, by, B, bricks);
-        else launch_simulate_shape<StF32, false, true>(s, by, B, bricks);
+        if (early) launch_simulate_shape<StF32, true>(s, by, B, bricks);
+        else launch_simulate_shape<StF32, false>(s, by, B, bricks);
     }
 }
 
@@ -1201,6 +1197,6 @@ void fx_launch_check_div(cudaStream_t s, float d, float rcp, float lo, float hi,
     fxk_check_div<<<num_sms() * 16, 256, 0, s>>>(d, rcp, lo, hi, mismatches);
 }
 
-void fx_launch_check_div_two(cudaStream_t s, float d, float rh, float rl, float lo, double rcp, unsigned long long* mismatches) {
-    fxk_check_div_two<<<num_sms() * 16, 256, 0, s>>>(d, rh, rl, lo, rcp, mismatches);
+void fx_launch_check_div_two(cudaStream_t s, float d, const FxTwoOp& two, unsigned* mismatches) {
+    fxk_check_div_two<<<dim3(num_sms() * 2, 5), 256, 0, s>>>(d, two, mismatches);
 }

@@ -91,6 +91,50 @@ FX_HOST_DEVICE long long fx_reg_smem_bytes(int X, const FxRegGeom& g) {
 // Quads a box sends per sweep: sections y low, y high (bz rows), z low, z high (by rows).
 FX_HOST_DEVICE int fx_reg_outbox_quads(int X, const FxResBox& bx) { return 2 * (bx.by + bx.bz) * (X / 4); }
 
+// ---- division by a constant in two operations (fx_div_two, fx_step_math.cuh) ------------------------
+// The reciprocal 1/d = rh + rl, rh rounded down so that rl > 0 (zeros keep their signs, infinities and
+// NaN pass), with rl rounded to nearest or one or two steps beside it: that rounding decides the few
+// quotients next to a midpoint. From lo on, x rl and x / d are normal: a power of two on x then
+// scales both products and the quotient exactly, and one binade of x decides.
+struct FxTwoOp {
+    float rh, rl[5], lo;
+};
+inline FxTwoOp fx_two_op_candidates(float d) {
+    FxTwoOp t;
+    const double rcp = 1.0 / (double)d;
+    t.rh = (float)rcp;
+    if ((double)t.rh > rcp) t.rh = std::nextafter(t.rh, 0.0f);
+    float rl = (float)(rcp - (double)t.rh);
+    if (rl == 0.0f) rl = std::ldexp(t.rh, -60);  // a power of two: any tiny positive term rounds away
+    t.rl[0] = rl;
+    t.rl[1] = std::nextafter(rl, INFINITY);
+    t.rl[2] = std::nextafter(rl, 0.0f);
+    t.rl[3] = std::nextafter(t.rl[1], INFINITY);
+    t.rl[4] = std::nextafter(t.rl[2], 0.0f);
+    t.lo = std::ldexp(1.0f, -60 + std::ilogb(d));
+    return t;
+}
+
+// The fixed divisors of simulate, by their slot (FxDivSlot): d and a reciprocal that is right for
+// zeros, infinities, NaN and every float x of magnitude 2^-27 and above (slot 0: FX_DIV_TWO_LO).
+struct FxDivTwo {
+    float d, rh, rl;
+};
+#define FX_DIV_TWO_LO 7.888609052210118e-31f  // 2^-100
+#define FX_DIV_TWO_COUNT 8
+FX_HOST_DEVICE FxDivTwo fx_div_two_of(int slot) {
+    switch (slot) {
+        case 0: return {6.0f, 0x1.555554p-3f, 0x1.555556p-27f};                    // DIVC_SIX
+        case 1: return {0.78f - 0.30f, 0x1.0aaaacp+1f, 0x1.238e4ap-26f};           // DIVC_FUELCORE
+        case 2: return {1500.0f - 400.0f, 0x1.dca01cp-11f, 0x1.ca01dcp-35f};       // DIVC_ENTRAIN_T
+        case 3: return {930.0f - 690.0f, 0x1.11111p-8f, 0x1.111112p-32f};          // DIVC_IGNITION
+        case 4: return {1650.0f - 520.0f, 0x1.cff8cp-11f, 0x1.cff8cp-39f};         // DIVC_HOTPLUME
+        case 5: return {1040.0f - 335.0f, 0x1.73d5ep-10f, 0x1.8b133ep-35f};        // DIVC_EVAP
+        case 6: return {0.48f - (-0.42f), 0x1.1c71c6p+0f, 0x1.9add3cp-24f};        // DIVC_LOBE
+        default: return {1500.0f, 0x1.5d867cp-11f, 0x1.f67152p-38f};               // DIVC_BUOYANCY
+    }
+}
+
 // ---- plans (host) ---------------------------------------------------------------------------------
 // Cells of these grids over the cells of the strip tiles that cover them: 1 where 32 x 14 tiles fit.
 inline double fx_zs_fill(const std::vector<std::array<int, 3>>& dims) {

@@ -88,56 +88,34 @@ FXD FxQuad fx_quad_zero() { return fx_quad(make_float4(0.0f, 0.0f, 0.0f, 0.0f));
 FXD float2 fx_bcast2(float v) { return make_float2(v, v); }
 
 // The fixed divisors of simulate in two operations: RN(x rh + RN(x rl)) with 1/d = rh + rl, rh
-// rounded down (fx_div_two below has the method), is x / d for every float x of magnitude 2^-100
-// and above, for zeros, infinities and NaN. The engine checks that on the device for every float
-// before the source pass uses them (FxSimDev::simTwo), else the pass divides by fx_divc.
-struct FxDivTwo {
-    float d, rh, rl;
-};
-#define FX_DIV_TWO_LO 7.888609052210118e-31f  // 2^-100
-#define FX_DIV_TWO_COUNT 8
-__host__ __device__ inline FxDivTwo fx_div_two_of(int slot) {
-    switch (slot) {
-        case DIVC_SIX: return {6.0f, 0x1.555554p-3f, 0x1.555556p-27f};
-        case DIVC_FUELCORE: return {0.78f - 0.30f, 0x1.0aaaacp+1f, 0x1.238e4ap-26f};
-        case DIVC_ENTRAIN_T: return {1500.0f - 400.0f, 0x1.dca01cp-11f, 0x1.ca01dcp-35f};
-        case DIVC_IGNITION: return {930.0f - 690.0f, 0x1.11111p-8f, 0x1.111112p-32f};
-        case DIVC_HOTPLUME: return {1650.0f - 520.0f, 0x1.cff8cp-11f, 0x1.cff8cp-39f};
-        case DIVC_EVAP: return {1040.0f - 335.0f, 0x1.73d5ep-10f, 0x1.8b133ep-35f};
-        case DIVC_LOBE: return {0.48f - (-0.42f), 0x1.1c71c6p+0f, 0x1.9add3cp-24f};
-        default: return {1500.0f, 0x1.5d867cp-11f, 0x1.f67152p-38f};  // DIVC_BUOYANCY
-    }
-}
-static_assert(DIVC_BUOYANCY == FX_DIV_TWO_COUNT - 1, "the fixed divisors come first");
-// x / d of slot SLOT without a range check, for an x that is 0 or no smaller than 2^-100: a
+// rounded down (fx_div_two below has the method), is x / d for every x that the pass divides so
+// (fx_div_two_of; tests/test_plan.py checks its literals).
+static_assert(DIVC_SIX == 0 && DIVC_FUELCORE == 1 && DIVC_ENTRAIN_T == 2 && DIVC_IGNITION == 3 && DIVC_HOTPLUME == 4 &&
+                  DIVC_EVAP == 5 && DIVC_LOBE == 6 && DIVC_BUOYANCY == FX_DIV_TWO_COUNT - 1,
+              "the slots of fx_div_two_of");
+// x / d of slot SLOT without a range check, for an x that is 0 or no smaller than 2^-27: a
 // difference from a constant of at least 0.3, whose neighbouring floats are 2^-26 apart.
 template <int SLOT>
 FXD float fx_div_fixed(float x) {
     const FxDivTwo c = fx_div_two_of(SLOT);
     return __fmaf_rn(x, c.rh, __fmul_rn(x, c.rl));
 }
-// (x - e0) / d of slot SLOT by the two operations (TWO) or by fx_divc, and its smoothstep.
-template <bool TWO, int SLOT>
-FXD float fx_div_from(float e0, float x, const FxDivc* dc) {
-    return TWO ? fx_div_fixed<SLOT>(x - e0) : fx_divc(x - e0, dc[SLOT]);
-}
-template <bool TWO, int SLOT>
-FXD float fx_smoothstep_from(float e0, float x, const FxDivc* dc) {
-    const float t = fx_clamp(fx_div_from<TWO, SLOT>(e0, x, dc), 0.0f, 1.0f);
+// The smoothstep from e0 with the denominator of slot SLOT.
+template <int SLOT>
+FXD float fx_smoothstep_from(float e0, float x) {
+    const float t = fx_clamp(fx_div_fixed<SLOT>(x - e0), 0.0f, 1.0f);
     return t * t * (3.0f - 2.0f * t);
 }
-// A sixth of each of four sums (shaders.ts:177-187). TWO: two operations a pair, unless one of the
+// A sixth of each of four sums (shaders.ts:177-187) in two operations a pair, unless one of the
 // sums is too small for them, as at the faint edge of a diffusing field (zeros are not).
-FXD float4 fx_sixth(const float4& s, const FxDivc* dc) {
-    return make_float4(fx_divc(s.x, dc[DIVC_SIX]), fx_divc(s.y, dc[DIVC_SIX]), fx_divc(s.z, dc[DIVC_SIX]), fx_divc(s.w, dc[DIVC_SIX]));
-}
 FXD unsigned fx_mag(float x) { return 2u * __float_as_uint(x) - 1u; }  // ascends with |x|; zeros come last
-FXD float4 fx_sixth_two(const FxQuad& s, const FxDivc* dc) {
+FXD float4 fx_sixth(const FxQuad& s, const FxDivc* dc) {
     const FxDivTwo c = fx_div_two_of(DIVC_SIX);
     const float2 rh = fx_bcast2(c.rh), rl = fx_bcast2(c.rl);
     const float2 a = __ffma2_rn(s.a, rh, __fmul2_rn(s.a, rl)), b = __ffma2_rn(s.b, rh, __fmul2_rn(s.b, rl));
     const unsigned least = min(min(fx_mag(s.a.x), fx_mag(s.a.y)), min(fx_mag(s.b.x), fx_mag(s.b.y)));
-    if (least < fx_mag(FX_DIV_TWO_LO)) return fx_sixth(make_float4(s.a.x, s.a.y, s.b.x, s.b.y), dc);
+    if (least < fx_mag(FX_DIV_TWO_LO))
+        return make_float4(fx_divc(s.a.x, dc[DIVC_SIX]), fx_divc(s.a.y, dc[DIVC_SIX]), fx_divc(s.b.x, dc[DIVC_SIX]), fx_divc(s.b.y, dc[DIVC_SIX]));
     return make_float4(a.x, a.y, b.x, b.y);
 }
 FXD FxQuad fx_add4(const FxQuad& a, const FxQuad& b) { return FxQuad{__fadd2_rn(a.a, b.a), __fadd2_rn(a.b, b.b)}; }
@@ -176,16 +154,7 @@ FXD FxTri fx_tri_setup(const FxGrid& g, const float* u, float px, float py, floa
     return t;
 }
 template <class Load>
-FXD float4 fx_trilinear(const FxGrid& g, const FxTri& t, Load load) {
-    const int X = g.X, XY = g.X * g.Y, b = t.base;
-    float4 c000 = load(b), c100 = load(b + 1), c010 = load(b + X), c110 = load(b + X + 1);
-    float4 c001 = load(b + XY), c101 = load(b + XY + 1), c011 = load(b + XY + X), c111 = load(b + XY + X + 1);
-    float4 z0 = fx_mix4(fx_mix4(c000, c100, t.fx), fx_mix4(c010, c110, t.fx), t.fy);
-    float4 z1 = fx_mix4(fx_mix4(c001, c101, t.fx), fx_mix4(c011, c111, t.fx), t.fy);
-    return fx_mix4(z0, z1, t.fz);
-}
-template <class Load>
-FXD float4 fx_trilinear_two(const FxGrid& g, const FxTri& t, float nz, Load load) {
+FXD float4 fx_trilinear(const FxGrid& g, const FxTri& t, float nz, Load load) {
     const int X = g.X, XY = g.X * g.Y, b = t.base;
     auto plane = [&](int i) {
         const FxQuad lo = fx_mix_two(fx_quad(load(i)), fx_quad(load(i + 1)), t.fx, nz);
@@ -366,8 +335,7 @@ struct FxCellOut {
 // P, ut (the per-step table's uniform entries, TU_*) and dc are the same for every cell of a
 // simulation: the source pass stages them in shared memory; tab (the per-coordinate tables)
 // and the fields come from global memory.
-// TWO: the fixed divisors in two operations and the records in pairs.
-template <bool EARLY, bool TWO, class Acc>
+template <bool EARLY, class Acc>
 FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y, int z, const Acc& a,
                                const float* __restrict__ tab, const FxTabLayout& L, const float* ut, const FxDivc* dc) {
     const float* u = P.u;
@@ -395,15 +363,9 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     float gx, gy, gz;         // normalised grad(T) (shaders.ts:264-268)
     float4 avg;               // species diffusion (shaders.ts:182-187)
     float4 left, right, bottom, top, back, front;
-    const float nz = TWO ? ut[TU_NZ] : 0.0f;
+    const float nz = ut[TU_NZ];
     auto sixth = [&](const float4& l, const float4& r, const float4& b, const float4& t, const float4& k, const float4& f) {
-        if constexpr (TWO) {
-            const FxQuad s = fx_add4(fx_add4(fx_add4(fx_add4(fx_add4(fx_quad(l), fx_quad(r)), fx_quad(b)), fx_quad(t)), fx_quad(k)), fx_quad(f));
-            return fx_sixth_two(s, dc);
-        } else {
-            return fx_sixth(make_float4(l.x + r.x + b.x + t.x + k.x + f.x, l.y + r.y + b.y + t.y + k.y + f.y,
-                                        l.z + r.z + b.z + t.z + k.z + f.z, l.w + r.w + b.w + t.w + k.w + f.w), dc);
-        }
+        return fx_sixth(fx_add4(fx_add4(fx_add4(fx_add4(fx_add4(fx_quad(l), fx_quad(r)), fx_quad(b)), fx_quad(t)), fx_quad(k)), fx_quad(f)), dc);
     };
     if constexpr (EARLY) {
         const float4 l = a.flow(oL), r = a.flow(oR), bo = a.flow(oB), t = a.flow(oT), k = a.flow(oK), f = a.flow(oF);
@@ -425,14 +387,8 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     float bty = picy - orig.y * dt * metric.y;
     float btz = picz - orig.z * dt * metric.z;
     const FxTri tri = fx_tri_setup(g, u, btx, bty, btz);
-    float4 flow, species;
-    if constexpr (TWO) {
-        flow = fx_trilinear_two(g, tri, nz, [&](int i) { return a.flow(i); });
-        species = fx_trilinear_two(g, tri, nz, [&](int i) { return a.species(i); });
-    } else {
-        flow = fx_trilinear(g, tri, [&](int i) { return a.flow(i); });
-        species = fx_trilinear(g, tri, [&](int i) { return a.species(i); });
-    }
+    float4 flow = fx_trilinear(g, tri, nz, [&](int i) { return a.flow(i); });
+    float4 species = fx_trilinear(g, tri, nz, [&](int i) { return a.species(i); });
     species = make_float4(fx_max(species.x, 0.0f), fx_max(species.y, 0.0f), fx_max(species.z, 0.0f),
                           fx_max(species.w, 0.0f));
 
@@ -455,8 +411,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     {  // species diffusion (shaders.ts:182-187)
         if constexpr (!EARLY)
             avg = sixth(a.species(oL), a.species(oR), a.species(oB), a.species(oT), a.species(oK), a.species(oF));
-        if constexpr (TWO) species = fx_f4(fx_mix_two(fx_quad(species), fx_quad(avg), ut[TU_SMIX], nz));
-        else species = fx_mix4(species, avg, ut[TU_SMIX]);
+        species = fx_f4(fx_mix_two(fx_quad(species), fx_quad(avg), ut[TU_SMIX], nz));
     }
 
     // Source injection (shaders.ts:189-201); the sphere list replaces the burner.
@@ -479,7 +434,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         const float vertical = __ldg(tab + L.y + TY_VERT * Y + y);
         const float cellular = FC(0.76) + FC(0.24) * __ldg(tab + L.x + TX_CELL * X + x) * __ldg(tab + L.z + TZ_CELL * Z + z);
         const float lobeArg = __ldg(tab + L.x + TX_LOBE * X + x) * __ldg(tab + L.z + TZ_LOBE * Z + z);
-        const float lobes = fx_mix(FC(0.48), FC(1.18), fx_smoothstep_from<TWO, DIVC_LOBE>(FC(-0.42), lobeArg, dc));
+        const float lobes = fx_mix(FC(0.48), FC(1.18), fx_smoothstep_from<DIVC_LOBE>(FC(-0.42), lobeArg));
         const float texture = fx_mix(cellular, cellular * lobes, ut[TU_CINE]);
         const float pulse = __ldg(tab + L.pulse + z * X + x);
         source = expf(-(radial + vertical)) * texture * pulse;
@@ -507,7 +462,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     const uint32_t liquidRaw = a.liquid(id);
     float water = fx_clamp((float)liquidRaw * (1.0f / 4096.0f) * FC(3.4), 0.0f, 5.0f);
     if (liquidRaw) {
-        float evaporation = water * fx_smoothstep_from<TWO, DIVC_EVAP>(335.0f, flow.w, dc) * dt * FC(13.5);
+        float evaporation = water * fx_smoothstep_from<DIVC_EVAP>(335.0f, flow.w) * dt * FC(13.5);
         flow.w = fx_max(u[U_T_AMBIENT], flow.w - evaporation * 2080.0f - water * dt * 260.0f);
         species.w = fx_clamp(species.w + evaporation * FC(2.15), 0.0f, 3.0f);
     } else {
@@ -519,11 +474,11 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     const float entrainment = ut[TU_ENTRAIN];
     const float ambientOxygen = ut[TU_AMB_O2];
     float oxygenDeficit = fx_clamp(fx_divc(ambientOxygen - species.y, dc[DIVC_AMBIENT_O2]), 0.0f, 1.0f);
-    float fuelCore = fx_smoothstep_from<TWO, DIVC_FUELCORE>(FC(0.30), species.x, dc);
+    float fuelCore = fx_smoothstep_from<DIVC_FUELCORE>(FC(0.30), species.x);
     float interfaceWeight = oxygenDeficit * fx_mix(1.0f, FC(0.18), fuelCore);
     float entrainmentMix = fx_clamp(dt * entrainment *
                                         (FC(0.12) + FC(0.28) * fx_length3(flow.x, flow.y, flow.z) +
-                                         FC(0.22) * fx_smoothstep_from<TWO, DIVC_ENTRAIN_T>(400.0f, flow.w, dc)) *
+                                         FC(0.22) * fx_smoothstep_from<DIVC_ENTRAIN_T>(400.0f, flow.w)) *
                                         interfaceWeight,
                                     0.0f, FC(0.08));
     species.y = fx_mix(species.y, ambientOxygen, entrainmentMix);
@@ -532,7 +487,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     float fuelBefore = fx_max(species.x, 0.0f);
     float oxygenBefore = fx_max(species.y, 0.0f);
     float availableFuel = fx_min(fuelBefore, oxygenBefore * FC(0.25));
-    float ignition = fx_smoothstep_from<TWO, DIVC_IGNITION>(690.0f, flow.w, dc);
+    float ignition = fx_smoothstep_from<DIVC_IGNITION>(690.0f, flow.w);
     // 1 - exp(-arrhenius * ignition * dt). Below ignition (ignition == +0) the exponent is
     // -0 for any finite rate (the rate is clamped to [0, 80]) and the factor is exactly
     // +0, so the rate need not be evaluated; with no liquid exp(-water * 18) is exactly 1.
@@ -581,7 +536,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         flow.z = flow.z + (gx * cy - gy * cx) * vs;
     }
     {  // height-enveloped turbulence (shaders.ts:274-285)
-        float hotPlume = fx_smoothstep_from<TWO, DIVC_HOTPLUME>(520.0f, flow.w, dc);
+        float hotPlume = fx_smoothstep_from<DIVC_HOTPLUME>(520.0f, flow.w);
         float heightEnvelope = __ldg(tab + L.y + TY_HE * Y + y);
         float ltx = __ldg(tab + L.ltx + z * Y + y);
         float lty = __ldg(tab + L.lty + z * X + x);
@@ -592,7 +547,7 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
         flow.z = flow.z + ltz * ts;
     }
     {  // buoyancy (shaders.ts:287-288)
-        float buoyancy = fx_clamp(fx_div_from<TWO, DIVC_BUOYANCY>(u[U_T_AMBIENT], flow.w, dc), FC(-0.1), FC(1.2));
+        float buoyancy = fx_clamp(fx_div_fixed<DIVC_BUOYANCY>(flow.w - u[U_T_AMBIENT]), FC(-0.1), FC(1.2));
         flow.y += buoyancy * dt * FC(0.72) * ut[TU_BUOY];
     }
     if (liquidRaw) species.z *= expf(-water * dt * FC(4.8));  // exp(-0) == 1 exactly otherwise
@@ -666,8 +621,9 @@ FXD float fx_jacobi_numerator(const FxJacobiConst& c, float l, float r, float b,
                      div);
 }
 // RN(x / d) for any finite x through double precision: the product by rcp = RN(1/d) with one
-// correction step is the correctly rounded double quotient, whose rounding to float is x / d
-// (53 >= 2 * 24 + 2 bits). Zeros, infinities and NaN are returned as they are.
+// correction step (Markstein's, as above) is the correctly rounded double quotient, whose rounding
+// to float is x / d (53 >= 2 * 24 + 2 bits; S. A. Figueroa, "When is double rounding innocuous?",
+// SIGNUM Newsletter 30(3), 1995). Zeros, infinities and NaN are returned as they are.
 FXD float fx_div_small(float x, double d, double rcp) {
     const double q = __dmul_rn((double)x, rcp);
     const float r = (float)__fma_rn(__fma_rn(-q, d, (double)x), rcp, q);
@@ -777,9 +733,10 @@ FXD float4 fx_jacobi4(const FxJacobiConst2& c, float l, float4 pc, float r, floa
 // Division by the constant d > 0 in two operations: with 1/d = rh + rl (two floats, rl > 0),
 // RN(x rh + RN(x rl)) (N. Brisebarre and J.-M. Muller, "Correctly rounded multiplication by
 // arbitrary precision constants", IEEE Trans. Computers 57(2), 2008). The engine enables it for
-// a d only after checking on the device that it equals x / d for every float x, with quotients
-// of 0 < |x| < lo taken by fx_div_small; of 1,450 denominators of grids tried it is exact for
-// 1,428 with one of five roundings of rl. rl > 0 keeps zeros' signs, infinities and NaN.
+// a d only after checking one binade of x on the device (fx_two_op_candidates has why that is
+// enough), with quotients of 0 < |x| < lo taken by fx_div_small; of 1,450 denominators of grids
+// tried it is exact for 1,428 with one of five roundings of rl. rl > 0 keeps zeros' signs,
+// infinities and NaN.
 FXD float fx_div_two(float x, float rh, float rl, float lo, double d, double rcp) {
     const float r = __fmaf_rn(x, rh, __fmul_rn(x, rl));
     return fabsf(x) < lo ? fx_div_small(x, d, rcp) : r;

@@ -410,7 +410,8 @@ typedef struct firex_diagnostics {
     int32_t project_resident; /* 1: the residual projection ran inside the resident Jacobi's launch */
     int32_t jacobi_zrun;      /* z planes per CTA the two-sweep launches took (AUTO fits them to the device) */
     int32_t jacobi_registers; /* 1: the resident Jacobi held the pressure in registers (variant 4) */
-    int32_t reserved[3];
+    int32_t jacobi_two_op;    /* 1: the Jacobi may divide in two operations (every member's denominator passed) */
+    int32_t reserved[2];
 } firex_diagnostics;
 int firex_get_diagnostics(const firex_sim* sim, firex_diagnostics* out);
 
