@@ -94,8 +94,9 @@ FX_HOST_DEVICE int fx_reg_outbox_quads(int X, const FxResBox& bx) { return 2 * (
 // ---- division by a constant in two operations (fx_div_two, fx_step_math.cuh) ------------------------
 // The reciprocal 1/d = rh + rl, rh rounded down so that rl > 0 (zeros keep their signs, infinities and
 // NaN pass), with rl rounded to nearest or one or two steps beside it: that rounding decides the few
-// quotients next to a midpoint. From lo on, x rl and x / d are normal: a power of two on x then
-// scales both products and the quotient exactly, and one binade of x decides.
+// quotients next to a midpoint. From lo, the smallest power of two for which x rl and x / d are
+// normal, a power of two on x scales both products and the quotient exactly, so one binade of x
+// decides.
 struct FxTwoOp {
     float rh, rl[5], lo;
 };
@@ -111,7 +112,7 @@ inline FxTwoOp fx_two_op_candidates(float d) {
     t.rl[2] = std::nextafter(rl, 0.0f);
     t.rl[3] = std::nextafter(t.rl[1], INFINITY);
     t.rl[4] = std::nextafter(t.rl[2], 0.0f);
-    t.lo = std::ldexp(1.0f, -60 + std::ilogb(d));
+    t.lo = std::ldexp(1.0f, std::max(-126 - std::ilogb(t.rl[4]), -125 + std::ilogb(d)));
     return t;
 }
 

@@ -658,7 +658,8 @@ FXD float4 fx_jacobi4_finish(const FxJacobiConst2& c, fx_f2 x01, fx_f2 x23, fx_f
         const float2 u = fx_unpack2(fx_fma2(n01, c.rcp, fx_mul2(n01, c.negDenom)));
         const float2 v = fx_unpack2(fx_fma2(n23, c.rcp, fx_mul2(n23, c.negDenom)));
         const float least = fminf(fminf(fabsf(a.x), fabsf(a.y)), fminf(fabsf(b.x), fabsf(b.y)));
-        if (least >= c.lo) return make_float4(u.x, u.y, v.x, v.y);
+        auto tiny = [&](float x) { return x != 0.0f && fabsf(x) < c.lo; };
+        if (least >= c.lo || !(tiny(a.x) || tiny(a.y) || tiny(b.x) || tiny(b.y))) return make_float4(u.x, u.y, v.x, v.y);
         const double D = c.denom, R = *c.rcpD;
         return make_float4(fx_div_small(a.x, D, R), fx_div_small(a.y, D, R), fx_div_small(b.x, D, R), fx_div_small(b.y, D, R));
     }
@@ -697,9 +698,11 @@ FXD float4 fx_jacobi4_finish(const FxJacobiConst2& c, fx_f2 x01, fx_f2 x23, fx_f
 // against 5.65 us per sweep in the resident kernel with the copy warp at HD.
 // TWO: the two-operation quotient instead of Markstein's three and their IEEE fallback, one
 // compare of the smallest magnitude instead of eight, and double precision for a group with
-// a numerator below c.lo or a zero: 128x192x128, 200 sweeps, 1,115 against 1,124 us; the first
-// steps of a fluid at rest, whose fronts are zeros and tiny numerators, 128 sweeps, 1,210
-// against 3,345 us.
+// a nonzero numerator below c.lo (zeros, as everywhere in a fluid at rest, pass through the two
+// operations): 128x192x128, 200 sweeps, 1,115 against 1,124 us; the first
+// steps of a fluid at rest, whose fronts are tiny numerators, 128 sweeps, 1,270 against 3,900 us,
+// and 882 against 949 once they have passed most of the grid (steps 5-8; 1,199 while zeros and
+// numerators from 2^-44 down were taken for tiny).
 template <bool INLINE_RARE = false, bool PACKED_W = false, bool TWO = false>
 FXD float4 fx_jacobi4(const FxJacobiConst2& c, float l, float4 pc, float r, float4 pb, float4 pt, float4 pk, float4 pf,
                       float4 d) {

@@ -150,7 +150,7 @@ def test_one_binade_decides_the_two_operation_quotient(plan, dims, extent):
     highest, and in between: the engine checks the one binade on the device."""
     d = denominator(plan, dims, extent)
     k = plan.two_op_choice(d)
-    assert k >= 0 and 0.0 < plan.two_op_lo(d) < 1e-9
+    assert k >= 0 and 0.0 < plan.two_op_lo(d) <= 2.0 ** -60
     for e in (1000, 1001, -40, 1, 60, 127):
         assert plan.two_op_wrong(d, k, e) == 0, (d, k, e)
 
