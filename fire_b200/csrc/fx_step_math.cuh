@@ -505,10 +505,10 @@ FXD FxCellOut fx_simulate_cell(const FxParams& P, const FxGrid& g, int x, int y,
     float burn = fx_clamp(requestedBurn, 0.0f, availableFuel);
     species.x = fx_max(0.0f, fuelBefore - burn);
     species.y = fx_max(0.0f, oxygenBefore - burn * 4.0f);
-    // richness and the reaction rate only where something burns (burn == +0 elsewhere: the
-    // products below are then +0, whatever the richness, which is in [0, 1])
+    // richness and the reaction rate only where something burns (burn is +0 elsewhere: the products
+    // below are then +0 for any richness in [0, 1], which it is unless the oxygen is NaN)
     float fumes = 0.0f, reaction = 0.0f;
-    if (!(burn == 0.0f)) {
+    if (__float_as_uint(burn) != 0u || !(oxygenBefore == oxygenBefore)) {
         const float richness = fx_clamp(1.0f - oxygenBefore / fx_max(fuelBefore * 4.0f, FC(0.00001)), 0.0f, 1.0f);
         fumes = burn * (1.0f + richness * FC(1.8));
         reaction = fx_clamp(fx_divc(burn, dc[DIVC_DT]) * FC(0.22), 0.0f, 4.0f);
