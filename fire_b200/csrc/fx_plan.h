@@ -204,9 +204,12 @@ inline int fx_zs_run(const std::vector<std::array<int, 3>>& dims, bool half, int
 //   FX_RES_REGISTERS: boxes of strips of two rows, their columns split along z (fx_reg_geom), at
 //     most FX_REG_MAXZ planes to a thread.
 // False when no box fits one CTA's shared memory and registers.
+// Shared memory of the largest box of a plan for FX_RES_REGISTERS, -1 when one does not fit. Boxes
+// differ only in their rows (the last of a row of boxes may have fewer) and by one plane (the
+// first along z has the fewest, the last the most).
 inline long long fx_reg_smem(int X, int Y, int Z, const FxResBox& bx) {
     long long most = 0;
-    for (int iz = 0; iz < bx.nbz; ++iz)
+    for (int iz : {0, bx.nbz - 1})
         for (int iy : {0, bx.nby - 1}) {
             const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, iz * bx.nby + iy);
             if (g.cols > FX_REG_THREADS || g.len > FX_REG_MAXZ || g.cols * g.parts > FX_REG_THREADS) return -1;

@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import ctypes as C
 import subprocess
+import time
 from pathlib import Path
 
 import pytest
@@ -69,6 +70,49 @@ static std::vector<std::array<int, 3>> grids(int n, const int* d) {
     for (int i = 0; i < n; ++i) v.push_back({d[3 * i], d[3 * i + 1], d[3 * i + 2]});
     return v;
 }
+// smem of a plan over every box (-1: one does not fit), as fx_reg_smem has it from four of them
+long long reg_smem_all(int X, int Y, int Z, int by, int nby, int nbz) {
+    const FxResBox bx{by, (Z + nbz - 1) / nbz, nby, nbz};
+    long long most = 0;
+    for (int b = 0; b < nby * nbz; ++b) {
+        const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, b);
+        if (g.cols > FX_REG_THREADS || g.len > FX_REG_MAXZ || g.cols * g.parts > FX_REG_THREADS ||
+            2 * (g.ny + g.nz) * (X / 4) > FX_REG_MAXH * FX_REG_THREADS)
+            return -1;
+        most = std::max(most, fx_reg_smem_bytes(X, g));
+    }
+    return most;
+}
+long long reg_smem(int X, int Y, int Z, int by, int nby, int nbz) {
+    return fx_reg_smem(X, Y, Z, FxResBox{by, (Z + nbz - 1) / nbz, nby, nbz});
+}
+int reg_plan(int n, const int* d, int cap, int* boxes) {  // by, nby, nbz of each member; 0: does not fit
+    std::vector<FxResBox> b;
+    int smem;
+    if (!fx_res_assign(grids(n, d), cap, FX_RES_REGISTERS, &b, &smem)) return 0;
+    for (int i = 0; i < n; ++i) {
+        boxes[3 * i] = b[i].by;
+        boxes[3 * i + 1] = b[i].nby;
+        boxes[3 * i + 2] = b[i].nbz;
+    }
+    return smem;
+}
+// every cell of the grid is stored by one thread of one box
+int reg_covers(int X, int Y, int Z, int by, int nby, int nbz) {
+    const FxResBox bx{by, (Z + nbz - 1) / nbz, nby, nbz};
+    std::vector<int> owners((size_t)Y * Z);
+    for (int b = 0; b < nby * nbz; ++b) {
+        const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, b);
+        if (g.ny % 2 || g.len > FX_REG_MAXZ) return 0;
+        auto start = [&](int r) { return g.parts > 1 ? r * (g.nz - g.len) / (g.parts - 1) : 0; };
+        for (int r = 0; r < g.parts; ++r)
+            for (int k = r > 0 ? start(r - 1) + g.len - start(r) : 0; k < g.len; ++k)
+                for (int y = 0; y < g.ny; ++y) ++owners[(size_t)(g.z0 + start(r) + k) * Y + g.y0 + y];
+    }
+    for (int n : owners)
+        if (n != 1) return 0;
+    return 1;
+}
 int default_kernel(int n, const int* d, int half) {
     const auto v = grids(n, d);
     long long cells = 0;
@@ -94,6 +138,8 @@ def plan(tmp_path_factory):
     for f in (lib.two_op_choice, lib.two_op_lo):
         f.argtypes = [C.c_float]
     lib.two_op_wrong.argtypes = [C.c_float, C.c_int, C.c_int]
+    for f in (lib.reg_smem, lib.reg_smem_all):
+        f.restype = C.c_longlong
     return lib
 
 
@@ -163,3 +209,43 @@ def test_fixed_divisors_of_the_source_pass(plan):
         for e in ((-100, -99, -98) if slot == 0 else (-27, -26)) + (0, 1, 24, 127 if slot != 1 else 125):
             assert plan.fixed_wrong(slot, e) == 0, (slot, e)
         assert plan.fixed_specials(slot) == 0, slot
+
+
+CTAS = 148
+
+
+def test_register_boxes_are_judged_by_their_largest(plan):
+    """Four boxes of a plan stand for all of them, whatever the remainders."""
+    fits = 0
+    for X, Y, Z in [(4, 4, 4), (16, 24, 20), (32, 48, 32), (36, 44, 28), (64, 96, 64), (100, 148, 92), (20, 400, 200), (128, 8, 148)]:
+        for by in range(2, min(Y, 40) + 1, 2):
+            nby = -(-Y // by)
+            for nbz in {n for n in (1, 2, 3, 5, 7, Z // 4, Z // 2, Z - 1) if 0 < n <= Z} | {Z}:
+                want = plan.reg_smem_all(X, Y, Z, by, nby, nbz)
+                assert plan.reg_smem(X, Y, Z, by, nby, nbz) == want, (X, Y, Z, by, nbz)
+                fits += want >= 0
+    assert fits > 100
+
+
+@pytest.mark.parametrize("grids", [[(4, 4, 4)], [(16, 24, 16)], [(32, 48, 32)], [(36, 44, 28)], [(100, 148, 92)], [(96, 144, 96)],
+                                   [(260, 12, 16)], [(64, 96, 64)] * 4, [(48, 72, 48), (32, 48, 32), (64, 96, 64)], [(16, 24, 16)] * 64])
+def test_register_plans_cover_every_cell_once(plan, grids):
+    boxes = (C.c_int * (3 * len(grids)))()
+    assert plan.reg_plan(*flat(grids), CTAS, boxes)
+    assert sum(boxes[3 * i + 1] * boxes[3 * i + 2] for i in range(len(grids))) <= CTAS
+    for i, (X, Y, Z) in enumerate(grids):
+        assert plan.reg_covers(X, Y, Z, *boxes[3 * i:3 * i + 3])
+
+
+def test_a_plan_costs_less_than_the_step_it_prepares(plan):
+    """The register plan of a preview grid, whose step takes 90 us on the device, made in the first step
+    of a handle: 17 us when four boxes are judged per row height, 109 when all of them were."""
+    grids, boxes = flat([(32, 48, 32)]), (C.c_int * 3)()
+    best = min(_timed(lambda: plan.reg_plan(*grids, CTAS, boxes)) for _ in range(200))
+    assert best < 50e-6, best
+
+
+def _timed(f):
+    t = time.perf_counter()
+    f()
+    return time.perf_counter() - t
