@@ -310,91 +310,6 @@ static TwoOpReciprocal two_op_reciprocal(int device, float d) {
     return r;
 }
 
-// Exchange buffers of the resident Jacobi between batches: a step of a new handle would otherwise
-// pay for the allocation (0.3 ms at 64x96x64, more than the step). Holds at most kPoolBytes and
-// nothing once no batch is left; the buffers of a batch are free of work when they come back.
-namespace {
-constexpr size_t kPoolBytes = 64u << 20;
-struct ExchangePool {
-    struct Buffer {
-        int device;
-        unsigned* p;
-        size_t bytes;
-    };
-    std::mutex mu;
-    std::vector<Buffer> idle;
-    size_t held = 0;
-    int batches = 0;
-
-    // Takes a buffer of the current device of at least `need` bytes; *bytes is its size. NULL: none to be had.
-    unsigned* take(int device, size_t need, size_t* bytes) {
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            size_t best = idle.size();
-            for (size_t i = 0; i < idle.size(); ++i)
-                if (idle[i].device == device && idle[i].bytes >= need && (best == idle.size() || idle[i].bytes < idle[best].bytes)) best = i;
-            if (best < idle.size()) {
-                const Buffer b = idle[best];
-                idle.erase(idle.begin() + best);
-                held -= b.bytes;
-                *bytes = b.bytes;
-                return b.p;
-            }
-        }
-        unsigned* p = nullptr;
-        if (cudaMalloc(&p, need) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        *bytes = need;
-        return p;
-    }
-    // Gives a buffer back; the caller has waited for the work that used it.
-    void give(int device, unsigned* p, size_t bytes) {
-        if (!p) return;
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            if (batches > 0 && held + bytes <= kPoolBytes) {
-                idle.push_back(Buffer{device, p, bytes});
-                held += bytes;
-                return;
-            }
-        }
-        cudaFree(p);
-    }
-    void enter() {
-        std::lock_guard<std::mutex> lock(mu);
-        ++batches;
-    }
-    void leave() {
-        std::vector<Buffer> last;
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            if (--batches > 0) return;
-            last.swap(idle);
-            held = 0;
-        }
-        release(last);
-    }
-    void trim() {  // before an allocation that does not fit
-        std::vector<Buffer> all;
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            all.swap(idle);
-            held = 0;
-        }
-        release(all);
-    }
-    static void release(const std::vector<Buffer>& v) {
-        for (const Buffer& b : v) {
-            DeviceGuard dg(b.device);
-            cudaFree(b.p);
-        }
-    }
-};
-ExchangePool g_exchange;
-}  // namespace
-
 // ---- one simulation ------------------------------------------------------------------------
 struct firex_sim {
     int X = 0, Y = 0, Z = 0;
@@ -421,6 +336,9 @@ struct firex_sim {
     std::vector<void*> allocations;
     size_t bytes = 0;
     void* d_tmp = nullptr;          // 4 B/cell scratch: emitter mask, final divergence
+    unsigned* ex = nullptr;         // the register Jacobi's exchange buffer for steps of the handle alone
+    size_t exBytes = 0;
+    int regCtas = -1;               // fewest CTAs of that kernel the grid fits in (0: none, -1: not asked yet)
     double* d_partial = nullptr;    // divergence-norm partials
     double* d_norm = nullptr;
     // overlapped readback (firex_read_field_async): the field is copied on the device into
@@ -480,6 +398,24 @@ struct firex_sim {
         allocations.push_back(p);
         bytes += nbytes;
         return p;
+    }
+
+    // The scratch field, with the register Jacobi's exchange buffer behind it where that kernel fits the
+    // grid and the budget and the device have room for it: one allocation, as a second one costs
+    // 0.3 ms, more than a step at 64x96x64. Without the buffer another variant runs.
+    bool alloc_scratch(size_t planned, size_t freeBytes) {
+        const size_t field = ((size_t)N * 4 + 255) / 256 * 256;
+        FxResBox bx;
+        if (!half && fx_reg_box(X, Y, Z, fx_res_capacity(FxResKernel{4, false, true}), &bx)) {
+            const size_t more = FX_REG_EXCHANGE_HEAD + fx_reg_packets(X, bx) * 16;
+            const size_t room = opt.memory_budget_bytes ? std::min<size_t>(opt.memory_budget_bytes, freeBytes) : freeBytes;
+            if (planned + more <= room && (d_tmp = alloc(field + more)) != nullptr) {
+                ex = reinterpret_cast<unsigned*>(static_cast<char*>(d_tmp) + field);
+                exBytes = more;
+                return true;
+            }
+        }
+        return (d_tmp = alloc((size_t)N * 4)) != nullptr;
     }
 
     static size_t planned_bytes(int X, int Y, int Z, int storage, int mode, int particles) {
@@ -641,9 +577,8 @@ struct firex_batch {
     bool resOk = false;                              // ... and the batch fits one resident launch
     FxResKernel resKernel{};                         // ... of this kernel
     int resSmem = 0;
-    unsigned* ex = nullptr;                          // variant 4's exchange buffer
-    size_t exBytes = 0;
-    bool counted = false;                            // among the pool's batches
+    unsigned* own = nullptr;                         // the register Jacobi's exchange buffer for several members
+    size_t ownBytes = 0;
     std::string err;
 
     // per-pass profiling (events between passes; graphs are bypassed while profiling)
@@ -666,31 +601,46 @@ struct firex_batch {
         tableDirty = true;
     }
 
-    // The exchange buffer of the resident Jacobi's variant 4 for these boxes, every tag cleared:
-    // kept by the batch and grown when a plan needs more (16 bytes a face cell, about 16 MB for a
-    // grid that fills the device). False when it cannot be had: another variant then runs.
+    // The exchange buffer of the register Jacobi for these boxes, every tag cleared. False when there is
+    // none: another variant then runs.
     bool ensure_exchange(const std::vector<std::array<int, 3>>& dims, std::vector<FxResBox>& boxes) {
         size_t packets = 0;
         int maxP = 0, maxR = 0;
         for (size_t i = 0; i < boxes.size(); ++i) {
             boxes[i].exOff = (int)packets;
-            packets += (size_t)boxes[i].nby * boxes[i].nbz * 2 * 2 * fx_reg_outbox_quads(dims[i][0], boxes[i]);
+            packets += fx_reg_packets(dims[i][0], boxes[i]);
             maxP = std::max(maxP, members[i]->h.P);
             maxR = std::max(maxR, members[i]->h.R);
         }
-        const size_t need = 128 + packets * 16;
-        if (need > exBytes) {
-            if (cudaStreamSynchronize(stream) != cudaSuccess) return false;
-            g_exchange.give(device, ex, exBytes);
-            exBytes = 0;
-            ex = g_exchange.take(device, need, &exBytes);
-            if (!ex) return false;
-        }
-        if (cudaMemsetAsync(ex, 0, need, stream) != cudaSuccess) return false;
+        const size_t need = FX_REG_EXCHANGE_HEAD + packets * 16;
+        // a member alone brings its own
+        unsigned* const ex = own ? own : (members.size() == 1 ? members[0]->ex : nullptr);
+        const size_t have = own ? ownBytes : (ex ? members[0]->exBytes : 0);
+        if (need > have || cudaMemsetAsync(ex, 0, need, stream) != cudaSuccess) return false;
         h->ex = ex;
         h->exPhase = maxP + 2;
         h->exStep = maxP + maxR + 8;
         return true;
+    }
+
+    // Allocates a batch's exchange buffer once its members fit one register launch together: of the size
+    // that serves every such launch, when a member joins and not in a step (cudaMalloc takes 0.3 ms).
+    void reserve_exchange() {
+        if (isSolo || own || members.empty() || members[0]->half || (members.size() == 1 && members[0]->ex)) return;
+        const int cap = fx_res_capacity(FxResKernel{4, false, true});
+        int least = 0;
+        for (firex_sim* s : members) {
+            if (s->regCtas < 0) s->regCtas = fx_reg_min_ctas(s->X, s->Y, s->Z, cap);
+            least += s->regCtas;
+            if (s->regCtas == 0 || least > cap) return;
+        }
+        const size_t bytes = fx_reg_exchange_most(cap);
+        if (cudaMalloc(&own, bytes) != cudaSuccess) {  // another variant runs
+            cudaGetLastError();
+            own = nullptr;
+            return;
+        }
+        ownBytes = bytes;
     }
 
     // Fills the brick prefix sums for the launch shape (k, zc); resident boxes when wanted,
@@ -1033,12 +983,9 @@ struct firex_batch {
         for (cudaEvent_t e : evPool) cudaEventDestroy(e);
         evPool.clear();
         if (d) cudaFree(d);
-        g_exchange.give(device, ex, exBytes);
-        if (counted) g_exchange.leave();
-        counted = false;
+        if (own) cudaFree(own);
         d = nullptr;
-        ex = nullptr;
-        exBytes = 0;
+        own = nullptr;
         delete h;
         h = nullptr;
         if (stream) cudaStreamDestroy(stream);
@@ -1060,8 +1007,6 @@ struct firex_batch {
             delete b;
             return nullptr;
         }
-        g_exchange.enter();
-        b->counted = true;
         b->rebuild_table();
         return b;
     }
@@ -1158,6 +1103,7 @@ void firex_sim::release() {
         auto& m = batch->members;
         m.erase(std::remove(m.begin(), m.end(), this), m.end());
         batch->rebuild_table();
+        batch->reserve_exchange();
         batch->drop_graphs();
         batch = nullptr;
     }
@@ -1352,11 +1298,8 @@ int firex_create(const int32_t dims[3], const firex_options* opt, firex_sim** ou
         return FIREX_ERR_CUDA;
     }
     size_t freeB = 0, totalB = 0;
-    if (cudaMemGetInfo(&freeB, &totalB) == cudaSuccess && need > freeB) {
-        g_exchange.trim();
-        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) freeB = need;
-    }
-    if (totalB > 0 && need > freeB) {
+    const bool knowFree = cudaMemGetInfo(&freeB, &totalB) == cudaSuccess;
+    if (knowFree && need > freeB) {
         g_create_error = "grid needs " + std::to_string(need) + " device bytes, " + std::to_string(freeB) + " free";
         s->release();
         delete s;
@@ -1385,7 +1328,7 @@ int firex_create(const int32_t dims[3], const firex_options* opt, firex_sim** ou
         ok = ok && h.corr[i];
     }
     ok = ok && (h.div = (float*)s->alloc((size_t)N * 4)) && (h.reaction = (float*)s->alloc((size_t)N * 4)) &&
-         (h.liquid = (uint32_t*)s->alloc((size_t)N * 4)) && (s->d_tmp = s->alloc((size_t)N * 4)) &&
+         (h.liquid = (uint32_t*)s->alloc((size_t)N * 4)) && s->alloc_scratch(need, knowFree ? freeB : need) &&
          (h.tab = (float*)s->alloc(s->table_bytes())) &&
          (s->d = (FxSimDev*)s->alloc(sizeof(FxSimDev))) &&
          (s->d_partial = (double*)s->alloc(2 * sizeof(double) * (size_t)fx_norm_partial_blocks(N))) &&
@@ -1927,6 +1870,7 @@ int firex_batch_add(firex_batch* b, firex_sim* s) {
     s->dirty = true;
     b->members.push_back(s);
     b->rebuild_table();
+    b->reserve_exchange();
     return FIREX_OK;
 }
 
@@ -1944,6 +1888,7 @@ int firex_batch_remove(firex_batch* b, firex_sim* s) {
     s->batch = nullptr;
     s->dirty = true;
     b->rebuild_table();
+    b->reserve_exchange();
     return FIREX_OK;
 }
 

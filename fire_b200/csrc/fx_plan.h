@@ -53,7 +53,7 @@ FX_HOST_DEVICE int fx_zs_bricks(int X, int Y, int Z, int zc, int txg) {
 // full x rows, nby x nbz of them (CTA b owns box (b % nby, b / nby)).
 struct FxResBox {
     int by, bz, nby, nbz;
-    int exOff;  // variant 4: the member's first packet (16 bytes) in the batch's exchange buffer
+    int exOff;  // FX_RES_REGISTERS: the member's first packet (16 bytes) in the exchange buffer
     int pad[3];
 };
 
@@ -90,6 +90,14 @@ FX_HOST_DEVICE long long fx_reg_smem_bytes(int X, const FxRegGeom& g) {
 }
 // Quads a box sends per sweep: sections y low, y high (bz rows), z low, z high (by rows).
 FX_HOST_DEVICE int fx_reg_outbox_quads(int X, const FxResBox& bx) { return 2 * (bx.by + bx.bz) * (X / 4); }
+// Exchange buffer of a launch: a head whose first word is the tag its packets start from in this step,
+// then each member's packets of 16 bytes, four for a quad that a box sends (two slots of two).
+#define FX_REG_EXCHANGE_HEAD 128
+inline size_t fx_reg_packets(int X, const FxResBox& bx) { return (size_t)bx.nby * bx.nbz * 4 * fx_reg_outbox_quads(X, bx); }
+// ... and the most that a launch of `cap` CTAs takes: a box sends no more than it may receive.
+inline size_t fx_reg_exchange_most(int cap) {
+    return FX_REG_EXCHANGE_HEAD + (size_t)cap * 4 * FX_REG_MAXH * FX_REG_THREADS * 16;
+}
 
 // ---- division by a constant in two operations (fx_div_two, fx_step_math.cuh) ------------------------
 // The reciprocal 1/d = rh + rl, rh rounded down so that rl > 0 (zeros keep their signs, infinities and
@@ -240,6 +248,18 @@ inline bool fx_reg_box(int X, int Y, int Z, int m, FxResBox* out) {
         }
     }
     return found;
+}
+// The fewest CTAs, up to cap, whose boxes hold the grid (0: none).
+inline int fx_reg_min_ctas(int X, int Y, int Z, int cap) {
+    FxResBox bx;
+    if (!fx_reg_box(X, Y, Z, cap, &bx)) return 0;
+    int lo = 1, hi = cap;
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (fx_reg_box(X, Y, Z, mid, &bx)) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo;
 }
 constexpr int FX_RES_REGISTERS = 5;  // variant 4 with the pressure in registers
 inline bool fx_res_box(int X, int Y, int Z, int m, int variant, FxResBox* out) {

@@ -103,7 +103,8 @@ def _percentile(xs, q):
 
 
 class FireXServer:
-    """Admission by HBM budget + one shared batch stepped per tick."""
+    """Admission by HBM budget (the members'; the batch itself holds up to 15 MB beside it) + one shared
+    batch stepped per tick."""
 
     def __init__(self, budget_bytes: int = DEFAULT_BUDGET, max_members: int = 512, clock=time.perf_counter,
                  device_timing: bool = True, dt: float = 1.0 / 60.0, precision: int = A.PRECISION_MIXED,
@@ -178,6 +179,8 @@ class FireXServer:
             if self.tick_budget is not None and not self.tick_budget.fits(self.work, work, len(self.slots)):
                 break  # ... and for the tick's time budget
             self.queue.popleft()
+            # a member takes what it was admitted for: no exchange buffer of its own (the batch has one)
+            opts.memory_budget_bytes = min(opts.memory_budget_bytes or need, need)
             sim = FireXSim(req.dims, opts)
             self.batch.add(sim)
             self.used += need

@@ -325,7 +325,11 @@ int firex_set_profiling(firex_sim* sim, int32_t on);
  * (launches[FIREX_PASS_COUNT]) since the previous call. Either pointer may be NULL. */
 int firex_pass_times(firex_sim* sim, double* ms, int64_t* launches);
 
-/* Device bytes firex_create would allocate for this grid and options (admission). */
+/* Device bytes a simulation of this grid and options cannot do without (admission). On top come
+ * buffers that firex_device_bytes has and this has not: those of the first firex_read_field_async
+ * and firex_set_render_packing, and, where memory_budget_bytes leaves room for it, what the register
+ * Jacobi exchanges its faces through in steps of the handle alone (FP32 pressure; 4.4 MB at 64x96x64,
+ * 12.8 MB at 100x148x92; another variant runs without it). */
 uint64_t firex_planned_device_bytes(const int32_t dims[3], const firex_options* opt);
 
 /* Replays each step from a captured CUDA graph (1, the default) or launches the passes
@@ -421,7 +425,9 @@ int firex_get_diagnostics(const firex_sim* sim, firex_diagnostics* out);
  * members, whatever their grid sizes, and the step is replayed from a CUDA graph. Members
  * must share the storage precision and the pressure storage type; their iteration counts
  * may differ. While a member, a simulation is stepped only through its batch; its field,
- * parameter and state calls stay valid and are ordered with the batch's work. */
+ * parameter and state calls stay valid and are ordered with the batch's work. A batch whose
+ * members fit one launch of the register Jacobi together holds 15 MB of its own from the
+ * firex_batch_add or firex_batch_remove on that made it so. */
 int firex_batch_create(firex_batch** out);
 int firex_batch_destroy(firex_batch* batch); /* members are detached, not destroyed */
 int firex_batch_add(firex_batch* batch, firex_sim* sim);

@@ -97,6 +97,11 @@ int reg_plan(int n, const int* d, int cap, int* boxes) {  // by, nby, nbz of eac
     }
     return smem;
 }
+long long reg_exchange(int X, int by, int bz, int nby, int nbz) {
+    return FX_REG_EXCHANGE_HEAD + 16 * (long long)fx_reg_packets(X, FxResBox{by, bz, nby, nbz});
+}
+long long reg_exchange_most(int cap) { return fx_reg_exchange_most(cap); }
+int reg_min_ctas(int X, int Y, int Z, int cap) { return fx_reg_min_ctas(X, Y, Z, cap); }
 // every cell of the grid is stored by one thread of one box
 int reg_covers(int X, int Y, int Z, int by, int nby, int nbz) {
     const FxResBox bx{by, (Z + nbz - 1) / nbz, nby, nbz};
@@ -138,7 +143,7 @@ def plan(tmp_path_factory):
     for f in (lib.two_op_choice, lib.two_op_lo):
         f.argtypes = [C.c_float]
     lib.two_op_wrong.argtypes = [C.c_float, C.c_int, C.c_int]
-    for f in (lib.reg_smem, lib.reg_smem_all):
+    for f in (lib.reg_smem, lib.reg_smem_all, lib.reg_exchange, lib.reg_exchange_most):
         f.restype = C.c_longlong
     return lib
 
@@ -249,3 +254,19 @@ def _timed(f):
     t = time.perf_counter()
     f()
     return time.perf_counter() - t
+
+
+@pytest.mark.parametrize("grids", [[(32, 48, 32)], [(100, 148, 92)], [(256, 64, 64)], [(64, 96, 64)] * 4, [(256, 32, 32)] * 4,
+                                   [(48, 72, 48), (32, 48, 32), (64, 96, 64)], [(16, 24, 16)] * 64, [(128, 192, 128), (32, 48, 32)],
+                                   [(64, 96, 64)] * 5, [(4, 4, 4)] * 148])
+def test_a_batchs_exchange_buffer_serves_every_plan(plan, grids):
+    """The batch reserves it when its members' fewest CTAs fit together, which is when a plan exists."""
+    boxes = (C.c_int * (3 * len(grids)))()
+    least = [plan.reg_min_ctas(*g, CTAS) for g in grids]
+    fits = plan.reg_plan(*flat(grids), CTAS, boxes) != 0
+    assert fits == (0 not in least and sum(least) <= CTAS)
+    need = 0
+    for i, (X, Y, Z) in enumerate(grids if fits else []):
+        by, nby, nbz = boxes[3 * i:3 * i + 3]
+        need += plan.reg_exchange(X, by, -(-Z // nbz), nby, nbz)
+    assert need <= plan.reg_exchange_most(CTAS) + 128 * len(grids) and plan.reg_exchange_most(CTAS) < 15 << 20
