@@ -571,7 +571,10 @@ struct firex_batch {
     int projFuse = FIREX_PROJECT_AUTO; // batch override of the projection fusion (AUTO: first member's)
     int tableK = -1, tableZc = -1, tableZmZc = -1;  // launch shapes the prefix sums were built for
     int tableSimBy = -1;
-    bool tableTma = false;
+    // what the plans take from the members' sizes, kept until the members change: the fill of the strip
+    // tiles (-1: not asked yet) and the fitted chunk by staging and quotient (0: not asked yet)
+    double fillKept = -1;
+    int zrunKept[2][2] = {};
     int tableRes = -1;                               // whether resident boxes were requested
     std::vector<char> tableWater;                    // which members sprayed when the table was filled
     bool resOk = false;                              // ... and the batch fits one resident launch
@@ -599,6 +602,8 @@ struct firex_batch {
         h->nsims = (int)members.size();
         tableK = -1;
         tableDirty = true;
+        fillKept = -1;
+        std::memset(zrunKept, 0, sizeof(zrunKept));
     }
 
     // The exchange buffer of the register Jacobi for these boxes, every tag cleared. False when there is
@@ -645,7 +650,7 @@ struct firex_batch {
 
     // Fills the brick prefix sums for the launch shape (k, zc); resident boxes when wanted,
     // of variant resForce when that is 0-4.
-    void fill_table(int k, int zc, int zmZc, bool wantRes, int resForce, int simBy, bool tma) {
+    void fill_table(int k, int zc, int zmZc, bool wantRes, int resForce, int simBy) {
         int acc[FX_NSHAPES] = {};
         h->nsims = (int)members.size();
         std::vector<FxResBox> boxes;
@@ -696,7 +701,6 @@ struct firex_batch {
         }
         tableK = k;
         tableSimBy = simBy;
-        tableTma = tma;
         tableZc = zc;
         tableZmZc = zmZc;
         tableRes = wantRes ? 2 + resForce : 0;
@@ -742,7 +746,8 @@ struct firex_batch {
         const bool autoKernel = wantRes, zcOwn = zc > 0;
         if (autoKernel) {
             int dk = 1, dzc = 32;
-            fx_default_jacobi(cells, fx_zs_fill(dims()), p.half, &kernel, &dk, &dzc);
+            if (fillKept < 0) fillKept = fx_zs_fill(dims());
+            fx_default_jacobi(cells, fillKept, p.half, &kernel, &dk, &dzc);
             k = dk;
             if (zc <= 0) zc = dzc;
         }
@@ -754,7 +759,6 @@ struct firex_batch {
         }
         p.k = k;
         p.zc = zc > 0 ? zc : 16;
-        p.zrun = zcOwn ? p.zc : (k == 2 ? fx_zs_run(dims(), p.half, fx_zs_capacity(p.half)) : 16);
         p.fuseP = k == 2 && uniformP && fused_pairs(p.maxP) > 0;
         // a cold start's two solves share their buffers, and the pressure is read from p[P & 1]: with P
         // and R of different parity that is the residual solve's other buffer
@@ -791,12 +795,16 @@ struct firex_batch {
         for (firex_sim* s : members) maps = maps && s->h.tmapOk;
         p.tma = p.k == 2 && maps;
         p.two = true;
-        for (firex_sim* s : members) {
-            p.two = p.two && s->h.jcTwo;
+        for (firex_sim* s : members) p.two = p.two && s->h.jcTwo;
+        p.zrun = p.zc;
+        if (p.k == 2 && !zcOwn) {  // (searching it takes 62 us of host time for a batch of 48)
+            int& run = zrunKept[p.tma][p.two];
+            if (run == 0) run = fx_zs_run(dims(), p.half, fx_zs_capacity(p.half, p.two, p.tma));
+            p.zrun = run;
         }
         if (tableK != p.k || tableZc != p.zrun || tableZmZc != p.zmZc || tableRes != (wantRes ? 2 + resForce : 0) ||
-            tableWater != water_signature() || tableSimBy != p.simBy || tableTma != p.tma)
-            fill_table(p.k, p.zrun, p.zmZc, wantRes, resForce, p.simBy, p.tma);
+            tableWater != water_signature() || tableSimBy != p.simBy)
+            fill_table(p.k, p.zrun, p.zmZc, wantRes, resForce, p.simBy);
         p.res = wantRes && resOk;
         if (p.res) {
             p.resSmem = resSmem;

@@ -27,7 +27,7 @@ void fx_launch_jacobi_zm(cudaStream_t s, bool half, const FxBatchDev* B, int bri
 // two-operation quotient (fx_div_two).
 void fx_launch_jacobi_two(cudaStream_t s, bool half, const FxBatchDev* B, int bricks, int phase, int launch, int zc, bool tma,
                           bool two);
-int fx_zs_capacity(bool half);  // CTAs of that launch the device holds at once
+int fx_zs_capacity(bool half, bool two, bool tma);  // CTAs of that launch the device holds at once
 // Tensor maps of a simulation's pressure pair, correction pair and divergence for the
 // TMA-staged two-sweep pass; false when the driver refuses one (the pass then uses cp.async).
 bool fx_make_tensor_maps(FxSimDev* h);

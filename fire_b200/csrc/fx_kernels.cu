@@ -1006,7 +1006,11 @@ static void launch_zs(cudaStream_t s, const FxBatchDev* B, int bricks, int phase
     const int g = zs_grid<PT, TWO, TMA>();
     fxk_jacobi_zs<PT, sizeof(PT) == 2, TWO, TMA><<<bricks < g ? bricks : g, FX_ZS_THREADS, sizeof(FxZsSmem<PT, FX_ZS_TXG>), s>>>(B, phase, launch, zc);
 }
-int fx_zs_capacity(bool half) { return half ? zs_grid<__half, true, false>() : zs_grid<float, true, false>(); }
+int fx_zs_capacity(bool half, bool two, bool tma) {
+    if (half) return two ? zs_grid<__half, true, false>() : zs_grid<__half, false, false>();
+    if (tma) return two ? zs_grid<float, true, true>() : zs_grid<float, false, true>();
+    return two ? zs_grid<float, true, false>() : zs_grid<float, false, false>();
+}
 
 #ifndef FX_ZS_L2_PROMOTION
 #define FX_ZS_L2_PROMOTION CU_TENSOR_MAP_L2_PROMOTION_L2_128B

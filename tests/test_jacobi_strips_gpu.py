@@ -242,3 +242,67 @@ def test_auto_with_a_cold_start_beyond_the_chip():
     one.step(2, DT)
     assert auto.diagnostics["jacobi_kernel"] == A.JACOBI_FUSED
     same(auto, one)
+
+
+# ---- the fitted chunk is kept with the members -----------------------------------------------------
+
+def test_the_fitted_chunk_follows_the_members():
+    """A batch's chunk is that of its present members: as in a batch that never had others."""
+    from fire_b200.sim import FireXBatch
+    dims = [(160, 216, 152), (128, 128, 96), (96, 144, 96)]
+
+    def chunk(sims, b):
+        b.step(1, DT)
+        b.sync()
+        d = sims[0].diagnostics
+        assert d["jacobi_kernel"] == A.JACOBI_FUSED, d
+        return d["jacobi_zrun"]
+
+    want = {}
+    for n in (1, 2, 3):
+        sims = [FireXSim(d, sphere_options(d, P=8, R=8)) for d in dims[:n]]
+        with FireXBatch() as b:
+            for s in sims:
+                b.add(s)
+            want[n] = chunk(sims, b)
+        for s in sims:
+            s.close()
+    assert len(set(want.values())) > 1, want
+    sims = [FireXSim(d, sphere_options(d, P=8, R=8)) for d in dims]
+    with FireXBatch() as b:
+        for n, s in enumerate(sims, 1):
+            b.add(s)
+            assert chunk(sims, b) == want[n]
+            assert chunk(sims, b) == want[n]
+        b.remove(sims[2])
+        assert chunk(sims, b) == want[2]
+        b.set_jacobi("fused", 2, 9)
+        assert chunk(sims, b) == 9
+        b.set_jacobi("auto")
+        assert chunk(sims, b) == want[2]
+
+
+def test_a_step_call_makes_no_plan_anew():
+    """The host's part of a step of 48 uneven members: a graph launch and a look at the members."""
+    import statistics
+    import time
+    from fire_b200.sim import FireXBatch
+    grids = [(64, 96, 64), (96, 144, 96), (128, 192, 128), (160, 240, 160)]
+    sims = [FireXSim(grids[i % 4], sphere_options(grids[i % 4], P=4, R=4, precision=A.PRECISION_MIXED)) for i in range(48)]
+    one = FireXSim(grids[0], sphere_options(grids[0], P=4, R=4))
+    with FireXBatch() as b:
+        for s in sims:
+            b.add(s)
+
+        def call(stepper):
+            times = []
+            for _ in range(25):
+                stepper.sync()
+                t = time.perf_counter()
+                stepper.step(1, DT)
+                times.append(time.perf_counter() - t)
+            stepper.sync()
+            return statistics.median(times[5:])
+
+        batch, alone = call(b), call(one)
+    assert batch < alone + 20e-6, (batch, alone)
