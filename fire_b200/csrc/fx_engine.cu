@@ -572,8 +572,9 @@ struct firex_batch {
     int tableK = -1, tableZc = -1, tableZmZc = -1;  // launch shapes the prefix sums were built for
     int tableSimBy = -1;
     // what the plans take from the members' sizes, kept until the members change: the fill of the strip
-    // tiles (-1: not asked yet) and the fitted chunk by staging and quotient (0: not asked yet)
+    // tiles (-1: not asked yet) with AUTO's staging, and the fitted chunk by staging and quotient (0: not asked yet)
     double fillKept = -1;
+    bool autoTma = true;
     int zrunKept[2][2] = {};
     int tableRes = -1;                               // whether resident boxes were requested
     std::vector<char> tableWater;                    // which members sprayed when the table was filled
@@ -746,7 +747,10 @@ struct firex_batch {
         const bool autoKernel = wantRes, zcOwn = zc > 0;
         if (autoKernel) {
             int dk = 1, dzc = 32;
-            if (fillKept < 0) fillKept = fx_zs_fill(dims());
+            if (fillKept < 0) {
+                fillKept = fx_zs_fill(dims());
+                autoTma = fx_zs_auto_tma(dims());
+            }
             fx_default_jacobi(cells, fillKept, p.half, &kernel, &dk, &dzc);
             k = dk;
             if (zc <= 0) zc = dzc;
@@ -784,14 +788,12 @@ struct firex_batch {
         // mixed storage HD 154 / 158; 300x452x276 2565 / 2220, 508^3 8302 / 8012, twelve uneven grids
         // of 38 M cells 1660 / 1530)
         p.simEarly = cells < FX_SIM_EARLY_CELLS;
-        // The two-sweep pass stages its planes by TMA (FP32 pressure, every member's tensor maps
-        // built) when asked to, or when AUTO chose the pass with chunks that fill the device's
-        // waves: tensor loads then cost a warp next to nothing (160x240x160: 2.14 against 2.56 ms
-        // of Jacobi per step with cp.async, 508^3: 31.6 against 34.8). A pass asked for with a chunk
-        // of the caller's keeps cp.async, whose planes land sooner in short chunks (188x284x196,
-        // 14-plane chunks: 2.63 against 2.85).
+        // The two-sweep pass stages its planes by TMA (FP32 pressure, every member's tensor maps built) when
+        // asked to, or when AUTO chose the pass with chunks that fill the device's waves (and
+        // fx_zs_auto_tma). A pass asked for with a chunk of the caller's keeps cp.async, whose planes
+        // land sooner in short chunks (188x284x196, 14-plane chunks: 2.63 against 2.85 ms per step).
         const int staging = this->staging != FIREX_STAGING_AUTO ? this->staging : members[0]->staging;
-        bool maps = !p.half && (staging == FIREX_STAGING_TMA || (staging == FIREX_STAGING_AUTO && autoKernel));
+        bool maps = !p.half && (staging == FIREX_STAGING_TMA || (staging == FIREX_STAGING_AUTO && autoKernel && autoTma));
         for (firex_sim* s : members) maps = maps && s->h.tmapOk;
         p.tma = p.k == 2 && maps;
         p.two = true;

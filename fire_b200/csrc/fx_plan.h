@@ -173,6 +173,22 @@ inline void fx_default_jacobi(long long cells, double fill, bool half, int* kern
     *zc = cells >= (16LL << 20) ? 64 : 16;
 }
 
+// Whether AUTO stages the strips' planes by tensor loads (FP32 pressure): they cost a warp next to nothing
+// (160x240x160: 2.14 against 2.56 ms of Jacobi per step with cp.async, 508^3: 31.6 against 34.8). Not for
+// several grids one tile across (17 to 32 cells), whose tiles have nothing beside them to skip and
+// start with two new tensor maps every few planes (us per sweep, tensor loads and cp.async: 60, 130
+// and 200 grids of 32x48x32 10.4 / 9.4, 23.7 / 15.5 and 32.4 / 27.8, 150 of 28x48x32 23.2 / 19.5; on the
+// other side 150 of 36x48x32 38.8 / 42.9, 500 of 16x24x16 16.6 / 17.7, 32x512x256 alone 8.4 / 9.4).
+inline bool fx_zs_auto_tma(const std::vector<std::array<int, 3>>& dims) {
+    double cells = 0, oneTile = 0;
+    for (const auto& d : dims) {
+        const double n = (double)d[0] * d[1] * d[2];
+        cells += n;
+        if (d[0] > 2 * FX_ZS_TXG && d[0] <= 4 * FX_ZS_TXG) oneTile += n;
+    }
+    return dims.size() < 2 || oneTile <= 0.5 * cells;
+}
+
 // z planes per CTA of the two-sweep pass when the caller did not ask for a number: the chunk
 // length that takes the fewest plane steps, counting a chunk's own planes, the one beside it
 // at each end and the time its first planes take to arrive (about two steps more), over the

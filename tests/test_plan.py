@@ -118,6 +118,7 @@ int reg_covers(int X, int Y, int Z, int by, int nby, int nbz) {
         if (n != 1) return 0;
     return 1;
 }
+int auto_tma(int n, const int* d) { return fx_zs_auto_tma(grids(n, d)); }
 int default_kernel(int n, const int* d, int half) {
     const auto v = grids(n, d);
     long long cells = 0;
@@ -270,3 +271,10 @@ def test_a_batchs_exchange_buffer_serves_every_plan(plan, grids):
         by, nby, nbz = boxes[3 * i:3 * i + 3]
         need += plan.reg_exchange(X, by, -(-Z // nbz), nby, nbz)
     assert need <= plan.reg_exchange_most(CTAS) + 128 * len(grids) and plan.reg_exchange_most(CTAS) < 15 << 20
+
+
+@pytest.mark.parametrize("grids,tma", [([(32, 48, 32)] * 60, 0), ([(32, 48, 32)] * 200, 0), ([(28, 48, 32)] * 150, 0), ([(32, 96, 32)] * 90, 0),
+                                       ([(20, 48, 24)] * 256, 0), ([(36, 48, 32)] * 150, 1), ([(16, 24, 16)] * 500, 1), ([(32, 512, 256)], 1),
+                                       ([(160, 240, 160)], 1), ([(64, 96, 64)] * 16, 1), ([(32, 48, 32), (160, 240, 160)], 1)])
+def test_auto_staging(plan, grids, tma):
+    assert plan.auto_tma(*flat(grids)) == tma
