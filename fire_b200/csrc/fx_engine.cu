@@ -668,7 +668,14 @@ struct firex_batch {
                 if (kernel.half && kernel.variant == 4) continue;  // FP32 rows only
                 const int cap = fx_res_capacity(kernel);
                 if (fx_res_assign(dims, cap, v, &boxes, &resSmem)) {
-                    if (kernel.reg && !ensure_exchange(dims, boxes)) continue;
+                    if (kernel.reg) {
+                        bool crowded = false;
+                        for (size_t i = 0; i < boxes.size(); ++i) crowded = crowded || fx_reg_crowded(dims[i][0], boxes[i]);
+                        std::vector<FxResBox> other;
+                        int smem = 0;
+                        if (crowded && fx_res_assign(dims, fx_res_capacity(FxResKernel{4, false, false}), 4, &other, &smem)) continue;
+                        if (!ensure_exchange(dims, boxes)) continue;
+                    }
                     resOk = true;
                     resKernel = kernel;
                     break;

@@ -265,6 +265,12 @@ inline bool fx_reg_box(int X, int Y, int Z, int m, FxResBox* out) {
     }
     return found;
 }
+// Whether the copy warp is the faster for a plan of the register kernel: rows of 244 cells and more, which
+// it brings with few copies, in boxes at the registers' limit (us per sweep, registers and copy warp:
+// 256x64x64 4.41 and 4.02, 252x80x44 4.34 and 4.14; of the 78 other grids measured none, nearest
+// 240x96x48 3.98 and 4.25, 200x80x72 4.08 and 4.31, 256x64x48 3.79 and 3.91).
+inline bool fx_reg_crowded(int X, const FxResBox& bx) { return X >= 244 && (long long)X * bx.by * bx.bz >= 7800; }
+
 // The fewest CTAs, up to cap, whose boxes hold the grid (0: none).
 inline int fx_reg_min_ctas(int X, int Y, int Z, int cap) {
     FxResBox bx;

@@ -59,6 +59,17 @@ def test_the_planner_takes_registers_for_short_columns():
         g.close()
 
 
+def test_the_planner_takes_the_copy_warp_for_crowded_boxes_of_wide_rows():
+    dims = (256, 64, 64)
+    opts = sphere_options(dims, P=6, R=5)
+    one, g = FireXSim(dims, opts), FireXSim(dims, opts)
+    one.set_jacobi("unblocked")
+    one.step(2, DT)
+    g.step(2, DT)
+    variant4(g, registers=0)
+    same(one, g)
+
+
 def test_a_batch_of_small_members_shares_one_register_launch():
     dims = [(32, 48, 32), (36, 44, 28), (48, 64, 48), (32, 48, 32)]
     alone = [FireXSim(d, sphere_options(d, P=7 + i, R=6 - i, seed=i)) for i, d in enumerate(dims)]

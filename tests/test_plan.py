@@ -119,6 +119,10 @@ int reg_covers(int X, int Y, int Z, int by, int nby, int nbz) {
     return 1;
 }
 int auto_tma(int n, const int* d) { return fx_zs_auto_tma(grids(n, d)); }
+int reg_crowded(int X, int Y, int Z, int cap) {
+    FxResBox bx;
+    return fx_reg_box(X, Y, Z, cap, &bx) ? fx_reg_crowded(X, bx) : -1;
+}
 int default_kernel(int n, const int* d, int half) {
     const auto v = grids(n, d);
     long long cells = 0;
@@ -278,3 +282,10 @@ def test_a_batchs_exchange_buffer_serves_every_plan(plan, grids):
                                        ([(160, 240, 160)], 1), ([(64, 96, 64)] * 16, 1), ([(32, 48, 32), (160, 240, 160)], 1)])
 def test_auto_staging(plan, grids, tma):
     assert plan.auto_tma(*flat(grids)) == tma
+
+
+@pytest.mark.parametrize("dims,crowded", [((256, 64, 64), 1), ((256, 60, 64), 1), ((252, 80, 44), 1), ((240, 96, 48), 0), ((240, 40, 100), 0),
+                                          ((200, 80, 72), 0), ((256, 64, 48), 0), ((256, 48, 48), 0), ((304, 208, 16), 0), ((512, 32, 32), 0),
+                                          ((96, 144, 96), 0), ((128, 128, 96), 0), ((60, 184, 144), 0)])
+def test_where_the_copy_warp_is_faster_than_registers(plan, dims, crowded):
+    assert plan.reg_crowded(*dims, CTAS) == crowded
