@@ -164,10 +164,11 @@ inline double fx_zs_fill(const std::vector<std::array<int, 3>>& dims) {
 // at any size (us per sweep, strips and unblocked: 4x1024x1024, fill 0.12, 37.9 and 14.8;
 // 8x512x1024, 0.25, 21.6 and 15.1; 200 grids of 36x16x36, 0.32, 30.4 and 21.7; 128 of 36x44x28, 0.44,
 // 24.5 and 27.9; 16x512x512, 0.49, 13.3 and 15.1). FP16 pressure gains less from strips while it
-// stays in L2: below 8 Mi cells the line is at 0.56 (60 grids of 36x60x36, 0.48, 23.6 and 21.6;
-// 36x400x300, 0.55, 16.2 and 16.0; 512x8x1024, 0.57, 13.5 and 14.4).
+// stays in L2: below 8 Mi cells the line is at 0.50 (60 grids of 36x60x36, 0.48, 23.6 and 21.6;
+// 16x512x512, 0.49, 15.3 and 15.0; 256 of 20x48x24, 0.54, 20.4 and 28.3; 48 of 40x60x40, 0.54, 19.4 and
+// 21.0; 36x400x300, 0.55, 16.2 and 15.9; 512x8x1024, 0.57, 13.5 and 14.4).
 inline void fx_default_jacobi(long long cells, double fill, bool half, int* kernel, int* k, int* zc) {
-    const bool fused = cells >= (2LL << 20) && fill >= (half && cells < (8LL << 20) ? 0.56 : 0.42);
+    const bool fused = cells >= (2LL << 20) && fill >= (half && cells < (8LL << 20) ? 0.50 : 0.42);
     *kernel = fused ? FIREX_JACOBI_FUSED : FIREX_JACOBI_UNBLOCKED;
     *k = fused ? 2 : 1;
     *zc = cells >= (16LL << 20) ? 64 : 16;

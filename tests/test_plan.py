@@ -178,10 +178,10 @@ def flat(grids):
     ([(8, 512, 1024)], 0, A.JACOBI_UNBLOCKED), ([(2048, 4, 512)], 0, A.JACOBI_UNBLOCKED),
     ([(36, 16, 36)] * 200, 0, A.JACOBI_UNBLOCKED), ([(36, 16, 36)] * 450, 0, A.JACOBI_UNBLOCKED),
     ([(4, 64, 64)] * 200, 0, A.JACOBI_UNBLOCKED), ([(4, 2048, 1024)], 0, A.JACOBI_UNBLOCKED),
-    ([(36, 60, 36)] * 60, 1, A.JACOBI_UNBLOCKED), ([(36, 400, 300)], 1, A.JACOBI_UNBLOCKED),
+    ([(36, 60, 36)] * 60, 1, A.JACOBI_UNBLOCKED), ([(16, 512, 512)], 1, A.JACOBI_UNBLOCKED),
     # and those on which the strips are the faster
     ([(16, 512, 512)], 0, A.JACOBI_FUSED), ([(36, 60, 36)] * 60, 0, A.JACOBI_FUSED),
-    ([(36, 60, 36)] * 120, 1, A.JACOBI_FUSED), ([(512, 8, 1024)], 1, A.JACOBI_FUSED),
+    ([(20, 48, 24)] * 256, 1, A.JACOBI_FUSED), ([(40, 60, 40)] * 48, 1, A.JACOBI_FUSED), ([(36, 60, 36)] * 120, 1, A.JACOBI_FUSED), ([(512, 8, 1024)], 1, A.JACOBI_FUSED),
     ([(160, 240, 160)], 0, A.JACOBI_FUSED), ([(160, 240, 160)], 1, A.JACOBI_FUSED),
     ([(36, 44, 28)] * 128, 0, A.JACOBI_FUSED), ([(508, 508, 508)], 0, A.JACOBI_FUSED),
     ([(64, 96, 64), (160, 240, 160), (128, 192, 128)], 0, A.JACOBI_FUSED),
