@@ -99,10 +99,11 @@ FXD void fx_zs_tensor(void* dst, const CUtensorMap* map, int x, int y, int z, un
 FXD void fx_zs_map_acquire(const CUtensorMap* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
 }
-// Bounded wait for the phase of bar with the given parity; the limit is read once the first poll has failed.
+// Bounded wait for the phase of bar with the given parity; the simulation's own limit counts while a test
+// holds a brick (fx_zs_held), and is read once the first poll has failed.
 FXD bool fx_zs_wait(const FxSimDev& S, unsigned long long* bar, unsigned parity) {
     if (fx_mbar_try_wait(bar, parity)) return true;
-    const unsigned own = S.sync[FX_SYNC_SPIN];
+    const unsigned own = S.sync[FX_SYNC_HOLD_BOX] ? S.sync[FX_SYNC_SPIN] : 0u;
     return fx_mbar_wait(bar, parity, own ? own : FX_ZS_WAIT_LIMIT);
 }
 // firex_test_hold_face: whether a test holds this brick. Read while the first planes are on their way (read

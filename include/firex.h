@@ -237,8 +237,9 @@ int firex_divergence_norm(firex_sim* sim, double out[3]);
 int firex_divergence_norm_noalloc(const void* flow, const int32_t dims[3], const float metric[3], void* stream,
                                   double out[3]);
 
-/* Bounded device waits. The resident Jacobi's CTAs wait on their neighbours' faces, the two-sweep
- * pass on its tensor loads; a wait gives up after `polls` polls (0: the library's limit, well over a second), sets the
+/* Bounded device waits. The resident Jacobi's CTAs wait on their neighbours' faces (and, while
+ * firex_test_hold_face holds one of its chunks, the two-sweep pass on its tensor loads); a wait
+ * gives up after `polls` polls (0: the library's limit, well over a second), sets the
  * simulation's error word and returns, and the next firex_sync / firex_batch_sync answers
  * FIREX_ERR_TIMEOUT and poisons the handle (the reference's device-lost state,
  * FireXEngine.ts:538-542,2887-2897: later calls fail with FIREX_ERR_STATE). */

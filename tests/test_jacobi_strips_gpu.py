@@ -306,3 +306,15 @@ def test_a_step_call_makes_no_plan_anew():
 
         batch, alone = call(b), call(one)
     assert batch < alone + 20e-6, (batch, alone)
+
+
+@pytest.mark.parametrize("P,R,launches", [(6, 8, 4 + 4), (13, 10, 7 + 6), (4, 3, 2 + 3), (3, 2, 3 + 2), (16, 1, 8 + 1)])
+def test_launches_of_a_fused_solve(P, R, launches):
+    """An even number of two-sweep launches and up to three single sweeps, beside the step's own seven."""
+    dims = (36, 32, 20)
+    s = FireXSim(dims, sphere_options(dims, P=P, R=R))
+    s.set_jacobi("fused", 2)
+    s.step(1, DT)
+    s.sync()
+    assert s.diagnostics["launches_per_step"] == 7 + launches, s.diagnostics
+    s.close()
