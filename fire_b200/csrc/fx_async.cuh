@@ -17,10 +17,6 @@ FXD void fx_mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fx_smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
-// Adds `bytes` without arriving.
-FXD void fx_mbar_expect_more(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n" ::"r"(fx_smem_u32(bar)), "r"(bytes) : "memory");
-}
 FXD void fx_mbar_arrive(unsigned long long* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(fx_smem_u32(bar)) : "memory");
 }

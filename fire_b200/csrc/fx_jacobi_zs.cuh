@@ -99,15 +99,8 @@ FXD void fx_zs_tensor(void* dst, const CUtensorMap* map, int x, int y, int z, un
 FXD void fx_zs_map_acquire(const CUtensorMap* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
 }
-// Bounded wait for the phase of bar with the given parity; the simulation's own limit counts while a test
-// holds a brick (fx_zs_held), and is read once the first poll has failed.
-FXD bool fx_zs_wait(const FxSimDev& S, unsigned long long* bar, unsigned parity) {
-    if (fx_mbar_try_wait(bar, parity)) return true;
-    const unsigned own = S.sync[FX_SYNC_HOLD_BOX] ? S.sync[FX_SYNC_SPIN] : 0u;
-    return fx_mbar_wait(bar, parity, own ? own : FX_ZS_WAIT_LIMIT);
-}
-// firex_test_hold_face: whether a test holds this brick. Read while the first planes are on their way (read
-// before they were asked for it cost 0.9 % of a step at 160x240x160).
+// firex_test_hold_face: whether a test holds this brick, whose first wait then counts as run out. Read while
+// the first planes are on their way.
 FXD bool fx_zs_held(const FxSimDev& S, int brick, int launch) {
     return S.sync[FX_SYNC_HOLD_BOX] == (unsigned)brick + 1u && (unsigned)launch >= S.sync[FX_SYNC_HOLD_SWEEP];
 }
@@ -169,17 +162,15 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         if (TMA && t == 0) fx_mbar_expect_tx(&sm.bar, (ZERO_IN ? 0 : nP) * BP + BD);
     };
     // the copies requested last have landed, for every thread; false when a bounded wait ran out
-    auto landed = [&](bool requested) {
+    auto landed = [&](bool requested, bool held = false) {
         if (!TMA) {
             fx_cp_wait<0>();
             __syncthreads();
             return true;
         }
-        const bool late = requested && !fx_zs_wait(S, &sm.bar, parity);
+        const bool late = requested && (held || !fx_mbar_wait(&sm.bar, parity, FX_ZS_WAIT_LIMIT));
         if (requested) parity ^= 1u;
-        if (!fx_bar_or(0, FX_ZS_THREADS, late)) return true;
-        if (t == 0) fx_zs_wait(S, &sm.bar, parity ^ 1u);  // the one phase in flight
-        return false;
+        return !fx_bar_or(0, FX_ZS_THREADS, late);
     };
     const FxJacobiK<TWO> K = fx_jacobi_k<TWO>(S);
     constexpr int ROWS = H::ROWS;
@@ -312,8 +303,7 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
     issueP(zs + 1, 1);
     issueD(zs, 0);
     if (!TMA) fx_cp_commit();
-    else if (t == 0 && fx_zs_held(S, brick, launch)) fx_mbar_expect_more(&sm.bar, 16);  // bytes that nothing brings
-    if (!landed(true)) return false;
+    bool ok = landed(true, TMA && t == 0 && fx_zs_held(S, brick, launch));
     FxQuad p0[FX_ZS_ROWS], p1[FX_ZS_ROWS], p2[FX_ZS_ROWS], s0[FX_ZS_ROWS], s1[FX_ZS_ROWS], s2[FX_ZS_ROWS];
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
@@ -329,12 +319,14 @@ FXD bool fx_zs_tile(const FxSimDev& S, const PT* __restrict__ pin, PT* __restric
         rm = ld1(2, ro);
         rc = ld1(0, ro);
     }
-    for (int z = zs; z <= z1; z += 3) {
-        if (!step(FxZsInt<0>(), z, p0, p1, p2, s0, s1, s2)) return false;
-        if (z + 1 > z1) break;
-        if (!step(FxZsInt<1>(), z + 1, p1, p2, p0, s1, s2, s0)) return false;
-        if (z + 2 > z1) break;
-        if (!step(FxZsInt<2>(), z + 2, p2, p0, p1, s2, s0, s1)) return false;
+    for (int z = zs; ok && z <= z1; z += 3) {
+        if (!(ok = step(FxZsInt<0>(), z, p0, p1, p2, s0, s1, s2)) || z + 1 > z1) break;
+        if (!(ok = step(FxZsInt<1>(), z + 1, p1, p2, p0, s1, s2, s0)) || z + 2 > z1) break;
+        ok = step(FxZsInt<2>(), z + 2, p2, p0, p1, s2, s0, s1);
+    }
+    if (!ok) {  // the loads of the phase whose wait ran out, the only ones in flight, land before the CTA ends
+        if (TMA && t == 0) fx_mbar_wait(&sm.bar, parity ^ 1u, FX_ZS_WAIT_LIMIT);
+        return false;
     }
     __syncthreads();  // the next brick's copies may refill every slot
     return true;

@@ -237,9 +237,8 @@ int firex_divergence_norm(firex_sim* sim, double out[3]);
 int firex_divergence_norm_noalloc(const void* flow, const int32_t dims[3], const float metric[3], void* stream,
                                   double out[3]);
 
-/* Bounded device waits. The resident Jacobi's CTAs wait on their neighbours' faces (and, while
- * firex_test_hold_face holds one of its chunks, the two-sweep pass on its tensor loads); a wait
- * gives up after `polls` polls (0: the library's limit, well over a second), sets the
+/* Bounded device waits. The resident Jacobi's CTAs wait on their neighbours' faces; a wait gives
+ * up after `polls` polls (0: the library's limit, well over a second), sets the
  * simulation's error word and returns, and the next firex_sync / firex_batch_sync answers
  * FIREX_ERR_TIMEOUT and poisons the handle (the reference's device-lost state,
  * FireXEngine.ts:538-542,2887-2897: later calls fail with FIREX_ERR_STATE). */
@@ -248,8 +247,8 @@ int firex_set_wait_limit(firex_sim* sim, uint32_t polls);
 /* Test hook for the error path above (no reference counterpart): from the next step on, box
  * `box` of the resident Jacobi stops publishing its faces from sweep `sweep` on (in either
  * phase), a flag that nothing sets, so its neighbours' bounded waits expire. In the two-sweep pass
- * staged by TMA, chunk `box` waits for bytes that nothing brings from launch `sweep` of a phase
- * on. box < 0 clears it. */
+ * staged by TMA, the first wait of chunk `box` counts as run out from launch `sweep` of a phase on.
+ * box < 0 clears it. */
 int firex_test_hold_face(firex_sim* sim, int32_t box, int32_t sweep);
 
 /* Counters that decide ping-pong parity and time (FireXEngine.ts:396-409). */

@@ -164,8 +164,8 @@ def test_flat_grids_fp16_pressure(dims):
 # ---- a wait on tensor loads that runs out -------------------------------------------------------
 
 def test_unfinished_tensor_loads_expire_the_wait():
-    """Chunk 0 waits for bytes that nothing brings, with a short limit: its CTA waits once more for its
-    loads, reports and returns, the host answers with a timeout, and a fresh handle steps exactly."""
+    """Chunk 0's first wait counts as run out: its CTA waits once more for its loads, reports and
+    returns, the host answers with a timeout, and a fresh handle steps exactly."""
     from fire_b200.sim import FireXError
     dims = (36, 32, 20)
     opts = sphere_options(dims, P=4, R=4)
@@ -180,7 +180,6 @@ def test_unfinished_tensor_loads_expire_the_wait():
     g.step(1, DT)
     g.sync()
     assert g.diagnostics["jacobi_staging"] == A.STAGING_TMA
-    g.set_wait_limit(16)
     g.test_hold_face(0, 1)
     g.step(1, DT)
     with pytest.raises(FireXError) as e:
