@@ -66,14 +66,15 @@ JACOBI_KERNEL_NAMES = {1: "fxk_jacobi<float>", 2: "fxk_jacobi_zm<float>", 3: "fx
 
 
 def two_sweep_roofline(jac: dict, cells: int, peak: float, peak_kind: str) -> dict:
-    """The two-sweep pass at 508^3 against the copy bandwidth: algorithmic bytes per launch
-    (2 sweeps x 12 B x cells) over the average launch time from the per-pass events, and the
-    DRAM traffic of a launch scaled from the 508x508x128 capture."""
+    """The two-sweep pass at 508^3 against the copy bandwidth: algorithmic bytes per launch (12 B x
+    cells: its two sweeps share one read of pressure and divergence and one write) over the
+    average launch time from the per-pass events, and the DRAM traffic of a launch scaled from the
+    508x508x256 capture."""
     launches = jac.get("launches_per_step") or 0
     if not launches or not jac.get("ms_per_step"):
         return {}
     us = jac["ms_per_step"] / launches * 1e3
-    alg = 2 * JACOBI_BYTES_PER_CELL * cells
+    alg = JACOBI_BYTES_PER_CELL * cells
     achieved = alg / (us / 1e6) / 1e9
     return {"roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": peak_kind, "avg_launch_us": us, "algorithmic_bytes_per_launch": alg,
@@ -609,9 +610,13 @@ def measure_508(warmup: int = 3, steps: int = STEPS_508) -> dict:
     n = DIMS_508[0] * DIMS_508[1] * DIMS_508[2]
     peak, peak_kind = measured_peak_hbm()
     ms = total_ms / steps
-    achieved = STEP_BYTES_PER_CELL * n / (ms / 1e3) / 1e9
+    pass_bytes = dict(PASS_BYTES_PER_CELL)
+    if diag.get("jacobi_block") == 2:  # two sweeps share a launch's bytes
+        pass_bytes["jacobi"] = JACOBI_BYTES_PER_CELL * passes["jacobi"][1] / prof
+    step_bytes = sum(pass_bytes.values())
+    achieved = step_bytes * n / (ms / 1e3) / 1e9
     per_pass = {}
-    for k, b in PASS_BYTES_PER_CELL.items():
+    for k, b in pass_bytes.items():
         t = passes[k][0] / prof
         a = b * n / (t / 1e3) / 1e9 if t > 0 else None
         per_pass[k] = {"ms_per_step": t, "launches_per_step": passes[k][1] / prof, "algorithmic_bytes_per_cell": b,
@@ -623,11 +628,11 @@ def measure_508(warmup: int = 3, steps: int = STEPS_508) -> dict:
         "value": n * steps / (total_ms / 1e3) / 1e9, "unit": METRIC, "ms_per_step": ms,
         "p50_step_ms": percentile(step_ms, 0.5), "p99_step_ms": percentile(step_ms, 0.99),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_kind": peak_kind, "bytes_per_cell_step": STEP_BYTES_PER_CELL,
+                     "peak_kind": peak_kind, "bytes_per_cell_step": step_bytes,
                      "target_frac": 0.70},
         "passes": per_pass, "profiled_steps": prof,
         "jacobi": {"kernel": jacobi_kernel_name(diag), "block": diag.get("jacobi_block"),
-                   "zchunk": diag.get("jacobi_zchunk"), **two_sweep_roofline(per_pass["jacobi"], n, peak, peak_kind)},
+                   "zchunk": diag.get("jacobi_zrun"), **two_sweep_roofline(per_pass["jacobi"], n, peak, peak_kind)},
         "launches_per_step": diag.get("launches_per_step"),
         "clocks": clk.summary(),
     }

@@ -158,8 +158,9 @@ inline double fx_zs_fill(const std::vector<std::array<int, 3>>& dims) {
 // Jacobi kernel when the caller did not choose one (measured on B200, 96+96 sweeps): below 2 Mi
 // cells per batch the unblocked kernel; from there two sweeps per pass by z-marching strips
 // (160x240x160: 2.14 ms of Jacobi per step against 3.95 unblocked; 508^3: 31.6 against 56.5
-// for one sweep per pass), in chunks of 16 planes, or 64 from 16 Mi cells, stretched or shortened
-// to fill the device's waves (fx_zs_run). fire_b200/autotune.py refines this per workload.
+// for one sweep per pass; near the line, 128x128x132, 6.6 us a sweep against 10.3, with FP16 pressure
+// 7.3 against 10.3), in chunks fitted to the device (fx_zs_run; zc, 16 or 64 by size, is what
+// firex_diagnostics.jacobi_zchunk reports). fire_b200/autotune.py refines this per workload.
 // Narrow and flat grids leave the tiles empty: below a fill of 0.42 the unblocked kernel is the faster
 // at any size (us per sweep, strips and unblocked: 4x1024x1024, fill 0.12, 37.9 and 14.8;
 // 8x512x1024, 0.25, 21.6 and 15.1; 200 grids of 36x16x36, 0.32, 30.4 and 21.7; 128 of 36x44x28, 0.44,
@@ -198,7 +199,10 @@ inline int fx_zs_run(const std::vector<std::array<int, 3>>& dims, bool half, int
     int best = 16, maxZ = 0;
     double least = 0;
     for (const auto& d : dims) maxZ = std::max(maxZ, d[2]);
-    if (half) maxZ = std::min(maxZ, 64);  // FP16 rows: 412x616x412 17.0 ms at 52 planes, 18.0 at 206
+    // FP16 rows do not gain from long chunks (412x616x412 10.3 ms at 52 planes, 10.8 at 206; 640x400x320 8.5
+    // at 54, 9.4 at 206); of eight grids from 10 to 131 M cells the chunk taken so is within 4 % of the
+    // best of eleven
+    if (half) maxZ = std::min(maxZ, 64);
     for (int zc = std::min(4, maxZ); zc <= maxZ; ++zc) {
         long long bricks = 0, steps = 0;
         for (const auto& d : dims) {
@@ -255,7 +259,8 @@ inline bool fx_reg_box(int X, int Y, int Z, int m, FxResBox* out) {
         const long long smem = fx_reg_smem(X, Y, Z, bx);
         if (smem < 0 || smem > FX_RES_SMEM_MAX) continue;
         const FxRegGeom g = fx_reg_geom(X, Y, Z, bx, (nbz - 1) * nby);
-        // cycles of a sweep, roughly: the warps' issue slots or one warp's chain, and the faces
+        // cycles of a sweep, roughly: the warps' issue slots or one warp's chain, and the faces. An estimate
+        // that orders plans; fx_reg_crowded has its one miss among the 81 grids measured.
         const double warps = (g.cols * g.parts + 31) / 32;
         const double cost = std::max(warps * g.len * 2 * 25.0, g.len * 2 * 100.0) + 2.0 * (by + bx.bz) * (X / 4) / FX_REG_THREADS * 100.0;
         if (!found || cost < best) {

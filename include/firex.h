@@ -403,7 +403,7 @@ int firex_batch_set_tiles(firex_batch* batch, int32_t simulate_by, int32_t proje
 typedef struct firex_diagnostics {
     int32_t fast_division;    /* 1: the Jacobi division uses the checked constant-divisor path */
     int32_t jacobi_block;     /* sweeps fused per Jacobi launch (1: one sweep per launch) */
-    int32_t jacobi_zchunk;    /* z planes per CTA of the Jacobi launches, as asked for or by AUTO's rule */
+    int32_t jacobi_zchunk;    /* z planes per CTA asked for, or AUTO's 16 or 64 by size (jacobi_zrun: those taken) */
     int32_t graph;            /* 1: steps replay a captured CUDA graph */
     int32_t launches_per_step;
     int32_t jacobi_kernel;    /* FIREX_JACOBI_* kernel the last step ran */
